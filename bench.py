@@ -438,22 +438,29 @@ def plain_kernel_leg(n, bits, mats, stream, barrier, ngates=120):
     complex128 with FP64 arithmetic: per kernel, launches, time per launch and
     achieved HBM bandwidth (bytes of the amplitudes each launch touches, read
     and written) against the measured peak."""
-    from q1tsim_gb300 import Plan, VectorState
+    from q1tsim_gb300 import VectorState
     peak, peak_kind = peaks()
     sub = bits[:ngates]
-    ndbl = sum(2 * (1 << len(b)) ** 2 for b in sub)
+    # gate by gate: a plan would apply several of them per pass
+    ends = np.cumsum([0] + [(1 << len(b)) ** 2 for b in sub])
+    flat = mats.view(np.complex128)
+    gate_mats = [flat[a:z].reshape(1 << len(b), 1 << len(b)) for a, z, b in zip(ends, ends[1:], sub)]
+
+    def apply_all(st):
+        for m, b in zip(gate_mats, sub):
+            st.apply_gate(m, b)
+
     out = {"gates": len(sub), "peak_gbs": peak, "peak_kind": peak_kind}
     for label, prec, exact in (("c64", "c64", False), ("c128", "c128", False), ("c128_fp64", "c128", True)):
         st = VectorState(n, 1, prec)
         st.set_stream(stream.cuda_stream)
         if exact:
             st.set_fp64_exact()
-        plan = Plan(n, sub, 0)
-        st.apply_plan(plan, mats[:ndbl])      # warm-up: allocation, first touch
+        apply_all(st)      # warm-up: allocation, first touch
         barrier()
         st.profile(True)
         st.profile_report(reset=True)
-        st.apply_plan(plan, mats[:ndbl])
+        apply_all(st)
         prof = st.profile_report(reset=True)
         st.profile(False)
         ks = {}

@@ -96,6 +96,18 @@ __device__ __forceinline__ T cmul(T a, T x)
     return r;
 }
 
+// x times a unit: code 0 -> x, 1 -> i x, 2 -> -x, 3 -> -i x.
+template <typename T>
+__device__ __forceinline__ T unit_times(int u, T x)
+{
+    switch (u) {
+        case 1: return T{-x.y, x.x};
+        case 2: return T{-x.x, -x.y};
+        case 3: return T{x.y, -x.x};
+        default: return x;
+    }
+}
+
 // Host-side error string of the current thread (the C-ABI's q1g_last_error).
 void set_last_error(const std::string& msg);
 

@@ -5,6 +5,7 @@
 // collapsed basis columns are kept as indices, and every amplitude pass is
 // one of the kernels in gate_kernels.cu / state_kernels.cu / measure_kernels.cu.
 #include "engine.h"
+#include "gate_run.h"
 
 #include <algorithm>
 #include <memory>
@@ -997,9 +998,12 @@ static void run_swap_block(q1g_state* s, const FusedBlock& b, const std::vector<
     });
 }
 
-// A phase-run block (fuse_runs): on complex64 states of up to 32
-// qubits one pass of run_phase/phase_pair kernels with the block's phase
-// function (and its trailing 1-qubit gate); otherwise its gates one by one.
+// Whether phase-run blocks of this state run as one pass of phase kernels
+// (otherwise their gates run as plain gates).
+static bool phase_kernels_take(const q1g_state* s) { return s->prec == kC64 && s->nbits <= 32; }
+
+// A phase-run block (fuse_runs) of a state phase_kernels_take: one pass with
+// the block's phase function (and its trailing 1-qubit gate).
 // Each gate of the run must be diagonal with unit-modulus entries: its
 // log-phases theta_s over its (at most two) qubits contribute, by the Moebius
 // transform, a constant, one linear term per qubit and, for two qubits, the
@@ -1010,13 +1014,6 @@ static void run_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, cons
 {
     const int n = s->nbits;
     const size_t ndiag = b.gates.size() - (b.trailing_pair ? 1 : 0);
-    if (s->prec != kC64 || n > 32) {
-        for (int g : b.gates) {
-            const GateOp op = classify(gates[g].mat.data(), (int)gates[g].bits.size(), gates[g].bits.data(), n);
-            if (op.kind != GateOp::Noop) s->apply_op(op, s->amps.as<char>(), s->total());
-        }
-        return;
-    }
     const int pivot_q = phase_run_pivot(b, p->gate_bits);
     const int pivot_pos = pivot_q >= 0 ? n - 1 - pivot_q : -1;
     std::vector<double> lin0(n, 0.0), lin1(n, 0.0);
@@ -1067,6 +1064,40 @@ static void run_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, cons
     s->launch(b.trailing_pair ? "phase_pair_run_c64" : "phase_run_c64", 2.0 * total * s->bsz(), [&] {
         return launch_phase_run(s->amps.as<float2>(), total, n, pivot_pos, dtab, q_pos, m2, s->sm_count(), s->stream);
     });
+}
+
+// Consecutive pair and phase updates (every one run_takes) as tile passes
+// (gate_run.h).  A pass of one op, or one whose ops together touch less than
+// the state where that is what costs (a state beyond the L2: two CX read and
+// write half of it each), goes gate by gate.
+template <typename Stage>
+static void run_plain_gates(q1g_state* s, const std::vector<GateOp>& ops, Stage&& stage)
+{
+    const uint64_t total = s->total();
+    std::vector<const GateOp*> list;
+    for (const GateOp& op : ops) list.push_back(&op);
+    auto one = [&](const GateOp& op) { s->apply_op(op, s->amps.as<char>(), total); };
+    if (ops.size() < 2) {
+        for (const GateOp& op : ops) one(op);
+        return;
+    }
+    const char* name = s->prec == kC64 ? "gate_run_c64" : s->fp64_exact ? "gate_run_c128_fp64" : "gate_run_c128";
+    std::vector<RunOp> table;
+    for (const RunPass& pass : group_runs(list, s->nbits, total, s->prec, s->fp64_exact)) {
+        uint64_t touched = 0;
+        for (int i : pass.ops) touched += ops[i].touched(total);
+        if (pass.ops.size() < 2 || (touched <= total && total * s->bsz() > (uint64_t(64) << 20))) {
+            for (int i : pass.ops) one(ops[i]);
+            continue;
+        }
+        table.clear();
+        for (int i : pass.ops) table.push_back(make_run_op(ops[i], pass.tile));
+        const RunOp* d = static_cast<const RunOp*>(stage(table.data(), table.size() * sizeof(RunOp)));
+        s->launch(name, 2.0 * total * s->bsz(), [&] {
+            return launch_gate_run(s->amps.p, s->prec, total, pass.tile, d, (int)table.size(), s->fp64_exact,
+                                   s->stream);
+        });
+    }
 }
 
 // Positions a plan may leave out of its start-of-run subspace: the compact
@@ -1258,8 +1289,10 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
     // slice of one pinned buffer (at most 32 KB per block).
     if (p->staged) check_cuda(cudaEventSynchronize(p->staged), "plan staging wait");
     else check_cuda(cudaEventCreateWithFlags(&p->staged, cudaEventDisableTiming), "cudaEventCreate");
-    p->hmats.ensure(std::max<size_t>(nb, 1) * 32768);
-    p->dmats.ensure(std::max<size_t>(nb, 1) * 32768);
+    // (plain gates 512 bytes each: a run table entry and its alignment)
+    const size_t staging = std::max<size_t>(nb, 1) * 32768 + ng * 512;
+    p->hmats.ensure(staging);
+    p->dmats.ensure(staging);
     size_t staged = 0;
     auto stage = [&](const void* src, size_t sz) -> const void* {
         char* h = p->hmats.as<char>() + staged;
@@ -1277,7 +1310,39 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
     const size_t first = (subspace_prefix && s->sparse && s->ncols == 1 && s->basis.size() == 1)
                              ? run_subspace_prefix(p, s, mats, n)
                              : 0;
+    // plain gates (pairs and phases) gathered until another kind of block
+    // comes, then grouped into tile passes
+    std::vector<GateOp> plain;
+    auto flush_plain = [&] {
+        if (plain.empty()) return;
+        begin();
+        run_plain_gates(s, plain, stage);
+        plain.clear();
+    };
     for (size_t i = first; i < nb; ++i) {
+        if (p->blocks[i].phase_run && !phase_kernels_take(s)) {
+            for (int g : p->blocks[i].gates) {
+                GateOp op = classify(gates[g].mat.data(), (int)gates[g].bits.size(), gates[g].bits.data(), s->nbits);
+                if (op.kind == GateOp::Noop) continue;
+                if (run_takes(op)) {
+                    plain.push_back(std::move(op));
+                } else {
+                    flush_plain();
+                    begin();
+                    s->apply_op(op, s->amps.as<char>(), s->total());
+                }
+            }
+            continue;
+        }
+        if (!p->blocks[i].phase_run && !p->blocks[i].swap_run) {
+            prepare(i);
+            if (ops[i].kind == GateOp::Noop) continue;
+            if (run_takes(ops[i])) {
+                plain.push_back(ops[i]);
+                continue;
+            }
+        }
+        flush_plain();
         if (p->blocks[i].phase_run) {
             begin();
             run_phase_block(p, s, p->blocks[i], gates, stage);
@@ -1288,9 +1353,7 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
             run_swap_block(s, p->blocks[i], gates, stage);
             continue;
         }
-        prepare(i);
         const GateOp& op = ops[i];
-        if (op.kind == GateOp::Noop) continue;
         if (eligible(i)) {
             // consecutive blocks share a pass when their qubits fit one
             // 12-position tile with runs of >= 128 amplitudes or as one
@@ -1401,6 +1464,7 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
             s->apply_op(op, s->amps.as<char>(), s->total());
         }
     }
+    flush_plain();
     if (staged) check_cuda(cudaEventRecord(p->staged, s->stream), "cudaEventRecord");
     p->last_h2d_bytes = staged;
     if (!launched) return;

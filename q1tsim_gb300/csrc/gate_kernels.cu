@@ -18,6 +18,7 @@
 #include "common.cuh"
 #include "df64.cuh"
 #include "kernels.h"
+#include "unit_code.h"
 
 namespace q1g {
 
@@ -128,19 +129,8 @@ k_pair_adj(float2* __restrict__ a, uint64_t units, IndexMap map, Mat2<float2> m)
 // ------------------------------------------------- exact unit shuffles
 //
 // A 2x2 matrix with one entry of 0, +-1 or +-i per row and column (X, Y,
-// CX, CY, CCX, Swap ...) moves and re-signs amplitudes; no arithmetic.
-// Unit code u: 0 -> x, 1 -> i x, 2 -> -x, 3 -> -i x.
-template <typename T>
-__device__ __forceinline__ T unit_times(int u, T x)
-{
-    switch (u) {
-        case 1: return T{-x.y, x.x};
-        case 2: return T{-x.x, -x.y};
-        case 3: return T{x.y, -x.x};
-        default: return x;
-    }
-}
-
+// CX, CY, CCX, Swap ...) moves and re-signs amplitudes; no arithmetic
+// (unit_times, common.cuh).
 // out0 = u0 * x[s0], out1 = u1 * x[s1] (s0 != s1)
 template <typename T, int U, int NZ>
 __global__ void __launch_bounds__(kThreads)
@@ -404,36 +394,6 @@ inline unsigned grid_for(uint64_t units, int per_block)
     return (unsigned)(g ? g : 1);
 }
 
-}  // namespace
-
-namespace {
-// Unit code of (re, im) if it is 1, i, -1 or -i (as unit_times), -1 for 0,
-// -2 otherwise.
-int unit_code(double re, double im)
-{
-    if (re == 0.0 && im == 0.0) return -1;
-    if (re == 1.0 && im == 0.0) return 0;
-    if (re == 0.0 && im == 1.0) return 1;
-    if (re == -1.0 && im == 0.0) return 2;
-    if (re == 0.0 && im == -1.0) return 3;
-    return -2;
-}
-
-// A 2x2 matrix with one unit entry per row and column: (swap, u0, u1).
-bool mono_pair(const double* m, int& swap, int& u0, int& u1)
-{
-    const int c00 = unit_code(m[0], m[1]), c01 = unit_code(m[2], m[3]);
-    const int c10 = unit_code(m[4], m[5]), c11 = unit_code(m[6], m[7]);
-    if (c00 >= 0 && c11 >= 0 && c01 == -1 && c10 == -1) {
-        swap = 0, u0 = c00, u1 = c11;
-        return true;
-    }
-    if (c01 >= 0 && c10 >= 0 && c00 == -1 && c11 == -1) {
-        swap = 1, u0 = c01, u1 = c10;
-        return true;
-    }
-    return false;
-}
 }  // namespace
 
 cudaError_t launch_pair(void* amps, int prec, uint64_t total, const IndexMap& map,

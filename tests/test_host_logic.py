@@ -129,3 +129,8 @@ def test_f16_rounding_and_tensor_core_images(gxx, tmp_path):
     want = vals.astype(np.float16).view(np.uint16)
     assert got.shape == want.shape
     assert np.array_equal(got, want), np.flatnonzero(got != want)[:10]
+
+
+def test_gate_runs_replay_the_sequence(gxx, tmp_path):
+    out = _run(_link_against_library(gxx, tmp_path, "gate_run_check"))
+    assert out.startswith("bad 0"), out
