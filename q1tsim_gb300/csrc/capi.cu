@@ -112,11 +112,14 @@ int q1g_state_from_qubit_coefs(const double* coefs, size_t nr_bits, size_t nr_sh
         }
         auto* s = new q1g_state((int)nr_bits, nr_shots, precision);
         try {
-            s->dscratch.ensure(std::max<size_t>(c.size(), 1) * sizeof(double));
+            // the coefficients, then the kernel's table of the high qubits
+            const size_t cbytes = (c.size() * sizeof(double) + 255) & ~size_t(255);
+            s->dscratch.ensure(std::max<size_t>(cbytes + product_state_tmp_bytes((int)nr_bits), 256));
             s->h2d(s->dscratch.p, c.data(), c.size() * sizeof(double), "upload coefs");
             s->amps.ensure(s->N * s->bsz());
             s->launch("product_state", double(s->N * s->bsz()), [&] {
-                return launch_product_state(s->amps.p, s->prec, (int)nr_bits, s->dscratch.as<double>(), s->stream);
+                return launch_product_state(s->amps.p, s->prec, (int)nr_bits, s->dscratch.as<double>(),
+                                            s->dscratch.as<char>() + cbytes, s->stream);
             });
             s->sync();
             s->sparse = false;

@@ -1,5 +1,6 @@
 // State construction, precision conversion and measurement collapse kernels.
 #include "common.cuh"
+#include "df64.cuh"
 #include "kernels.h"
 #include "sampling.cuh"
 
@@ -41,6 +42,86 @@ __global__ void k_product_state(T* a, int nbits, const double* coefs)
             im = ni;
         }
         a[i] = cmake<T>(re, im);
+    }
+}
+
+// Larger product states: amplitude hi * 2^kProductLow + lo is high[hi] *
+// low[lo], high the product state of the other qubits (k_product_state) and
+// low[] a table that each block builds by doubling.  One complex product per
+// amplitude instead of one per qubit: the n FP64 products were 26.5 ms at 27
+// qubits (complex128), this is 1.0 ms (FP64 pipe, 4 operations per
+// amplitude; the write alone takes 0.32 ms).
+constexpr int kProductLow = 10;
+constexpr int kProductPerThread = (1 << kProductLow) / kThreads;
+// From this size on: below it the two launches cost more than the products.
+constexpr int kProductTwoLevelBits = 15;
+
+__device__ __forceinline__ void product_store(double2* a, double2 h, double2 l)
+{
+    *a = make_double2(h.x * l.x - h.y * l.y, h.x * l.y + h.y * l.x);
+}
+
+struct DfAmp {
+    DF re, im;
+};
+__device__ __forceinline__ DF df_of(double v)
+{
+    const float h = (float)v;
+    return DF{h, (float)(v - (double)h)};
+}
+__device__ __forceinline__ DfAmp df_amp(double2 v) { return DfAmp{df_of(v.x), df_of(v.y)}; }
+// complex64: the product in double-float arithmetic (2^-48), rounded once to
+// FP32 as the FP64 product was; the FP64 pipe would bound it at 0.9 ms at 27
+// qubits, against 0.16 ms for the write
+__device__ __forceinline__ void product_store(float2* a, const DfAmp& h, const DfAmp& l)
+{
+    const DF u[2] = {h.re, DF{-h.im.h, -h.im.l}}, v[2] = {l.re, l.im};
+    const DF w[2] = {h.re, h.im}, z[2] = {l.im, l.re};
+    const DF re = dot<2>(u, v), im = dot<2>(w, z);
+    *a = make_float2(re.h, im.h);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+k_product_rows(T* __restrict__ a, uint64_t rows, const double2* __restrict__ high, int nbits,
+               const double* __restrict__ coefs)
+{
+    constexpr int N = 1 << kProductLow;
+    __shared__ double2 low[N];
+    if (threadIdx.x == 0) low[0] = make_double2(1.0, 0.0);
+    __syncthreads();
+    // the last qubit is the lowest bit: entries of bits 0..b-1 give those of
+    // bit b by its qubit's two coefficients
+    for (int b = 0; b < kProductLow; ++b) {
+        const double* c = coefs + 4 * (nbits - 1 - b);
+        const double2 c0 = make_double2(c[0], c[1]), c1 = make_double2(c[2], c[3]);
+        for (int j = threadIdx.x; j < (1 << b); j += kThreads) {
+            const double2 v = low[j];
+            low[j] = cmul(c0, v);
+            low[j + (1 << b)] = cmul(c1, v);
+        }
+        __syncthreads();
+    }
+    if constexpr (sizeof(T) == sizeof(double2)) {
+        double2 l[kProductPerThread];
+#pragma unroll
+        for (int k = 0; k < kProductPerThread; ++k) l[k] = low[threadIdx.x + k * kThreads];
+        for (uint64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+            const double2 h = high[r];
+#pragma unroll
+            for (int k = 0; k < kProductPerThread; ++k)
+                product_store(a + r * N + threadIdx.x + k * kThreads, h, l[k]);
+        }
+    } else {
+        DfAmp l[kProductPerThread];
+#pragma unroll
+        for (int k = 0; k < kProductPerThread; ++k) l[k] = df_amp(low[threadIdx.x + k * kThreads]);
+        for (uint64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+            const DfAmp h = df_amp(high[r]);
+#pragma unroll
+            for (int k = 0; k < kProductPerThread; ++k)
+                product_store(a + r * N + threadIdx.x + k * kThreads, h, l[k]);
+        }
     }
 }
 
@@ -228,15 +309,36 @@ cudaError_t launch_fill_basis(void* amps, int prec, uint64_t n_amps, const uint6
     return cudaGetLastError();
 }
 
-cudaError_t launch_product_state(void* amps, int prec, int nbits, const double* d_coefs,
-                                 cudaStream_t st)
+uint64_t product_state_tmp_bytes(int nbits)
+{
+    return nbits < kProductTwoLevelBits ? 0 : sizeof(double2) << (nbits - kProductLow);
+}
+
+template <typename T>
+static void product_direct(T* a, int nbits, const double* d_coefs, cudaStream_t st)
 {
     const uint64_t n = uint64_t(1) << nbits;
     const unsigned grid = blocks_for(n, kThreads) > 152 * 64 ? 152 * 64 : blocks_for(n, kThreads);
+    k_product_state<T><<<grid, kThreads, 0, st>>>(a, nbits, d_coefs);
+}
+
+cudaError_t launch_product_state(void* amps, int prec, int nbits, const double* d_coefs, void* tmp, cudaStream_t st)
+{
+    if (nbits < kProductTwoLevelBits) {
+        if (prec == kC128) product_direct((double2*)amps, nbits, d_coefs, st);
+        else product_direct((float2*)amps, nbits, d_coefs, st);
+        return cudaGetLastError();
+    }
+    // qubits 0 .. n-1-kProductLow are the row's bits, in the same order
+    product_direct((double2*)tmp, nbits - kProductLow, d_coefs, st);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const uint64_t rows = uint64_t(1) << (nbits - kProductLow);
+    const unsigned grid = (unsigned)(rows < 152 * 6 ? rows : 152 * 6);
     if (prec == kC128)
-        k_product_state<double2><<<grid, kThreads, 0, st>>>((double2*)amps, nbits, d_coefs);
+        k_product_rows<double2><<<grid, kThreads, 0, st>>>((double2*)amps, rows, (const double2*)tmp, nbits, d_coefs);
     else
-        k_product_state<float2><<<grid, kThreads, 0, st>>>((float2*)amps, nbits, d_coefs);
+        k_product_rows<float2><<<grid, kThreads, 0, st>>>((float2*)amps, rows, (const double2*)tmp, nbits, d_coefs);
     return cudaGetLastError();
 }
 
