@@ -637,16 +637,24 @@ def main():
     plain_kernels = None if args.no_plain else plain_kernel_leg(n, bits, mats, stream, barrier)
 
     # ---- end to end through the public Circuit API (host in, results out)
+    # every step has its own angles, so its matrices are evaluated, lowered and
+    # copied to the device within the timed region
     circ = Circuit(n, n, precision="c64", fusion_width=args.fusion)
-    for g, b in gates:
-        circ.add_gate(g, b)
+    angles = []
+    for nm, par, b in gl:
+        refs = [G.Parameter(v) for v in par]
+        angles += refs
+        circ.add_gate(G.by_name(nm, refs), b)
     circ.measure_all(cbits)
+    step_angles = np.random.default_rng(args.seed + 17).uniform(0.0, 2 * math.pi, (args.steps, len(angles))).tolist()
     del fused
     circ.execute(shots, Rng(args.seed))
     barrier()
     circ.q_state.transfer_bytes(reset=True)
     t0 = time.perf_counter()
     for k in range(args.steps):
+        for ref, v in zip(angles, step_angles[k]):
+            ref.assign(v)
         circ.execute(shots, Rng(args.seed + k))
         _ = circ.cstate()
     barrier()

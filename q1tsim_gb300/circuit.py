@@ -21,6 +21,74 @@ from .vectorstate import Plan, Rng, VectorState
 BASES = ("x", "y", "z")
 
 
+class _SegmentMatrices:
+    """The matrices of a run of gates, row-major (re, im) one after the
+    other.  What does not change between evaluations (the layout, fixed gates
+    and gates with plain values) is worked out once; U3 gates (most of a random
+    circuit) and controlled U1 gates are evaluated together with numpy, with
+    the formulas of gates._u3 (src/gates/u3.rs:74-84) and gates._u1.  A server
+    builds these for every request, under the interpreter lock."""
+
+    def __init__(self, seq):
+        n = len(seq)
+        sizes = np.asarray([1 << (2 * op[1].nr_affected_bits()) for op in seq], dtype=np.int64)
+        offs = np.zeros(n + 1, dtype=np.int64)
+        np.cumsum(sizes, out=offs[1:])
+        self.fixed = np.empty(int(offs[-1]), dtype=np.complex128)
+        self.refs = []        # reference parameters of the U3 and controlled U1 gates
+        self.others = []      # (gate, start, end): other gates that can change
+        u3_rows, self.u3_par, cu1_rows, self.cu1_par = [], [], [], []
+        for i, op in enumerate(seq):
+            g = op[1]
+            tg = type(g)
+            if tg is G._Param and g._fn is G._u3:
+                u3_rows.append(i)
+                self.u3_par.append(g.params)
+                self.refs += g._refs
+            elif tg is G.C and type(g.gate) is G._Param and g.gate._fn is G._u1:
+                cu1_rows.append(i)
+                self.cu1_par.append(g.gate.params[0])
+                self.refs += g.gate._refs
+            elif g.param_key():
+                self.others.append((g, offs[i], offs[i + 1]))
+            else:
+                shared = getattr(g, "_shared_matrix", None)
+                m = shared() if shared is not None else None
+                if m is None:
+                    m = np.asarray(g.matrix(), dtype=np.complex128)
+                self.fixed[offs[i]:offs[i + 1]] = m.ravel()
+        self.u3_at = offs[np.asarray(u3_rows, dtype=np.int64)][:, None] + np.arange(4)
+        self.cu1_at = offs[np.asarray(cu1_rows, dtype=np.int64)][:, None] + np.arange(16)
+
+    def key(self):
+        """The current values of every reference parameter."""
+        return [r.value for r in self.refs], [g.param_key() for g, _, _ in self.others]
+
+    def evaluate(self):
+        out = self.fixed.copy()
+        for g, a, z in self.others:
+            out[a:z] = np.asarray(g.matrix(), dtype=np.complex128).ravel()
+        if self.u3_par:
+            p = np.asarray([[float(v) for v in par] for par in self.u3_par])
+            theta, phi, lmb = p[:, 0], p[:, 1], p[:, 2]
+            c, s = np.cos(0.5 * theta), np.sin(0.5 * theta)
+            pl = phi + lmb
+            m = np.empty((len(p), 4), dtype=np.complex128)
+            m.real[:, 0], m.imag[:, 0] = c, 0.0
+            m.real[:, 1], m.imag[:, 1] = -(s * np.cos(lmb)), -(s * np.sin(lmb))
+            m.real[:, 2], m.imag[:, 2] = s * np.cos(phi), s * np.sin(phi)
+            m.real[:, 3], m.imag[:, 3] = c * np.cos(pl), c * np.sin(pl)
+            out[self.u3_at] = m
+        if self.cu1_par:
+            # C(U1(lmb)) = diag(1, 1, 1, e^(i lmb)) (src/gates/u1.rs:69-84)
+            lmb = np.asarray([float(v) for v in self.cu1_par])
+            m = np.zeros((len(lmb), 16), dtype=np.complex128)
+            m[:, 0] = m[:, 5] = m[:, 10] = 1.0
+            m.real[:, 15], m.imag[:, 15] = np.cos(lmb), np.sin(lmb)
+            out[self.cu1_at] = m
+        return out.view(np.float64)
+
+
 class Circuit:
     def __init__(self, nr_qbits, nr_cbits=0, precision="c128", fusion_width=0):
         """fusion_width: qubits per fused block (0 = one pass per gate, the
@@ -37,7 +105,7 @@ class Circuit:
         self._plans = {}
         self._frozen = None
         self._segs = None
-        self._flats = {}    # segment index -> (gates with reference parameters, their values, matrices)
+        self._flats = {}    # segment index -> [its matrices' evaluator, matrices, the parameter values they are of]
 
     # ------------------------------------------------------------ building
     def _check_qbits(self, qbits):
@@ -73,71 +141,20 @@ class Circuit:
     @staticmethod
     def _flat(seq):
         """The segment's gate matrices, concatenated row-major as (re, im)
-        doubles.  Fixed gates contribute their stored matrices; U3 gates (most
-        of a random circuit) are evaluated together with numpy, with the
-        formulas of gates._u3 (src/gates/u3.rs:74-84).  A server builds these
-        for every request, under the interpreter lock."""
-        n = len(seq)
-        if n == 0:
-            return np.zeros(0)
-        sizes = np.empty(n, dtype=np.int64)
-        parts = [None] * n
-        u3_rows, u3_par, cu1_rows, cu1_par = [], [], [], []
-        for i, op in enumerate(seq):
-            g = op[1]
-            sizes[i] = 1 << (2 * g.nr_affected_bits())
-            tg = type(g)
-            if tg is G._Param and g._fn is G._u3:
-                u3_rows.append(i)
-                u3_par.append([float(p) for p in g.params])
-                continue
-            if tg is G.C and type(g.gate) is G._Param and g.gate._fn is G._u1:
-                cu1_rows.append(i)
-                cu1_par.append(float(g.gate.params[0]))
-                continue
-            shared = getattr(g, "_shared_matrix", None)
-            m = shared() if shared is not None else None
-            parts[i] = m if m is not None else np.asarray(g.matrix(), dtype=np.complex128)
-        offs = np.zeros(n + 1, dtype=np.int64)
-        np.cumsum(sizes, out=offs[1:])
-        out = np.empty(int(offs[-1]), dtype=np.complex128)
-        for i, m in enumerate(parts):
-            if m is not None:
-                out[offs[i]:offs[i + 1]] = m.ravel()
-        if u3_rows:
-            p = np.asarray(u3_par)
-            theta, phi, lmb = p[:, 0], p[:, 1], p[:, 2]
-            c, s = np.cos(0.5 * theta), np.sin(0.5 * theta)
-            pl = phi + lmb
-            m = np.empty((len(u3_rows), 4), dtype=np.complex128)
-            m.real[:, 0], m.imag[:, 0] = c, 0.0
-            m.real[:, 1], m.imag[:, 1] = -(s * np.cos(lmb)), -(s * np.sin(lmb))
-            m.real[:, 2], m.imag[:, 2] = s * np.cos(phi), s * np.sin(phi)
-            m.real[:, 3], m.imag[:, 3] = c * np.cos(pl), c * np.sin(pl)
-            out[offs[np.asarray(u3_rows)][:, None] + np.arange(4)] = m
-        if cu1_rows:
-            # C(U1(lmb)) = diag(1, 1, 1, e^(i lmb)) (src/gates/u1.rs:69-84)
-            lmb = np.asarray(cu1_par)
-            m = np.zeros((len(cu1_rows), 16), dtype=np.complex128)
-            m[:, 0] = m[:, 5] = m[:, 10] = 1.0
-            m.real[:, 15], m.imag[:, 15] = np.cos(lmb), np.sin(lmb)
-            out[offs[np.asarray(cu1_rows)][:, None] + np.arange(16)] = m
-        return out.view(np.float64)
+        doubles."""
+        return _SegmentMatrices(seq).evaluate()
 
     def _flat_current(self, idx, seq):
         """The segment's matrices for this execution.  They are evaluated
         again only when a reference parameter of one of its gates has changed
         (src/gates/parameter.rs:23-75); gates with plain values keep theirs."""
         ent = self._flats.get(idx)
-        if ent is not None:
-            dyn, key, flat = ent
-            now = tuple(v for i in dyn for v in seq[i][1].param_key())
-            if now == key:
-                return flat
-        dyn = [i for i, op in enumerate(seq) if op[1].param_key()]
-        flat = self._flat(seq)
-        self._flats[idx] = (dyn, tuple(v for i in dyn for v in seq[i][1].param_key()), flat)
-        return flat
+        if ent is None:
+            ent = self._flats[idx] = [_SegmentMatrices(seq), None, None]
+        now = ent[0].key()
+        if ent[1] is None or now != ent[2]:
+            ent[1], ent[2] = ent[0].evaluate(), now
+        return ent[1]
 
     @staticmethod
     def _gate(gate, params):

@@ -443,8 +443,7 @@ int q1g_plan_set_gate_kinds(q1g_plan* p, const unsigned char* kinds, size_t ngat
             p->blocks = fuse_runs(p->gate_bits, p->kinds, p->nbits, p->width);
             order_blocks_for_tc_pairs(p->blocks, p->nbits, p->tc_max_high, p->tc_pairs == 5 ? 3 : 2);
         }
-        p->prefix_known = false;
-        p->prefix_plan.reset();
+        p->regrouped();
     });
 }
 
@@ -516,8 +515,7 @@ int q1g_plan_set_tc_tiling(q1g_plan* p, int allow_pairs, int max_high_positions,
         p->tc_slack = conflict_slack;
         if (regroup) order_blocks_for_tc_pairs(p->blocks, p->nbits, p->tc_max_high, p->tc_pairs == 5 ? 3 : 2);
         // the compact prefix plan copies the tiling when it is made
-        p->prefix_known = false;
-        p->prefix_plan.reset();
+        p->regrouped();
     });
 }
 
@@ -526,8 +524,7 @@ int q1g_plan_set_tensor_cores(q1g_plan* p, int enable)
     return guarded([&] {
         need(p, "plan");
         p->tensor_cores = enable != 0;
-        p->prefix_known = false;
-        p->prefix_plan.reset();
+        p->regrouped();
     });
 }
 

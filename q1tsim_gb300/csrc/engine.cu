@@ -8,6 +8,7 @@
 #include "gate_run.h"
 
 #include <algorithm>
+#include <array>
 #include <memory>
 #include <set>
 #include <cmath>
@@ -175,6 +176,12 @@ void q1g_state::ensure_dense()
     sync();
     sparse = false;
     basis.clear();
+}
+
+void q1g_state::clear_error_flag()
+{
+    errbuf.ensure(sizeof(int));
+    check_cuda(cudaMemsetAsync(errbuf.p, 0, sizeof(int), stream), "clear error flag");
 }
 
 void q1g_state::apply_op(const GateOp& op, char* base, uint64_t total_amps)
@@ -688,6 +695,13 @@ void q1g_state::download(double* out, size_t len)
 
 // ---------------------------------------------------------------- plans
 
+void q1g_plan::regrouped()
+{
+    prefix_known = false;
+    prefix_plan.reset();
+    for (auto& l : lowered) l.valid = false;
+}
+
 q1g_plan::~q1g_plan()
 {
     if (staged) {
@@ -742,10 +756,10 @@ constexpr int kHighPosition = 18;
 // pass's tile: 8 amplitudes, 64 bytes.
 constexpr int kMinTripleRunBits = 3;
 
-static TcPass lower_tc_pass(const std::vector<const std::vector<cd>*>& mats,
-                            const std::vector<const std::vector<int>*>& bits, int nbits, uint64_t ncols, int slack,
+static TcPass lower_tc_pass(const std::vector<const std::vector<int>*>& bits, int nbits, uint64_t ncols, int slack,
                             int pair_mode)
 {
+    const size_t nblk = bits.size();
     const bool shuffle = pair_mode == 2;
     TcPass t;
     const std::vector<int> T = tile_positions(bits, nbits);
@@ -765,9 +779,8 @@ static TcPass lower_tc_pass(const std::vector<const std::vector<cd>*>& mats,
             if ((r >> (b - L)) & 1) o |= uint64_t(1) << T[b];
         t.offs.run_off[r] = o;
     }
-    t.offs.nblocks = (uint32_t)mats.size();
-    t.images.assign(mats.size() * kTcImageHalves, 0);
-    for (size_t bi = 0; bi < mats.size(); ++bi) {
+    t.offs.nblocks = (uint32_t)nblk;
+    for (size_t bi = 0; bi < nblk; ++bi) {
         // gate qubits: the block's own, padded from the tile's highest positions
         std::vector<int> gpos = positions_of(*bits[bi], nbits);
         for (int j = 11; (int)gpos.size() < 5; --j)
@@ -775,14 +788,7 @@ static TcPass lower_tc_pass(const std::vector<const std::vector<cd>*>& mats,
         std::vector<int> q;
         for (int p : gpos) q.push_back(nbits - 1 - p);
         std::sort(q.begin(), q.end());   // ascending qubits: q[0] is the matrix MSB
-        const auto m32 = embed_matrix(*mats[bi], *bits[bi], q);
-        std::vector<double> md(2 * 32 * 32);
-        for (size_t e = 0; e < m32.size(); ++e) {
-            md[2 * e] = m32[e].real();
-            md[2 * e + 1] = m32[e].imag();
-        }
-        build_tc_image(md.data(), t.images.data() + bi * kTcImageHalves,
-                       bi + 1 == mats.size() ? kTcLastBScaleLog2 : 0);
+        t.order[bi] = q;
         TcBlockGeom& G = t.offs.blk[bi];
         int r = 0;
         for (int j = 0; j < 12; ++j)
@@ -797,91 +803,70 @@ static TcPass lower_tc_pass(const std::vector<const std::vector<cd>*>& mats,
     }
     t.offs.shuffle = 0;
     int reg1[5];
-    if (mats.size() == 2 && shuffle && tc_shuffle_layout(t.offs.blk[0], t.offs.blk[1], t.offs.swap_lane, reg1)) {
-        // the second block takes the first block's results in registers:
-        // its image in their order, matrix index bit k = tile bit reg1[k]
+    if (nblk == 2 && shuffle && tc_shuffle_layout(t.offs.blk[0], t.offs.blk[1], t.offs.swap_lane, reg1)) {
+        // the second block takes the first block's results in registers, in
+        // their order: matrix index bit k = tile bit reg1[k]
         t.offs.shuffle = 1;
-        std::vector<int> q2(5);
-        for (int k = 0; k < 5; ++k) q2[4 - k] = nbits - 1 - T[reg1[k]];
-        const auto m32 = embed_matrix(*mats[1], *bits[1], q2);
-        std::vector<double> md(2 * 32 * 32);
-        for (size_t e = 0; e < m32.size(); ++e) {
-            md[2 * e] = m32[e].real();
-            md[2 * e + 1] = m32[e].imag();
-        }
-        build_tc_image(md.data(), t.images.data() + kTcImageHalves, kTcLastBScaleLog2);
+        for (int k = 0; k < 5; ++k) t.order[1][4 - k] = nbits - 1 - T[reg1[k]];
     }
     // pair modes 4 and 5: the four-group kernel, every A operand in shared
     // memory (5: three blocks per pass where they fit)
     const bool quad = pair_mode >= 4;
+    // block bi in the gate order a layout chose: matrix index bit k = tile
+    // bit gb[k]
+    auto reorder = [&](size_t bi, const int* gb) {
+        for (int k = 0; k < 5; ++k) t.order[bi][4 - k] = nbits - 1 - T[gb[k]];
+    };
     auto finish = [&] {
         if (!quad) return;
         t.offs.groups = 4;
         t.offs.stage_bytes = (t.offs.stage_bytes + 1023u) & ~1023u;
         // the first block's split is dealt to the threads by a map of its
-        // own, in a gate order that map chooses: its image in that order
+        // own, in a gate order that map chooses
         int gbit0[5];
         tc_split_map(t.offs, gbit0);
-        std::vector<int> q0(5);
-        for (int k = 0; k < 5; ++k) q0[4 - k] = nbits - 1 - T[gbit0[k]];
-        const auto m32 = embed_matrix(*mats[0], *bits[0], q0);
-        std::vector<double> md(2 * 32 * 32);
-        for (size_t e = 0; e < m32.size(); ++e) {
-            md[2 * e] = m32[e].real();
-            md[2 * e + 1] = m32[e].imag();
-        }
-        build_tc_image(md.data(), t.images.data(), mats.size() == 1 ? kTcLastBScaleLog2 : 0);
-    };
-    auto rebuild_image = [&](size_t bi, const int* gb) {
-        // block bi in the gate order a layout chose: matrix index bit k =
-        // tile bit gb[k]
-        std::vector<int> qk(5);
-        for (int k = 0; k < 5; ++k) qk[4 - k] = nbits - 1 - T[gb[k]];
-        const auto m32 = embed_matrix(*mats[bi], *bits[bi], qk);
-        std::vector<double> md(2 * 32 * 32);
-        for (size_t e = 0; e < m32.size(); ++e) {
-            md[2 * e] = m32[e].real();
-            md[2 * e + 1] = m32[e].imag();
-        }
-        build_tc_image(md.data(), t.images.data() + bi * kTcImageHalves,
-                       bi + 1 == mats.size() ? kTcLastBScaleLog2 : 0);
+        reorder(0, gbit0);
     };
     int gbits[kTcMaxBlocks][5];
     // store boxes for the last block's write-back (an unpadded one-box tile)
     std::vector<TcStoreBox> stores;
-    if (quad && mats.size() >= 2 && t.box.usable)
-        stores = tc_store_boxes(T.data(), nbits, ncols, t.offs.blk[mats.size() - 1].jgate[31]);
+    if (quad && nblk >= 2 && t.box.usable)
+        stores = tc_store_boxes(T.data(), nbits, ncols, t.offs.blk[nblk - 1].jgate[31]);
     int store = -1;
-    if (quad && mats.size() >= 2 &&
+    if (quad && nblk >= 2 &&
         tc_chain_layout(t.offs, t.box.usable != 0, slack, gbits, &t.cost, &t.ideal, &stores, &store)) {
         if (t.offs.st_box) t.sbox = stores[(size_t)store].box;
         // the later blocks read the operands the previous block's
         // write-back scattered, in the gate orders the layout chose
-        for (size_t bi = 1; bi < mats.size(); ++bi) rebuild_image(bi, gbits[bi]);
+        for (size_t bi = 1; bi < nblk; ++bi) reorder(bi, gbits[bi]);
         finish();
         return t;
     }
-    if (mats.size() > 2) throw Error(Q1G_ERR_INVALID_ARGUMENT, "a three-block pass needs the four-group kernel");
+    if (nblk > 2) throw Error(Q1G_ERR_INVALID_ARGUMENT, "a three-block pass needs the four-group kernel");
     int gbit1[5];
-    if (mats.size() == 2 && (pair_mode == 3 || quad) && tc_direct_layout(t.offs, t.box.usable != 0, slack, gbit1)) {
+    if (nblk == 2 && (pair_mode == 3 || quad) && tc_direct_layout(t.offs, t.box.usable != 0, slack, gbit1)) {
         // the second block reads the operands the first block's write-back
-        // scattered: its image in the gate order that layout chose, matrix
-        // index bit k = tile bit gbit1[k]
-        std::vector<int> q2(5);
-        for (int k = 0; k < 5; ++k) q2[4 - k] = nbits - 1 - T[gbit1[k]];
-        const auto m32 = embed_matrix(*mats[1], *bits[1], q2);
-        std::vector<double> md(2 * 32 * 32);
-        for (size_t e = 0; e < m32.size(); ++e) {
-            md[2 * e] = m32[e].real();
-            md[2 * e + 1] = m32[e].imag();
-        }
-        build_tc_image(md.data(), t.images.data() + kTcImageHalves, kTcLastBScaleLog2);
+        // scattered, in the gate order that layout chose
+        reorder(1, gbit1);
         finish();
         return t;
     }
     tc_choose_padding(t.offs, t.box.usable != 0, slack);
     finish();
     return t;
+}
+
+// The f16 images of a pass's blocks, one after the other.
+static std::vector<uint16_t> tc_images(const TcPass& t, const std::vector<cd>* const* mats,
+                                       const std::vector<int>* const* bits, int nblk)
+{
+    std::vector<uint16_t> images((size_t)nblk * kTcImageHalves);
+    for (int bi = 0; bi < nblk; ++bi) {
+        const auto m32 = embed_matrix(*mats[bi], *bits[bi], t.order[bi]);
+        build_tc_image(reinterpret_cast<const double*>(m32.data()), images.data() + bi * kTcImageHalves,
+                       bi + 1 == nblk ? kTcLastBScaleLog2 : 0);
+    }
+    return images;
 }
 
 // Whether blocks on these qubit sets could share a tensor-core pass: their
@@ -966,8 +951,9 @@ void order_blocks_for_tc_pairs(std::vector<FusedBlock>& blocks, int nbits, int m
 // A swap-run block (fuse_runs): every gate must be the swap permutation;
 // one permutation pass (swap_run.cu), or the swaps one by one when the
 // state has fewer than 10 qubits.
-template <typename Stage>
-static void run_swap_block(q1g_state* s, const FusedBlock& b, const std::vector<SeqGate>& gates, Stage&& stage)
+template <typename Stage, typename Emit>
+static void lower_swap_block(q1g_state* s, const FusedBlock& b, const std::vector<SeqGate>& gates, Stage&& stage,
+                             Emit&& emit)
 {
     const int n = s->nbits;
     std::vector<int> pa, pb;
@@ -987,14 +973,16 @@ static void run_swap_block(q1g_state* s, const FusedBlock& b, const std::vector<
     if (!swap_run_layout(*t, pa.data(), pb.data(), (int)pa.size(), n, (int)amp_bytes(s->prec))) {
         for (int g : b.gates) {
             const GateOp op = classify(gates[g].mat.data(), 2, gates[g].bits.data(), n);
-            if (op.kind != GateOp::Noop) s->apply_op(op, s->amps.as<char>(), s->total());
+            if (op.kind != GateOp::Noop) emit([op](q1g_state* x) { x->apply_op(op, x->amps.as<char>(), x->total()); });
         }
         return;
     }
     const void* dt = stage(t.get(), sizeof(SwapTile));
-    const uint64_t total = s->total();
-    s->launch("swap_run", 2.0 * total * s->bsz(), [&] {
-        return launch_swap_run(s->amps.p, (int)amp_bytes(s->prec), total, dt, s->sm_count(), s->stream);
+    emit([dt](q1g_state* x) {
+        const uint64_t total = x->total();
+        x->launch("swap_run", 2.0 * total * x->bsz(), [&] {
+            return launch_swap_run(x->amps.p, (int)amp_bytes(x->prec), total, dt, x->sm_count(), x->stream);
+        });
     });
 }
 
@@ -1008,9 +996,9 @@ static bool phase_kernels_take(const q1g_state* s) { return s->prec == kC64 && s
 // log-phases theta_s over its (at most two) qubits contribute, by the Moebius
 // transform, a constant, one linear term per qubit and, for two qubits, the
 // product term, which contains the run's pivot.
-template <typename Stage>
-static void run_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, const std::vector<SeqGate>& gates,
-                            Stage&& stage)
+template <typename Stage, typename Emit>
+static void lower_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, const std::vector<SeqGate>& gates,
+                              Stage&& stage, Emit&& emit)
 {
     const int n = s->nbits;
     const size_t ndiag = b.gates.size() - (b.trailing_pair ? 1 : 0);
@@ -1051,7 +1039,7 @@ static void run_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, cons
     phase_run_tables(n, c, lin0.data(), lin1.data(), tab.data());
     const void* dtab = stage(tab.data(), tab.size() * sizeof(float2));
     int q_pos = -1;
-    double m2[8] = {1, 0, 0, 0, 0, 0, 1, 0};
+    std::array<double, 8> m2 = {1, 0, 0, 0, 0, 0, 1, 0};
     if (b.trailing_pair) {
         const SeqGate& t = gates[b.gates.back()];
         q_pos = n - 1 - t.bits[0];
@@ -1060,9 +1048,12 @@ static void run_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, cons
             m2[2 * e + 1] = t.mat[e].imag();
         }
     }
-    const uint64_t total = s->total();
-    s->launch(b.trailing_pair ? "phase_pair_run_c64" : "phase_run_c64", 2.0 * total * s->bsz(), [&] {
-        return launch_phase_run(s->amps.as<float2>(), total, n, pivot_pos, dtab, q_pos, m2, s->sm_count(), s->stream);
+    emit([=](q1g_state* x) {
+        const uint64_t total = x->total();
+        x->launch(q_pos >= 0 ? "phase_pair_run_c64" : "phase_run_c64", 2.0 * total * x->bsz(), [&] {
+            return launch_phase_run(x->amps.as<float2>(), total, n, pivot_pos, dtab, q_pos, m2.data(), x->sm_count(),
+                                    x->stream);
+        });
     });
 }
 
@@ -1070,13 +1061,15 @@ static void run_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, cons
 // (gate_run.h).  A pass of one op, or one whose ops together touch less than
 // the state where that is what costs (a state beyond the L2: two CX read and
 // write half of it each), goes gate by gate.
-template <typename Stage>
-static void run_plain_gates(q1g_state* s, const std::vector<GateOp>& ops, Stage&& stage)
+template <typename Stage, typename Emit>
+static void lower_plain_gates(q1g_state* s, const std::vector<GateOp>& ops, Stage&& stage, Emit&& emit)
 {
     const uint64_t total = s->total();
     std::vector<const GateOp*> list;
     for (const GateOp& op : ops) list.push_back(&op);
-    auto one = [&](const GateOp& op) { s->apply_op(op, s->amps.as<char>(), total); };
+    auto one = [&](const GateOp& op) {
+        emit([op](q1g_state* x) { x->apply_op(op, x->amps.as<char>(), x->total()); });
+    };
     if (ops.size() < 2) {
         for (const GateOp& op : ops) one(op);
         return;
@@ -1093,11 +1086,24 @@ static void run_plain_gates(q1g_state* s, const std::vector<GateOp>& ops, Stage&
         table.clear();
         for (int i : pass.ops) table.push_back(make_run_op(ops[i], pass.tile));
         const RunOp* d = static_cast<const RunOp*>(stage(table.data(), table.size() * sizeof(RunOp)));
-        s->launch(name, 2.0 * total * s->bsz(), [&] {
-            return launch_gate_run(s->amps.p, s->prec, total, pass.tile, d, (int)table.size(), s->fp64_exact,
-                                   s->stream);
+        emit([name, tile = pass.tile, d, n = (int)table.size()](q1g_state* x) {
+            x->launch(name, 2.0 * x->total() * x->bsz(), [&] {
+                return launch_gate_run(x->amps.p, x->prec, x->total(), tile, d, n, x->fp64_exact, x->stream);
+            });
         });
     }
+}
+
+// Device bytes of a block's staged data at most: a run table entry per gate
+// (and its alignment), a swap tile or phase tables, a dense matrix in one of
+// its forms, or a tensor-core image.
+static size_t staging_bytes(const q1g_plan* p, const FusedBlock& b)
+{
+    size_t n = b.gates.size() * 512;
+    if (b.phase_run || b.swap_run || b.qubits.size() >= 3) n += 32768;
+    else n += 2048;
+    (void)p;
+    return n;
 }
 
 // Positions a plan may leave out of its start-of-run subspace: the compact
@@ -1196,12 +1202,11 @@ static size_t run_subspace_prefix(q1g_plan* p, q1g_state* s, const double* mats,
     return p->prefix_len;
 }
 
-void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subspace_prefix)
+// Lowers the plan's blocks from `first` on into L and launches each pass as
+// it is ready, so the host work of pass i+1 (block product, classification,
+// tensor-core image) runs while the device executes pass i.
+static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t first, q1g_plan::Lowered& L)
 {
-    if (n != p->mat_doubles)
-        throw Error(Q1G_ERR_INVALID_ARGUMENT, "expected " + std::to_string(p->mat_doubles) + " matrix doubles");
-    if (s->nbits != p->nbits)
-        throw Error(Q1G_ERR_INVALID_ARGUMENT, "plan and state differ in qubit count");
     const size_t ng = p->gate_bits.size();
     std::vector<SeqGate> gates(ng);
     for (size_t g = 0; g < ng; ++g) {
@@ -1214,9 +1219,6 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
     }
     const bool use_tc = s->prec == kC64 && s->nbits >= 12 && p->tensor_cores;
     const size_t nb = p->blocks.size();
-    // Blocks are lowered one pass ahead of the launches, so the host work of
-    // pass i+1 (block product, classification, tensor-core image) runs while
-    // the device executes pass i.
     std::vector<GateOp> ops(nb);
     std::vector<std::vector<cd>> bmats(nb);
     std::vector<std::vector<int>> bbits(nb);
@@ -1234,47 +1236,28 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
         ops[bi] = classify(bmats[bi].data(), (int)bbits[bi].size(), bbits[bi].data(), s->nbits);
         ready[bi] = 1;
     };
-    // The lowering of a tensor-core pass (tile geometry, padding and the f16
-    // images) is kept with the plan, keyed by its first block and block count
-    // and checked against the blocks' matrices and qubits and the state's
-    // shape: a circuit run again builds no images (about 50 us per block on
-    // the host, which small states do not hide behind their passes).
-    auto lower_tc_cached = [&](size_t i, int nblk) -> TcPass {
-        if (p->tc_memo.size() != kTcMaxBlocks * nb) p->tc_memo.assign(kTcMaxBlocks * nb, TcPassMemo{});
-        TcPassMemo& e = p->tc_memo[kTcMaxBlocks * i + (size_t)(nblk - 1)];
-        const int variant = 8 * p->tc_slack + p->tc_pairs;
-        bool hit = e.nblocks == nblk && e.nbits == s->nbits && e.ncols == s->ncols && e.slack == variant;
-        for (int j = 0; hit && j < nblk; ++j) hit = e.bits[j] == bbits[i + j] && e.mats[j] == bmats[i + j];
-        if (!hit) {
-            if (nblk == 3) {
-                e.pass = lower_tc_pass({&bmats[i], &bmats[i + 1], &bmats[i + 2]},
-                                       {&bbits[i], &bbits[i + 1], &bbits[i + 2]}, s->nbits, s->ncols, p->tc_slack,
-                                       p->tc_pairs);
-            } else if (nblk == 2) {
-                e.pass = lower_tc_pass({&bmats[i], &bmats[i + 1]}, {&bbits[i], &bbits[i + 1]}, s->nbits, s->ncols,
-                                       p->tc_slack, p->tc_pairs);
-                if ((e.pass.offs.shuffle || e.pass.offs.direct) && e.pass.offs.pad_shift < 31) {
-                    // the shuffled or direct row layout needs padding (bank
-                    // conflicts); the staged one, free to order its rows,
-                    // may not: one tensor-map copy per tile is kept if it can
-                    TcPass staged =
-                        lower_tc_pass({&bmats[i], &bmats[i + 1]}, {&bbits[i], &bbits[i + 1]}, s->nbits, s->ncols,
-                                      p->tc_slack, 1);
-                    if (staged.offs.pad_shift >= 31) e.pass = std::move(staged);
-                }
-            } else
-                e.pass = lower_tc_pass({&bmats[i]}, {&bbits[i]}, s->nbits, s->ncols, p->tc_slack,
-                                       p->tc_pairs >= 4 ? 4 : 1);
-            e.nblocks = nblk;
-            e.slack = variant;
-            e.nbits = s->nbits;
-            e.ncols = s->ncols;
-            for (int j = 0; j < nblk; ++j) {
-                e.bits[j] = bbits[i + j];
-                e.mats[j] = bmats[i + j];
-            }
+    // The layout of a tensor-core pass of nblk blocks from block i on
+    auto layout = [&](size_t i, int nblk) -> std::shared_ptr<const TcPass> {
+        std::vector<int> key = {s->nbits, (int)s->ncols, p->tc_slack, p->tc_pairs, nblk};
+        std::vector<const std::vector<int>*> bits;
+        for (int j = 0; j < nblk; ++j) {
+            bits.push_back(&bbits[i + j]);
+            key.push_back(-1);
+            key.insert(key.end(), bbits[i + j].begin(), bbits[i + j].end());
         }
-        return e.pass;
+        auto& e = p->tc_layouts[key];
+        if (e) return e;
+        auto pass = std::make_shared<TcPass>(lower_tc_pass(bits, s->nbits, s->ncols, p->tc_slack,
+                                                           nblk > 1 ? p->tc_pairs : p->tc_pairs >= 4 ? 4 : 1));
+        if (nblk == 2 && (pass->offs.shuffle || pass->offs.direct) && pass->offs.pad_shift < 31) {
+            // the shuffled or direct row layout needs padding (bank
+            // conflicts); the staged one, free to order its rows, may not:
+            // one tensor-map copy per tile is kept if it can
+            TcPass staged = lower_tc_pass(bits, s->nbits, s->ncols, p->tc_slack, 1);
+            if (staged.offs.pad_shift >= 31) *pass = std::move(staged);
+        }
+        e = std::move(pass);
+        return e;
     };
     // tensor-core eligible: dense blocks of >= 3 target qubits
     auto eligible = [&](size_t bi) {
@@ -1283,40 +1266,42 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
         return use_tc && ops[bi].kind == GateOp::Dense && ops[bi].t >= 3 && bbits[bi].size() <= 5 &&
                tc_block_bounded(bmats[bi].data(), 1 << bbits[bi].size());
     };
-    double max_norm = 0.0;
-    for (double v : s->norms) max_norm = std::max(max_norm, v);
     // Staging: every pass uploads its matrix or tensor-core image from its own
-    // slice of one pinned buffer (at most 32 KB per block).
+    // slice of one pinned buffer into its own slice of L's device buffer.
+    // Nothing may still read that buffer: earlier launches on this stream
+    // precede the copies, those on others are waited for.
     if (p->staged) check_cuda(cudaEventSynchronize(p->staged), "plan staging wait");
     else check_cuda(cudaEventCreateWithFlags(&p->staged, cudaEventDisableTiming), "cudaEventCreate");
-    // (plain gates 512 bytes each: a run table entry and its alignment)
-    const size_t staging = std::max<size_t>(nb, 1) * 32768 + ng * 512;
+    if (L.several_streams || (L.stream && L.stream != s->stream)) check_cuda(cudaDeviceSynchronize(), "plan upload wait");
+    L.several_streams = false;
+    L.stream = s->stream;
+    L.launches.clear();
+    L.tensor_cores = false;
+    size_t staging = 256;
+    for (const auto& b : p->blocks) staging += staging_bytes(p, b);
     p->hmats.ensure(staging);
-    p->dmats.ensure(staging);
+    L.dmats.ensure(staging);
     size_t staged = 0;
     auto stage = [&](const void* src, size_t sz) -> const void* {
+        if (staged + sz > staging) throw Error(Q1G_ERR_DEVICE, "plan staging buffer too small");
         char* h = p->hmats.as<char>() + staged;
-        char* d = p->dmats.as<char>() + staged;
+        char* d = L.dmats.as<char>() + staged;
         std::memcpy(h, src, sz);
         s->h2d(d, h, sz, "upload plan matrix");
         staged += (sz + 255) & ~size_t(255);
         return d;
     };
-    bool launched = false, any_tc = false;
-    auto begin = [&] {
-        if (!launched) s->ensure_dense();
-        launched = true;
+    auto emit = [&](std::function<void(q1g_state*)> f) {
+        if (L.launches.empty()) s->ensure_dense();
+        f(s);
+        L.launches.push_back(std::move(f));
     };
-    const size_t first = (subspace_prefix && s->sparse && s->ncols == 1 && s->basis.size() == 1)
-                             ? run_subspace_prefix(p, s, mats, n)
-                             : 0;
     // plain gates (pairs and phases) gathered until another kind of block
     // comes, then grouped into tile passes
     std::vector<GateOp> plain;
     auto flush_plain = [&] {
         if (plain.empty()) return;
-        begin();
-        run_plain_gates(s, plain, stage);
+        lower_plain_gates(s, plain, stage, emit);
         plain.clear();
     };
     for (size_t i = first; i < nb; ++i) {
@@ -1328,8 +1313,7 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
                     plain.push_back(std::move(op));
                 } else {
                     flush_plain();
-                    begin();
-                    s->apply_op(op, s->amps.as<char>(), s->total());
+                    emit([op](q1g_state* x) { x->apply_op(op, x->amps.as<char>(), x->total()); });
                 }
             }
             continue;
@@ -1344,13 +1328,11 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
         }
         flush_plain();
         if (p->blocks[i].phase_run) {
-            begin();
-            run_phase_block(p, s, p->blocks[i], gates, stage);
+            lower_phase_block(p, s, p->blocks[i], gates, stage, emit);
             continue;
         }
         if (p->blocks[i].swap_run) {
-            begin();
-            run_swap_block(s, p->blocks[i], gates, stage);
+            lower_swap_block(s, p->blocks[i], gates, stage, emit);
             continue;
         }
         const GateOp& op = ops[i];
@@ -1359,7 +1341,7 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
             // 12-position tile with runs of >= 128 amplitudes or as one
             // tensor-map box: up to three in the four-group kernel's direct
             // chain in pair mode 5, else two
-            TcPass t;
+            std::shared_ptr<const TcPass> t;
             int group = 1;
             // -1: blocks i .. i+k-1 do not fit one tile; else its run bits
             auto fits = [&](int k) {
@@ -1382,7 +1364,7 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
             if (p->tc_pairs == 5 && i + 2 < nb && eligible(i + 1) && eligible(i + 2)) {
                 const int L3 = fits(3);
                 if (L3 >= 0) {
-                    t = lower_tc_cached(i, 3);
+                    t = layout(i, 3);
                     // short runs only as one unpadded tensor-map copy; a
                     // third block only where the tile's runs are at least
                     // 64 bytes (a copy of 16- or 32-byte runs wastes DRAM
@@ -1390,37 +1372,41 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
                     // the layout keeps the bank wavefronts within twice the
                     // minimum (a conflicted write-back costs more than the
                     // saved pass)
-                    if ((L3 >= kMinTcRunBits || t.offs.pad_shift >= 31) && L3 >= kMinTripleRunBits &&
-                        t.cost <= 2 * t.ideal)
+                    if ((L3 >= kMinTcRunBits || t->offs.pad_shift >= 31) && L3 >= kMinTripleRunBits &&
+                        t->cost <= 2 * t->ideal)
                         group = 3;
                 }
             }
             if (group == 1 && p->tc_pairs && i + 1 < nb && eligible(i + 1)) {
                 const int L2 = fits(2);
                 if (L2 >= 0) {
-                    t = lower_tc_cached(i, 2);
-                    if (L2 >= kMinTcRunBits || t.offs.pad_shift >= 31) group = 2;
+                    t = layout(i, 2);
+                    if (L2 >= kMinTcRunBits || t->offs.pad_shift >= 31) group = 2;
                 }
             }
-            if (group == 1) t = lower_tc_cached(i, 1);
-            begin();
-            if (!any_tc) {
-                s->errbuf.ensure(sizeof(int));
-                check_cuda(cudaMemsetAsync(s->errbuf.p, 0, sizeof(int), s->stream), "clear error flag");
-                any_tc = true;
+            if (group == 1) t = layout(i, 1);
+            if (!L.tensor_cores) {
+                s->clear_error_flag();
+                L.tensor_cores = true;
             }
-            tc_operand_scales(max_norm, t.offs);
-            const void* img = stage(t.images.data(), t.images.size() * sizeof(uint16_t));
-            const uint64_t total = s->total();
-            s->launch("fused_tc_c64", 2.0 * total * s->bsz(), [&] {
-                return launch_fused_tc(s->amps.as<float2>(), total >> 12, t.tilemap, t.offs, t.box, img,
-                                       s->errbuf.as<int>(), s->sm_count(), s->stream, s->tc_wait_ns,
-                                       t.offs.st_box ? &t.sbox : nullptr);
+            const std::vector<cd>* gm[kTcMaxBlocks];
+            const std::vector<int>* gq[kTcMaxBlocks];
+            for (int j = 0; j < group; ++j) gm[j] = &bmats[i + j], gq[j] = &bbits[i + j];
+            const std::vector<uint16_t> images = tc_images(*t, gm, gq, group);
+            const void* img = stage(images.data(), images.size() * sizeof(uint16_t));
+            emit([t, img](q1g_state* x) {
+                TcOffsets offs = t->offs;
+                tc_operand_scales(*std::max_element(x->norms.begin(), x->norms.end()), offs);
+                const uint64_t total = x->total();
+                x->launch("fused_tc_c64", 2.0 * total * x->bsz(), [&] {
+                    return launch_fused_tc(x->amps.as<float2>(), total >> 12, t->tilemap, offs, t->box, img,
+                                           x->errbuf.as<int>(), x->sm_count(), x->stream, x->tc_wait_ns,
+                                           offs.st_box ? &t->sbox : nullptr);
+                });
             });
             i += (size_t)(group - 1);   // the next blocks rode in this pass
         } else if (op.kind == GateOp::Dense &&
                    dense_tiled_applies(s->prec, s->nbits, op.t, op.map, s->fp64_exact)) {
-            begin();
             const size_t d2 = op.dense.size();
             std::vector<double> v(2 * d2);
             for (size_t e = 0; e < d2; ++e) {
@@ -1430,14 +1416,13 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
             std::vector<unsigned char> img(dense_tiled_matrix_bytes(s->prec, op.t));
             dense_tiled_matrix(s->prec, op.t, v.data(), img.data());
             const void* dm = stage(img.data(), img.size());
-            const uint64_t total = s->total();
-            s->launch(s->prec == kC128 ? "dense_tiled_c128" : "dense_tiled_c64", 2.0 * s->bsz() * op.touched(total),
-                      [&] {
-                          return launch_dense_tiled(s->amps.p, s->prec, total, s->nbits, op.map, op.offs, op.t, dm,
-                                                    s->sm_count(), s->stream);
-                      });
+            emit([map = op.map, offs = op.offs, t = op.t, touched = op.touched(s->total()), dm](q1g_state* x) {
+                x->launch(x->prec == kC128 ? "dense_tiled_c128" : "dense_tiled_c64", 2.0 * x->bsz() * touched, [&] {
+                    return launch_dense_tiled(x->amps.p, x->prec, x->total(), x->nbits, map, offs, t, dm,
+                                              x->sm_count(), x->stream);
+                });
+            });
         } else if (op.kind == GateOp::Dense) {
-            begin();
             const size_t d2 = op.dense.size();
             const void* dm;
             if (s->prec == kC128) {
@@ -1455,20 +1440,61 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
                 }
                 dm = stage(v.data(), v.size() * sizeof(float));
             }
-            const uint64_t total = s->total();
-            s->launch(s->prec == kC128 ? "dense_c128" : "dense_c64", 2.0 * s->bsz() * op.touched(total), [&] {
-                return launch_dense(s->amps.p, s->prec, total, op.map, op.offs, op.t, dm, s->stream);
+            emit([map = op.map, offs = op.offs, t = op.t, touched = op.touched(s->total()), dm](q1g_state* x) {
+                x->launch(x->prec == kC128 ? "dense_c128" : "dense_c64", 2.0 * x->bsz() * touched, [&] {
+                    return launch_dense(x->amps.p, x->prec, x->total(), map, offs, t, dm, x->stream);
+                });
             });
         } else {
-            begin();
-            s->apply_op(op, s->amps.as<char>(), s->total());
+            emit([op](q1g_state* x) { x->apply_op(op, x->amps.as<char>(), x->total()); });
         }
     }
     flush_plain();
-    if (staged) check_cuda(cudaEventRecord(p->staged, s->stream), "cudaEventRecord");
-    p->last_h2d_bytes = staged;
-    if (!launched) return;
-    if (any_tc) {
+    check_cuda(cudaEventRecord(p->staged, s->stream), "cudaEventRecord");
+}
+
+void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subspace_prefix)
+{
+    if (n != p->mat_doubles)
+        throw Error(Q1G_ERR_INVALID_ARGUMENT, "expected " + std::to_string(p->mat_doubles) + " matrix doubles");
+    if (s->nbits != p->nbits)
+        throw Error(Q1G_ERR_INVALID_ARGUMENT, "plan and state differ in qubit count");
+    const size_t first = (subspace_prefix && s->sparse && s->ncols == 1 && s->basis.size() == 1)
+                             ? run_subspace_prefix(p, s, mats, n)
+                             : 0;
+    q1g_plan::Lowered& L = p->lowered[first > 0];
+    const int tiling[4] = {p->tensor_cores, p->tc_pairs, p->tc_max_high, p->tc_slack};
+    const bool same = L.valid && L.prec == s->prec && L.fp64_exact == s->fp64_exact && L.ncols == s->ncols &&
+                      L.first == first && std::memcmp(L.tiling, tiling, sizeof tiling) == 0 &&
+                      std::memcmp(L.mats.data(), mats, n * sizeof(double)) == 0;
+    if (same) {
+        if (!L.launches.empty()) s->ensure_dense();
+        if (L.tensor_cores) s->clear_error_flag();
+        if (L.stream != s->stream) {
+            // uploaded on another stream
+            check_cuda(cudaStreamWaitEvent(s->stream, p->staged, 0), "plan upload wait");
+            L.several_streams = true;
+            L.stream = s->stream;
+        }
+        for (auto& f : L.launches) f(s);
+    } else {
+        L.valid = false;
+        try {
+            lower_and_run(p, s, mats, first, L);
+        } catch (...) {
+            // copies out of the staging buffer may be under way
+            cudaStreamSynchronize(s->stream);
+            throw;
+        }
+        L.prec = s->prec;
+        L.fp64_exact = s->fp64_exact;
+        L.ncols = s->ncols;
+        L.first = first;
+        std::copy(tiling, tiling + 4, L.tiling);
+        L.mats.assign(mats, mats + n);
+        L.valid = true;
+    }
+    if (L.tensor_cores) {
         // the tensor-core passes' bounded waits: report an expiry now
         s->hstage.ensure(sizeof(int));
         int* h_flag = s->hstage.as<int>();

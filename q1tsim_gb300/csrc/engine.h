@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <exception>
+#include <functional>
 #include <utility>
 #include <map>
 #include <memory>
@@ -178,6 +179,7 @@ struct q1g_state {
     void collect_profile();
 
     void ensure_dense();
+    void clear_error_flag();               // of the tensor-core passes
     void settle_norms();
     std::vector<double> measure_norms();   // each column's squared norm, FP64, now
     void apply_op(const q1g::GateOp& op, char* base, uint64_t total_amps);
@@ -197,27 +199,19 @@ struct q1g_state {
 };
 
 namespace q1g {
-// Tensor-core lowering of a pass: one or two fused blocks (each <= 5
+// Tensor-core lowering of a pass: one to three fused blocks (each <= 5
 // qubits) whose positions fit in one 12-position tile.  Each block is padded
 // with untouched tile positions to five gate positions; its other seven tile
-// positions are its rows.
+// positions are its rows.  It depends on the blocks' qubits alone: a plan
+// keeps one per list of them (tc_layouts), whatever the matrices.
 struct TcPass {
     IndexMap tilemap{};
     TcOffsets offs{};
     TcTileBox box{};                // the tile as a tensor-map box
-    std::vector<uint16_t> images;   // nblocks x kTcImageHalves f16
+    // each block's five qubits in its image's order (first = matrix MSB)
+    std::vector<int> order[kTcMaxBlocks];
     long cost = 0, ideal = 0;       // the layout's predicted bank wavefronts per warp (chain layouts)
     TcTileBox sbox{};               // the storers' box when offs.st_box
-};
-// A pass's lowering kept by its plan, with what it was made from.
-struct TcPassMemo {
-    int nblocks = 0;
-    int nbits = -1;
-    int slack = 0;          // 8 x conflict slack + pair mode the lowering was made for
-    uint64_t ncols = 0;
-    std::vector<int> bits[kTcMaxBlocks];
-    std::vector<std::complex<double>> mats[kTcMaxBlocks];
-    TcPass pass;
 };
 }  // namespace q1g
 
@@ -238,7 +232,9 @@ struct q1g_plan {
     size_t prefix_len = 0;
     uint64_t prefix_mask = 0;
     std::unique_ptr<q1g_plan> prefix_plan;
-    std::vector<q1g::TcPassMemo> tc_memo;   // by 3 * first block + block count - 1 (plan_run)
+    // Layouts of tensor-core passes, keyed by the state's shape, the tiling
+    // and the blocks' qubits (plan_run).
+    std::map<std::vector<int>, std::shared_ptr<const q1g::TcPass>> tc_layouts;
     // Tensor-core tiling (q1g_plan_set_tc_tiling, tuned by autotune.py):
     // whether two blocks may share a pass (0 no; 1 the second block reads
     // the first's results from the staged tile; 2 from registers, by warp
@@ -252,9 +248,28 @@ struct q1g_plan {
     int tc_max_high = 8;
     int tc_slack = 4;
     q1g::HostBuf hmats;            // pinned staging of dense matrices
-    q1g::DevBuf dmats;
     cudaEvent_t staged = nullptr;  // last upload of hmats finished
-    size_t last_h2d_bytes = 0;     // matrices uploaded by the last run
+    // The launches of a run, kept with the matrices that they were made from
+    // and uploaded: a run with the same matrices (compared byte by byte) on a
+    // state of the same shape makes them again without lowering anything.
+    // Two of them: from the plan's start, and from behind its prefix.
+    struct Lowered {
+        bool valid = false;
+        int prec = -1;
+        bool fp64_exact = false;
+        uint64_t ncols = 0;
+        size_t first = 0;
+        int tiling[4] = {0, 0, 0, 0};     // tensor_cores, tc_pairs, tc_max_high, tc_slack
+        std::vector<double> mats;
+        q1g::DevBuf dmats;                // what the launches read
+        bool tensor_cores = false;        // some launch runs on them
+        cudaStream_t stream = nullptr;    // of the last run
+        bool several_streams = false;     // since the upload
+        std::vector<std::function<void(q1g_state*)>> launches;
+    };
+    Lowered lowered[2];
+    // The grouping changed: nothing made from it holds any more.
+    void regrouped();
     ~q1g_plan();
 };
 

@@ -1916,24 +1916,30 @@ void build_tc_image(const double* m, uint16_t* image, int scale_log2)
     // at chunk position j ^ (r & 7).  Entries below f16's normal range keep
     // their remainder in B_lo' (scaled by 2^11), to 2^-35 absolute.
     const double bs = std::ldexp(1.0, scale_log2);
+    // hi and lo bits of v and of -v (rounding is symmetric; a remainder of
+    // exactly 0 is +0 for both)
+    auto split = [](double v, uint16_t (&b)[2][2]) {
+        double hi = 0.0, lo = 0.0;
+        b[0][0] = host_f16_bits(v, &hi);
+        const double r = (v - hi) * 2048.0;
+        b[0][1] = host_f16_bits(r, &lo);
+        b[1][0] = b[0][0] ^ 0x8000u;
+        b[1][1] = r == 0.0 ? 0 : b[0][1] ^ 0x8000u;
+    };
+    auto put = [&](int n, int k, const uint16_t (&b)[2]) {
+        const size_t off = (size_t)(n >> 3) * 512 + (size_t)(n & 7) * 64 + (size_t)(((k >> 3) ^ (n & 7)) << 3) + (k & 7);
+        image[off] = b[0];
+        image[off + 8 * 512] = b[1];     // row 64 + n
+    };
     for (int gp = 0; gp < 32; ++gp)
         for (int g = 0; g < 32; ++g) {
-            const double re = m[2 * (gp * 32 + g)], im = m[2 * (gp * 32 + g) + 1];
-            const double rv[2][2] = {{re, -im}, {im, re}};
-            for (int cp = 0; cp < 2; ++cp)
-                for (int c = 0; c < 2; ++c) {
-                    const int n = 2 * gp + cp, k = 2 * g + c;
-                    const double v = rv[cp][c] * bs;
-                    double hi = 0.0, lo = 0.0;
-                    const uint16_t hb = host_f16_bits(v, &hi);
-                    const uint16_t lb = host_f16_bits((v - hi) * 2048.0, &lo);
-                    for (int half = 0; half < 2; ++half) {
-                        const int row = n + 64 * half;
-                        const size_t off = (size_t)(row >> 3) * 1024 + (size_t)(row & 7) * 128 +
-                                           (size_t)(((k >> 3) ^ (row & 7)) << 4) + (size_t)(k & 7) * 2;
-                        image[off / 2] = half ? lb : hb;
-                    }
-                }
+            uint16_t re[2][2], im[2][2];
+            split(m[2 * (gp * 32 + g)] * bs, re);
+            split(m[2 * (gp * 32 + g) + 1] * bs, im);
+            put(2 * gp, 2 * g, re[0]);
+            put(2 * gp, 2 * g + 1, im[1]);
+            put(2 * gp + 1, 2 * g, im[0]);
+            put(2 * gp + 1, 2 * g + 1, re[0]);
         }
 }
 

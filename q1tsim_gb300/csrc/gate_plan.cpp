@@ -2,6 +2,7 @@
 #include "gate_plan.h"
 
 #include <algorithm>
+#include <cmath>
 #include <stdexcept>
 
 #include "engine.h"
@@ -68,8 +69,10 @@ GateOp classify(const cd* mat, int k, const int* bits, int nbits)
 
     const int tdim = 1 << t;
     std::vector<cd> G((size_t)tdim * tdim);
+    std::vector<int> full(tdim);
+    for (int r = 0; r < tdim; ++r) full[r] = full_index(r);
     for (int r = 0; r < tdim; ++r)
-        for (int c = 0; c < tdim; ++c) G[(size_t)r * tdim + c] = M(full_index(r), full_index(c));
+        for (int c = 0; c < tdim; ++c) G[(size_t)r * tdim + c] = M(full[r], full[c]);
 
     std::vector<int> nonfixed;
     for (int s = 0; s < tdim; ++s) {
@@ -142,13 +145,18 @@ std::vector<cd> embed_matrix(const std::vector<cd>& mat, const std::vector<int>&
 std::vector<cd> block_matrix(const FusedBlock& b, const std::vector<SeqGate>& gates)
 {
     // acc = G_last ... G_first, each gate applied to the rows of acc as a
-    // k-qubit operator on its bits (32 * 2^k multiply-adds per column, not a
-    // dense product with the embedded matrix).
+    // k-qubit operator on its bits.  Real and imaginary parts in planes, so
+    // that the loops over a row's columns vectorise; zero coefficients of
+    // finite gates are skipped (a CX only moves rows).
     const int m = (int)b.qubits.size();
     const int dim = 1 << m;
-    std::vector<double> acc(2 * (size_t)dim * dim, 0.0);   // row-major (re, im)
-    for (int i = 0; i < dim; ++i) acc[2 * ((size_t)i * dim + i)] = 1.0;
-    double vin[2 * 32], vout[2 * 32];
+    std::vector<double> acc(2 * (size_t)dim * dim, 0.0), tmp(2 * (size_t)dim * dim);
+    double* const are = acc.data();
+    double* const aim = are + (size_t)dim * dim;
+    for (int i = 0; i < dim; ++i) are[(size_t)i * dim + i] = 1.0;
+    bool finite = true;
+    for (int gi : b.gates)
+        for (const cd& v : gates[gi].mat) finite = finite && std::isfinite(v.real()) && std::isfinite(v.imag());
     int rowof[32];
     for (int gi : b.gates) {
         const auto& g = gates[gi];
@@ -166,34 +174,35 @@ std::vector<cd> block_matrix(const FusedBlock& b, const std::vector<SeqGate>& ga
             rowof[gs] = r;
         }
         const double* gm = reinterpret_cast<const double*>(g.mat.data());
+        double* const tre = tmp.data();
+        double* const tim = tre + (size_t)gdim * dim;
         for (int base = 0; base < dim; ++base) {
             if (base & gmask) continue;
-            for (int c = 0; c < dim; ++c) {
+            for (int go = 0; go < gdim; ++go) {
+                double* __restrict__ re = tre + (size_t)go * dim;
+                double* __restrict__ im = tim + (size_t)go * dim;
+                std::fill(re, re + dim, 0.0);
+                std::fill(im, im + dim, 0.0);
+                const double* row = gm + 2 * (size_t)go * gdim;
                 for (int gs = 0; gs < gdim; ++gs) {
-                    const double* a = &acc[2 * ((size_t)(base | rowof[gs]) * dim + c)];
-                    vin[2 * gs] = a[0];
-                    vin[2 * gs + 1] = a[1];
-                }
-                for (int go = 0; go < gdim; ++go) {
-                    double re = 0.0, im = 0.0;
-                    const double* row = gm + 2 * (size_t)go * gdim;
-                    for (int gs = 0; gs < gdim; ++gs) {
-                        re += row[2 * gs] * vin[2 * gs] - row[2 * gs + 1] * vin[2 * gs + 1];
-                        im += row[2 * gs] * vin[2 * gs + 1] + row[2 * gs + 1] * vin[2 * gs];
+                    const double mr = row[2 * gs], mi = row[2 * gs + 1];
+                    if (finite && mr == 0.0 && mi == 0.0) continue;
+                    const double* vr = are + (size_t)(base | rowof[gs]) * dim;
+                    const double* vi = aim + (size_t)(base | rowof[gs]) * dim;
+                    for (int c = 0; c < dim; ++c) {
+                        re[c] += mr * vr[c] - mi * vi[c];
+                        im[c] += mr * vi[c] + mi * vr[c];
                     }
-                    vout[2 * go] = re;
-                    vout[2 * go + 1] = im;
                 }
-                for (int go = 0; go < gdim; ++go) {
-                    double* a = &acc[2 * ((size_t)(base | rowof[go]) * dim + c)];
-                    a[0] = vout[2 * go];
-                    a[1] = vout[2 * go + 1];
-                }
+            }
+            for (int go = 0; go < gdim; ++go) {
+                std::copy_n(tre + (size_t)go * dim, dim, are + (size_t)(base | rowof[go]) * dim);
+                std::copy_n(tim + (size_t)go * dim, dim, aim + (size_t)(base | rowof[go]) * dim);
             }
         }
     }
     std::vector<cd> out((size_t)dim * dim);
-    for (size_t e = 0; e < out.size(); ++e) out[e] = cd(acc[2 * e], acc[2 * e + 1]);
+    for (size_t e = 0; e < out.size(); ++e) out[e] = cd(are[e], aim[e]);
     return out;
 }
 

@@ -272,7 +272,7 @@ class C(Gate):
     def _shared_matrix(self):
         """For a fixed inner gate, one matrix shared by every instance with
         that inner matrix (a CX per gate of a circuit would otherwise build
-        its 4x4 each time); None otherwise.  Read by Circuit._flat only."""
+        its 4x4 each time); None otherwise.  Read when a circuit lays out its matrices."""
         if not isinstance(self.gate, _Fixed):
             return None
         key = (self.gate._m.shape[0], self.gate._m.tobytes())
