@@ -990,22 +990,24 @@ static void lower_swap_block(q1g_state* s, const FusedBlock& b, const std::vecto
 // (otherwise their gates run as plain gates).
 static bool phase_kernels_take(const q1g_state* s) { return s->prec == kC64 && s->nbits <= 32; }
 
-// A phase-run block (fuse_runs) of a state phase_kernels_take: one pass with
-// the block's phase function (and its trailing 1-qubit gate).
-// Each gate of the run must be diagonal with unit-modulus entries: its
-// log-phases theta_s over its (at most two) qubits contribute, by the Moebius
-// transform, a constant, one linear term per qubit and, for two qubits, the
-// product term, which contains the run's pivot.
-template <typename Stage, typename Emit>
-static void lower_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, const std::vector<SeqGate>& gates,
-                              Stage&& stage, Emit&& emit)
+// The phase function of a phase-run block: c + L0 + x_pivot L1, coefficients
+// per bit position.  Each gate of the run must be diagonal with unit-modulus
+// entries: its log-phases theta_s over its (at most two) qubits contribute, by
+// the Moebius transform, a constant, one linear term per qubit and, for two
+// qubits, the product term, which contains the run's pivot.
+struct PhaseFunction {
+    int pivot_pos = -1;
+    double c = 0.0;
+    std::vector<double> lin0, lin1;
+};
+static PhaseFunction phase_function(const q1g_plan* p, int n, const FusedBlock& b, const std::vector<SeqGate>& gates)
 {
-    const int n = s->nbits;
+    PhaseFunction f;
     const size_t ndiag = b.gates.size() - (b.trailing_pair ? 1 : 0);
     const int pivot_q = phase_run_pivot(b, p->gate_bits);
-    const int pivot_pos = pivot_q >= 0 ? n - 1 - pivot_q : -1;
-    std::vector<double> lin0(n, 0.0), lin1(n, 0.0);
-    double c = 0.0;
+    f.pivot_pos = pivot_q >= 0 ? n - 1 - pivot_q : -1;
+    f.lin0.assign(n, 0.0);
+    f.lin1.assign(n, 0.0);
     for (size_t j = 0; j < ndiag; ++j) {
         const SeqGate& g = gates[b.gates[j]];
         const size_t k = g.bits.size(), dim = size_t(1) << k;
@@ -1022,21 +1024,33 @@ static void lower_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, co
                 }
             }
         if (k == 1) {
-            c += th[0];
-            lin0[n - 1 - g.bits[0]] += th[1] - th[0];
+            f.c += th[0];
+            f.lin0[n - 1 - g.bits[0]] += th[1] - th[0];
         } else {
             // matrix index bit 1 = g.bits[0], bit 0 = g.bits[1]
-            c += th[0];
-            lin0[n - 1 - g.bits[0]] += th[2] - th[0];
-            lin0[n - 1 - g.bits[1]] += th[1] - th[0];
+            f.c += th[0];
+            f.lin0[n - 1 - g.bits[0]] += th[2] - th[0];
+            f.lin0[n - 1 - g.bits[1]] += th[1] - th[0];
             const double w = th[3] - th[2] - th[1] + th[0];
-            if (g.bits[0] == pivot_q) lin1[n - 1 - g.bits[1]] += w;
-            else if (g.bits[1] == pivot_q) lin1[n - 1 - g.bits[0]] += w;
+            if (g.bits[0] == pivot_q) f.lin1[n - 1 - g.bits[1]] += w;
+            else if (g.bits[1] == pivot_q) f.lin1[n - 1 - g.bits[0]] += w;
             else throw Error(Q1G_ERR_INVALID_ARGUMENT, "phase run without a common qubit");
         }
     }
+    return f;
+}
+
+// A phase-run block of a state phase_kernels_take: one pass with the block's
+// phase function (and its trailing 1-qubit gate).
+template <typename Stage, typename Emit>
+static void lower_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, const std::vector<SeqGate>& gates,
+                              Stage&& stage, Emit&& emit)
+{
+    const int n = s->nbits;
+    const PhaseFunction f = phase_function(p, n, b, gates);
+    const int pivot_pos = f.pivot_pos;
     std::vector<float2> tab(2048);
-    phase_run_tables(n, c, lin0.data(), lin1.data(), tab.data());
+    phase_run_tables(n, f.c, f.lin0.data(), f.lin1.data(), tab.data());
     const void* dtab = stage(tab.data(), tab.size() * sizeof(float2));
     int q_pos = -1;
     std::array<double, 8> m2 = {1, 0, 0, 0, 0, 0, 1, 0};
@@ -1055,6 +1069,69 @@ static void lower_phase_block(q1g_plan* p, q1g_state* s, const FusedBlock& b, co
                                     x->stream);
         });
     });
+}
+
+// The trailing gate's position of a phase-run block that can be a step of a
+// group (phase_run.cu), -1 otherwise.  Positions 0 and 1 stay out: a thread's
+// amplitudes would lie within one 32-byte sector, and every access of a warp
+// would touch each sector several times.
+static int group_position(const q1g_plan* p, const FusedBlock& b)
+{
+    if (!b.phase_run || !b.trailing_pair) return -1;
+    const int t = p->nbits - 1 - p->gate_bits[b.gates.back()][0];
+    return t >= 2 ? t : -1;
+}
+
+// Blocks i .. as one group as far as they go (two at least), after the plain
+// gate `before` when the group starts with one (an uncontrolled 1-qubit
+// gate).  Returns the number of blocks taken, 0 for none.
+template <typename Stage, typename Emit>
+static size_t lower_phase_group(q1g_plan* p, q1g_state* s, size_t i, const GateOp* before,
+                                const std::vector<SeqGate>& gates, Stage&& stage, Emit&& emit)
+{
+    const int n = s->nbits;
+    PhaseGroup g{};
+    auto taken = [&](int t) { return std::find(g.t, g.t + g.nsteps, t) != g.t + g.nsteps; };
+    if (before) g.t[g.nsteps++] = before->map.zpos[0];
+    size_t count = 0;
+    while (g.nsteps < kPhaseGroupMax && i + count < p->blocks.size()) {
+        const int t = group_position(p, p->blocks[i + count]);
+        if (t < 0 || taken(t)) break;
+        g.t[g.nsteps++] = t;
+        ++count;
+    }
+    if (g.nsteps < 2) return 0;
+    std::vector<PhaseStepTables> tables(g.nsteps);
+    const std::vector<double> none(n, 0.0);
+    for (int k = 0; k < g.nsteps; ++k) {
+        double m2[8];
+        PhaseFunction f;
+        if (before && k == 0) {
+            f.lin0 = f.lin1 = none;
+            std::copy(before->m2, before->m2 + 8, m2);
+        } else {
+            const FusedBlock& b = p->blocks[i + k - (before ? 1 : 0)];
+            f = phase_function(p, n, b, gates);
+            const SeqGate& t = gates[b.gates.back()];
+            for (int e = 0; e < 4; ++e) {
+                m2[2 * e] = t.mat[e].real();
+                m2[2 * e + 1] = t.mat[e].imag();
+            }
+        }
+        g.pivot[k] = f.pivot_pos;
+        g.trivial0[k] = f.c == 0.0 && f.lin0 == none;
+        g.real[k] = m2[1] == 0.0 && m2[3] == 0.0 && m2[5] == 0.0 && m2[7] == 0.0;
+        for (int e = 0; e < 8; ++e) g.m2[k][e] = (float)m2[e];
+        phase_group_tables(g, n, f.c, f.lin0.data(), f.lin1.data(), tables[k]);
+    }
+    const auto* d = static_cast<const PhaseStepTables*>(stage(tables.data(), tables.size() * sizeof(PhaseStepTables)));
+    emit([=](q1g_state* x) {
+        const uint64_t total = x->total();
+        x->launch("phase_group_c64", 2.0 * total * x->bsz(), [&] {
+            return launch_phase_group(x->amps.as<float2>(), total, n, g, d, x->sm_count(), x->stream);
+        });
+    });
+    return count;
 }
 
 // Consecutive pair and phase updates (every one run_takes) as tile passes
@@ -1323,6 +1400,25 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
             if (ops[i].kind == GateOp::Noop) continue;
             if (run_takes(ops[i])) {
                 plain.push_back(ops[i]);
+                continue;
+            }
+        }
+        if (p->blocks[i].phase_run) {
+            // an uncontrolled gate just before (a Fourier transform's first
+            // Hadamard) is the group's first step
+            const GateOp* before = plain.size() == 1 && plain[0].kind == GateOp::Pair && plain[0].map.nz == 1 &&
+                                           plain[0].map.zpos[0] >= 2
+                                       ? &plain[0]
+                                       : nullptr;
+            size_t count = before ? lower_phase_group(p, s, i, before, gates, stage, emit) : 0;
+            if (count) {
+                plain.clear();
+            } else {
+                flush_plain();
+                count = lower_phase_group(p, s, i, nullptr, gates, stage, emit);
+            }
+            if (count) {
+                i += count - 1;
                 continue;
             }
         }

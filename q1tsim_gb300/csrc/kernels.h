@@ -44,6 +44,34 @@ void phase_run_tables(int nbits, double c, const double* lin0, const double* lin
 cudaError_t launch_phase_run(float2* amps, uint64_t total, int nbits, int pivot_pos, const void* dtab, int q_pos,
                              const double* m2, int sm_count, cudaStream_t st);
 
+// Several such passes with trailing gates as one (phase_run.cu): two to
+// kPhaseGroupMax steps, each a phase function and then a 2x2 matrix on the
+// pairs along its position t.
+constexpr int kPhaseGroupMax = 4;
+// Step's device tables: the phases of L0 (with c) and of L0 + L1 per index
+// byte, as 32-bit fractions of a turn, without the group's own positions;
+// and the factors of those (index bit i = step i's position).
+struct PhaseStepTables {
+    uint32_t a0[4][256];
+    uint32_t a1[4][256];
+    float2 g0[1 << kPhaseGroupMax];
+    float2 g1[1 << kPhaseGroupMax];
+};
+struct PhaseGroup {
+    int nsteps;
+    int t[kPhaseGroupMax];        // positions, distinct, >= 2
+    int pivot[kPhaseGroupMax];    // position whose bit selects L0 + L1, -1: none
+    int trivial0[kPhaseGroupMax]; // L0 and c are zero
+    int real[kPhaseGroupMax];     // m2 has no imaginary part
+    float m2[kPhaseGroupMax][8];
+};
+// Fills out with the tables of a step with these coefficients per position
+// (g's nsteps and t are set).
+void phase_group_tables(const PhaseGroup& g, int nbits, double c, const double* lin0, const double* lin1,
+                        PhaseStepTables& out);
+cudaError_t launch_phase_group(float2* amps, uint64_t total, int nbits, const PhaseGroup& g,
+                               const PhaseStepTables* d_tables, int sm_count, cudaStream_t st);
+
 // ---- swap_run.cu: a run of swaps on disjoint qubit pairs as one pass
 // Layout of the pass (host): tiles of 1024 amplitudes over 10 positions
 // closed under the swaps, the swaps outside them, and the stage offsets of
