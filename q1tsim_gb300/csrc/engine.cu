@@ -1119,6 +1119,9 @@ static size_t lower_phase_group(q1g_plan* p, q1g_state* s, size_t i, const GateO
             }
         }
         g.pivot[k] = f.pivot_pos;
+        g.inner[k] = -1;
+        for (int j = 0; j < g.nsteps; ++j)
+            if (g.t[j] == f.pivot_pos) g.inner[k] = j;
         g.trivial0[k] = f.c == 0.0 && f.lin0 == none;
         g.real[k] = m2[1] == 0.0 && m2[3] == 0.0 && m2[5] == 0.0 && m2[7] == 0.0;
         for (int e = 0; e < 8; ++e) g.m2[k][e] = (float)m2[e];

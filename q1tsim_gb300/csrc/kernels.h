@@ -61,6 +61,7 @@ struct PhaseGroup {
     int nsteps;
     int t[kPhaseGroupMax];        // positions, distinct, >= 2
     int pivot[kPhaseGroupMax];    // position whose bit selects L0 + L1, -1: none
+    int inner[kPhaseGroupMax];    // the step whose position the pivot is, -1: none of the group's
     int trivial0[kPhaseGroupMax]; // L0 and c are zero
     int real[kPhaseGroupMax];     // m2 has no imaginary part
     float m2[kPhaseGroupMax][8];

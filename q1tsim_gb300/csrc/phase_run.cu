@@ -97,7 +97,9 @@ k_phase_pair(float2* a, uint64_t pairs, IndexMap map, uint64_t bit, uint64_t nma
 // per-byte tables) and turned into a factor once per thread and step
 // (sincospif on at most an eighth of a turn): more accurate than the product
 // of eight FP32 factors, and 2^S amplitudes share it.  28-qubit QFT, 26 steps
-// in 7 passes: QFT_NEW ms instead of 21.1.
+// in 7 passes of 0.78 ms (0.64 for the memory alone; 24 warps per SM, more or
+// fewer registers and a prefetch of the next amplitudes measured slower), the
+// transform 8.3 ms instead of 21.4.
 
 constexpr int kGroupThreads = 256;
 
@@ -122,35 +124,44 @@ __device__ __forceinline__ uint32_t byte_sum(const uint32_t (&a)[4][256], uint32
     return a[0][x & 255u] + a[1][(x >> 8) & 255u] + a[2][(x >> 16) & 255u] + a[3][x >> 24];
 }
 
+// y[m] times f g[m] for the m with index bit BIT set (BIT < 0: every m; the
+// set is known at compile time, so no amplitude is tested for it) or clear.
+template <int S, int BIT, bool SET>
+__device__ __forceinline__ void group_phase(float2 (&y)[1 << S], float2 f, const float2* g)
+{
+#pragma unroll
+    for (int m = 0; m < (1 << S); ++m)
+        if (BIT < 0 || ((m >> (BIT < 0 ? 0 : BIT)) & 1) == (SET ? 1 : 0)) y[m] = cmulf(cmulf(f, g[m]), y[m]);
+}
+
+template <int S, bool SET>
+__device__ __forceinline__ void group_phase_at(float2 (&y)[1 << S], int bit, float2 f, const float2* g)
+{
+    switch (bit) {
+        case 0: group_phase<S, 0, SET>(y, f, g); break;
+        case 1: group_phase<S, 1, SET>(y, f, g); break;
+        case 2:
+            if constexpr (S > 2) group_phase<S, 2, SET>(y, f, g);
+            break;
+        case 3:
+            if constexpr (S > 3) group_phase<S, 3, SET>(y, f, g);
+            break;
+        default: group_phase<S, -1, SET>(y, f, g); break;
+    }
+}
+
 // One step on the 2^S amplitudes y; step K's position is index bit K.
 template <int S, int K>
 __device__ __forceinline__ void group_step(float2 (&y)[1 << S], const PhaseGroup& g, const PhaseStepTables& T,
                                            uint32_t x)
 {
-    // amplitudes whose pivot bit is set
-    uint32_t on = 0;
-    const int v = g.pivot[K];
-    if (v >= 0) {
-        on = ((x >> v) & 1u) ? 0xffffu : 0u;
-#pragma unroll
-        for (int b = 0; b < S; ++b)
-            if (g.t[b] == v) {
-                constexpr uint32_t kBit[4] = {0xaaaau, 0xccccu, 0xf0f0u, 0xff00u};
-                on = kBit[b];
-            }
-    }
-    if (!g.trivial0[K]) {
-        const float2 f = turn_factor(byte_sum(T.a0, x));
-#pragma unroll
-        for (int m = 0; m < (1 << S); ++m)
-            if (!((on >> m) & 1u)) y[m] = cmulf(cmulf(f, T.g0[m]), y[m]);
-    }
-    if (on & ((1u << (1 << S)) - 1u)) {
-        const float2 f = turn_factor(byte_sum(T.a1, x));
-#pragma unroll
-        for (int m = 0; m < (1 << S); ++m)
-            if ((on >> m) & 1u) y[m] = cmulf(cmulf(f, T.g1[m]), y[m]);
-    }
+    // pivot in the group: half of the amplitudes each way; outside it (or
+    // none): all of them one way
+    const int in = g.inner[K], v = g.pivot[K];
+    const bool on = in >= 0 || (v >= 0 && ((x >> v) & 1u));
+    if (!g.trivial0[K] && (in >= 0 || !on))
+        group_phase_at<S, false>(y, in, turn_factor(byte_sum(T.a0, x)), T.g0);
+    if (on) group_phase_at<S, true>(y, in, turn_factor(byte_sum(T.a1, x)), T.g1);
     const float* m2 = g.m2[K];
     if (g.real[K]) {
 #pragma unroll
