@@ -24,7 +24,7 @@ namespace q1g {
 namespace {
 
 constexpr int kSwapTileBits = 10;
-constexpr size_t kSwapStageBytes = 128 * 1024;   // 2 tiles per warp: 8 warps of 8-byte, 4 of 16-byte amplitudes
+constexpr size_t kSwapStageBytes = 192 * 1024;   // 2 tiles per warp: 12 warps of 8-byte, 6 of 16-byte amplitudes
 
 template <typename E, int W>
 __global__ void __launch_bounds__(W * 32, 1)
@@ -187,13 +187,13 @@ cudaError_t launch_swap_run(void* amps, int amp_bytes, uint64_t total, const voi
     const SwapTile* t = static_cast<const SwapTile*>(dtile);
     cudaError_t e;
     if (amp_bytes == 8) {
-        constexpr int W = 8;
+        constexpr int W = 12;
         e = swap_opt_in(k_swap_run<uint2, W>);
         if (e != cudaSuccess) return e;
         const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sm_count, (tiles + W - 1) / W);
         k_swap_run<uint2, W><<<grid, W * 32, kSwapStageBytes, st>>>((uint2*)amps, total, t);
     } else {
-        constexpr int W = 4;
+        constexpr int W = 6;
         e = swap_opt_in(k_swap_run<uint4, W>);
         if (e != cudaSuccess) return e;
         const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sm_count, (tiles + W - 1) / W);
