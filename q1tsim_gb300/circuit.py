@@ -318,7 +318,8 @@ class Circuit:
     def _run_seq(self, q_state, idx, seq):
         if hasattr(q_state, "apply_plan"):
             flat = self._frozen[idx] if self._frozen is not None else self._flat_current(idx, seq)
-            key = (idx, q_state.precision)
+            widest = getattr(q_state, "max_fusion_width", 5)
+            key = (idx, q_state.precision, widest)
             plan = self._plans.get(key)
             if plan is None:
                 bits = [op[2] for op in seq]
@@ -327,10 +328,9 @@ class Circuit:
                 if width == "auto":
                     from . import autotune
                     width, tc, tiling = autotune.tune(self.nr_qbits, q_state.precision, bits, flat, kinds=kinds)
-                if q_state.precision == "c128" and width > 3:
-                    # complex128 blocks of up to 3 qubits run on double-float
-                    # pairs in warp tiles; larger ones would take the FP64 pipe
-                    width = 3
+                # complex128 blocks beyond 3 qubits take the FP64 pipe where the
+                # tensor cores do not apply
+                width = min(width, widest)
                 plan = Plan(self.nr_qbits, bits, width, tensor_cores=tc, kinds=kinds)
                 if tiling is not None and tiling != Plan.DEFAULT_TC_TILING:
                     plan.set_tc_tiling(*tiling)

@@ -275,8 +275,8 @@ void q1g_state::apply_gate(const double* mat, size_t k, const size_t* bits, size
 
 // src/vectorstate.rs:180-189: the same one-qubit gate on every qubit.  The
 // reference makes one pass per qubit.  The gates act on different qubits, so
-// they commute and fuse into blocks of up to five qubits (complex64: one
-// tensor-core pass per block, 6 passes at 30 qubits) or three (complex128:
+// they commute and fuse into blocks of up to five qubits (one tensor-core pass
+// per block, 6 passes at 30 qubits; three in complex128 below 12 qubits:
 // double-float warp tiles).  With FP64 arithmetic requested, the gates run
 // one by one, as the reference rounds.
 void q1g_state::apply_unary_all(const double* mat)
@@ -286,7 +286,7 @@ void q1g_state::apply_unary_all(const double* mat)
         for (size_t b = 0; b < (size_t)nbits; ++b) apply_gate(mat, 1, &b, 1);
         return;
     }
-    const int width = prec == kC64 ? 5 : 3;
+    const int width = prec == kC64 || nbits >= 12 ? 5 : 3;
     if (!unary_plan || unary_plan->nbits != nbits || unary_plan->width != width) {
         auto p = std::make_unique<q1g_plan>();
         p->nbits = nbits;
@@ -1137,6 +1137,53 @@ static size_t lower_phase_group(q1g_plan* p, q1g_state* s, size_t i, const GateO
     return count;
 }
 
+// Whether a dense block (its classified op, matrix and qubits) on this state
+// runs on the tensor cores: complex64 in pairs of f16 halves (fused_tc.cu),
+// complex128 in six digits (fused_tc_c128.cu) unless FP64 arithmetic was asked
+// for.
+static bool tc_takes(const q1g_plan* p, const q1g_state* s, const GateOp& op, const std::vector<cd>& mat,
+                     const std::vector<int>& bits)
+{
+    return p->tensor_cores && s->nbits >= 12 && !(s->prec == kC128 && s->fp64_exact) && op.kind == GateOp::Dense &&
+           op.t >= 3 && bits.size() <= 5 && tc_block_bounded(mat.data(), 1 << bits.size());
+}
+
+// A block as a tensor-core pass of a complex128 state.
+template <typename Stage, typename Emit>
+static void lower_z_block(q1g_state* s, const std::vector<cd>& mat, const std::vector<int>& bits, Stage&& stage,
+                          Emit&& emit)
+{
+    const int n = s->nbits;
+    const std::vector<int> T = tile_positions({&bits}, n);
+    // gate positions: the block's own, padded from the tile's highest (rows
+    // at the lowest positions make whole runs of the copies)
+    std::vector<int> gpos = positions_of(bits, n);
+    for (int j = 11; (int)gpos.size() < 5; --j)
+        if (std::find(gpos.begin(), gpos.end(), T[j]) == gpos.end()) gpos.push_back(T[j]);
+    std::sort(gpos.begin(), gpos.end());
+    uint32_t gate_bits = 0;
+    int gate_of[5];
+    std::vector<int> order(5);      // qubits, matrix MSB first
+    for (int k = 0; k < 5; ++k) {
+        gate_of[k] = (int)(std::find(T.begin(), T.end(), gpos[k]) - T.begin());
+        gate_bits |= 1u << gate_of[k];
+        order[4 - k] = n - 1 - gpos[k];
+    }
+    ZPass pass;
+    z_pass_layout(pass, T.data(), gate_bits, gate_of);
+    const auto m32 = embed_matrix(mat, bits, order);
+    std::vector<unsigned char> img(kZImageBytes);
+    z_pass_image(reinterpret_cast<const double*>(m32.data()), img.data());
+    const void* d = stage(img.data(), img.size());
+    emit([pass, d](q1g_state* x) {
+        const uint64_t total = x->total();
+        x->launch("fused_tc_c128", 2.0 * total * x->bsz(), [&] {
+            return launch_fused_tc_c128(x->amps.as<double2>(), total, pass, d, x->errbuf.as<int>(), x->sm_count(),
+                                        x->stream, x->tc_wait_ns);
+        });
+    });
+}
+
 // Consecutive pair and phase updates (every one run_takes) as tile passes
 // (gate_run.h).  A pass of one op, or one whose ops together touch less than
 // the state where that is what costs (a state beyond the L2: two CX read and
@@ -1177,12 +1224,11 @@ static void lower_plain_gates(q1g_state* s, const std::vector<GateOp>& ops, Stag
 // Device bytes of a block's staged data at most: a run table entry per gate
 // (and its alignment), a swap tile or phase tables, a dense matrix in one of
 // its forms, or a tensor-core image.
-static size_t staging_bytes(const q1g_plan* p, const FusedBlock& b)
+static size_t staging_bytes(const FusedBlock& b)
 {
     size_t n = b.gates.size() * 512;
-    if (b.phase_run || b.swap_run || b.qubits.size() >= 3) n += 32768;
+    if (b.phase_run || b.swap_run || b.qubits.size() >= 3) n += std::max<size_t>(32768, kZImageBytes);
     else n += 2048;
-    (void)p;
     return n;
 }
 
@@ -1297,7 +1343,6 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
         const double* m = mats + p->mat_off[g];
         for (size_t e = 0; e < dim * dim; ++e) gates[g].mat[e] = cd(m[2 * e], m[2 * e + 1]);
     }
-    const bool use_tc = s->prec == kC64 && s->nbits >= 12 && p->tensor_cores;
     const size_t nb = p->blocks.size();
     std::vector<GateOp> ops(nb);
     std::vector<std::vector<cd>> bmats(nb);
@@ -1339,12 +1384,15 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
         e = std::move(pass);
         return e;
     };
-    // tensor-core eligible: dense blocks of >= 3 target qubits
     auto eligible = [&](size_t bi) {
         if (p->blocks[bi].phase_run || p->blocks[bi].swap_run) return false;
         prepare(bi);
-        return use_tc && ops[bi].kind == GateOp::Dense && ops[bi].t >= 3 && bbits[bi].size() <= 5 &&
-               tc_block_bounded(bmats[bi].data(), 1 << bbits[bi].size());
+        return tc_takes(p, s, ops[bi], bmats[bi], bbits[bi]);
+    };
+    auto tensor_cores = [&] {
+        if (L.tensor_cores) return;
+        s->clear_error_flag();
+        L.tensor_cores = true;
     };
     // Staging: every pass uploads its matrix or tensor-core image from its own
     // slice of one pinned buffer into its own slice of L's device buffer.
@@ -1358,7 +1406,7 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
     L.launches.clear();
     L.tensor_cores = false;
     size_t staging = 256;
-    for (const auto& b : p->blocks) staging += staging_bytes(p, b);
+    for (const auto& b : p->blocks) staging += staging_bytes(b);
     p->hmats.ensure(staging);
     L.dmats.ensure(staging);
     size_t staged = 0;
@@ -1435,7 +1483,10 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
             continue;
         }
         const GateOp& op = ops[i];
-        if (eligible(i)) {
+        if (s->prec == kC128 && eligible(i)) {
+            tensor_cores();
+            lower_z_block(s, bmats[i], bbits[i], stage, emit);
+        } else if (eligible(i)) {
             // consecutive blocks share a pass when their qubits fit one
             // 12-position tile with runs of >= 128 amplitudes or as one
             // tensor-map box: up to three in the four-group kernel's direct
@@ -1484,10 +1535,7 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
                 }
             }
             if (group == 1) t = layout(i, 1);
-            if (!L.tensor_cores) {
-                s->clear_error_flag();
-                L.tensor_cores = true;
-            }
+            tensor_cores();
             const std::vector<cd>* gm[kTcMaxBlocks];
             const std::vector<int>* gq[kTcMaxBlocks];
             for (int j = 0; j < group; ++j) gm[j] = &bmats[i + j], gq[j] = &bbits[i + j];
@@ -1600,7 +1648,8 @@ void plan_run(q1g_plan* p, q1g_state* s, const double* mats, size_t n, bool subs
         s->d2h(h_flag, s->errbuf.p, sizeof(int), "read error flag");
         s->sync();
         if (*h_flag) throw Error(Q1G_ERR_TIMEOUT, "a tensor-core block kernel gave up waiting on its MMAs");
-        s->norm_pending = true;
+        // (complex128 passes round to nearest and keep the norm)
+        s->norm_pending = s->norm_pending || s->prec == kC64;
     }
 }
 

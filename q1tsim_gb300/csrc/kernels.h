@@ -299,6 +299,26 @@ void tc_operand_scales(double max_norm, TcOffsets& offs);
 // amplitude outgrows its column norm, as the operand scale assumes).
 bool tc_block_bounded(const std::complex<double>* m, int dim);
 
+// ---- fused_tc_c128.cu: the same contraction on complex128 states
+// One block per pass.  Tile coordinate x (bit j: the tile's j-th position)
+// lies at amplitude offset OR off[j] and staged slot XOR slot[j].
+struct ZPass {
+    IndexMap tilemap;
+    uint64_t off[12];
+    uint32_t slot[12];
+    uint32_t row[7];         // slot of row bit r
+    uint16_t gate[32];       // slot of gate state g
+};
+// gate_bits: the five tile bits that are gates; gate_of[k]: the tile bit of
+// matrix index bit k.
+void z_pass_layout(ZPass& p, const int* tile_pos /* 12, ascending */, uint32_t gate_bits, const int* gate_of);
+// Device data of a pass with the 32x32 complex matrix m (rows of 2-norm <= 1):
+// six digits of the 64x64 real embedding, then m itself.
+constexpr size_t kZImageBytes = 6 * 8192 + 2048 * sizeof(double);
+void z_pass_image(const double* m, unsigned char* out);
+cudaError_t launch_fused_tc_c128(double2* amps, uint64_t total, const ZPass& p, const void* d_image, int* d_err,
+                                 int sm_count, cudaStream_t st, uint64_t wait_ns);
+
 // ---- state_kernels.cu: construction, conversion, collapse
 cudaError_t launch_fill_basis(void* amps, int prec, uint64_t n_amps, const uint64_t* d_col_index,
                               uint64_t ncols, uint64_t col_len, cudaStream_t st);

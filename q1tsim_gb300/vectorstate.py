@@ -86,6 +86,7 @@ class VectorState:
         self._h = _handle
         self._nr_bits = nr_bits
         self._nr_shots = nr_shots
+        self._fp64_exact = False
 
     @classmethod
     def from_qubit_coefs(cls, coefs, nr_shots, precision="c128"):
@@ -169,6 +170,16 @@ class VectorState:
         """complex128: FP64 arithmetic (the reference's rounding) instead of
         the default double-float pairs (within the 1e-12 contract)."""
         check(_lib.load().q1g_state_set_fp64_exact(self._h, 1 if exact else 0))
+        self._fp64_exact = bool(exact)
+
+    @property
+    def max_fusion_width(self):
+        """Qubits per fused block that pay: five where blocks run on the
+        tensor cores (complex64; complex128 from 12 qubits on, in
+        double-float-like accuracy), three in warp tiles otherwise."""
+        if self.precision == "c64" or (self._nr_bits >= 12 and not self._fp64_exact):
+            return 5
+        return 3
 
     def set_stream(self, stream):
         """Run on a caller-owned cudaStream_t (an int handle), None = own."""

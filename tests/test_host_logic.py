@@ -134,3 +134,8 @@ def test_f16_rounding_and_tensor_core_images(gxx, tmp_path):
 def test_gate_runs_replay_the_sequence(gxx, tmp_path):
     out = _run(_link_against_library(gxx, tmp_path, "gate_run_check"))
     assert out.startswith("bad 0"), out
+
+
+def test_complex128_tensor_core_layout_and_image(gxx, tmp_path):
+    out = _run(_link_against_library(gxx, tmp_path, "z_pass_check"))
+    assert out.startswith("bad 0"), out
