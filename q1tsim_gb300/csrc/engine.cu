@@ -1161,20 +1161,16 @@ static void lower_z_block(q1g_state* s, const std::vector<cd>& mat, const std::v
     for (int j = 11; (int)gpos.size() < 5; --j)
         if (std::find(gpos.begin(), gpos.end(), T[j]) == gpos.end()) gpos.push_back(T[j]);
     std::sort(gpos.begin(), gpos.end());
-    uint32_t gate_bits = 0;
     int gate_of[5];
     std::vector<int> order(5);      // qubits, matrix MSB first
     for (int k = 0; k < 5; ++k) {
         gate_of[k] = (int)(std::find(T.begin(), T.end(), gpos[k]) - T.begin());
-        gate_bits |= 1u << gate_of[k];
         order[4 - k] = n - 1 - gpos[k];
     }
     ZPass pass;
-    z_pass_layout(pass, T.data(), gate_bits, gate_of);
+    z_pass_layout(pass, T.data(), gate_of);
     const auto m32 = embed_matrix(mat, bits, order);
-    std::vector<unsigned char> img(kZImageBytes);
-    z_pass_image(reinterpret_cast<const double*>(m32.data()), img.data());
-    const void* d = stage(img.data(), img.size());
+    const void* d = stage(m32.data(), m32.size() * sizeof(cd));
     emit([pass, d](q1g_state* x) {
         const uint64_t total = x->total();
         x->launch("fused_tc_c128", 2.0 * total * x->bsz(), [&] {
@@ -1227,7 +1223,7 @@ static void lower_plain_gates(q1g_state* s, const std::vector<GateOp>& ops, Stag
 static size_t staging_bytes(const FusedBlock& b)
 {
     size_t n = b.gates.size() * 512;
-    if (b.phase_run || b.swap_run || b.qubits.size() >= 3) n += std::max<size_t>(32768, kZImageBytes);
+    if (b.phase_run || b.swap_run || b.qubits.size() >= 3) n += 32768;
     else n += 2048;
     return n;
 }

@@ -10,41 +10,50 @@
 // integers of at most 2^8, a product a_s b_t summed over the row's 64
 // components stays below 2^22, and the products of equal weight d = s + t
 // share an FP32 accumulator D_d: exact for d <= 3 (four products, 2^24) and
-// good to a unit of 2^-36 for d = 4.  The products of d = 5 (their B digits
-// times 2^-9) go to D_4 too, where their fraction is below what matters; d >= 6
-// (2^-54 of the row's maximum each) is dropped.  21 of the 36 digit products
-// remain: with the digits of B stacked, A_s times [B_0; ..; B_(4-s)] is one
-// product of N = 64 (5 - s) into D_s .. D_4, and A_s times B_(5-s) one of N = 64.
+// good to a unit of 2^-36 and 2^-45 for d = 4 and 5; d >= 6 (2^-54 of the row's
+// maximum each) is dropped.  21 of the 36 digit products remain: with the
+// digits of B stacked, A_s times [B_0; ..; B_(5-s)] is one product of
+// N = 64 (6 - s) into D_s .. D_5 (two instructions where that is above 256).
 // Measured against 64 bits the result of a block is about 1e-15 off (relative
 // 2-norm), where the ~15 gates it replaces left 2.4e-15 each.
 //
-// One 16-warp CTA per SM, persistent over tiles.  Thread (row t, quarter q)
-// holds 8 of the row's amplitudes: it reads them from the stage, agrees on
-// the row's exponent through shared memory, and stores the digits to TMEM
-// (A_s in columns 32 s ..: one 32-bit column per amplitude); one thread issues
-// the 48 MMAs; each thread then reads its 16 columns of the five accumulators,
-// carries them into one double-float value per component (rounding each
-// accumulator's upper part into the next; all exact), and writes the new
-// amplitudes over the old ones in the stage.  The next tile's copies
-// (cp.async, 16 bytes per amplitude, whole runs per warp) are under way from
-// the split on.  TMEM: 192 columns of A, 320 of accumulators.  Shared memory:
-// B_0..B_4 (40 KB), the scaled B_0..B_5 (48 KB), two 64 KB stages, whose slots
-// are XOR-swizzled so that the lanes of a row read hit distinct banks.
+// One 16-warp CTA per SM, persistent over tiles.  Thread (row t, part) holds 8
+// of the row's amplitudes, so a warp's 256 amplitudes lie in whole runs of at
+// least 8 (its rows' and states' low bits include the tile's three lowest): it
+// copies them in (cp.async) and, rearranged through shared memory, out by
+// itself.  TMEM has room for one tile only: 128 columns of A (digit s < 4 in
+// columns 32 s ..: one 32-bit column per amplitude; the other two digits are in
+// shared memory), 384 of accumulators.  So the next tile's digits wait in
+// registers while the MMAs of a tile run; when these are done every thread
+// stores those digits and reads its 16 columns of the accumulators, and under
+// the next MMAs the threads carry the accumulators into one double-float value
+// per component (rounding each accumulator's upper part into the next; all
+// exact), write the tile out, and read and split the one after the next.  One
+// thread issues the MMAs, a K step at a time between its own work: the issue
+// blocks while the tensor cores' queue is full.
+// Shared memory: B_0..B_5 (48 KB, made from the matrix by each CTA), A_4 and A_5
+// (32 KB), the tile coming in and the tile going out (64 KB each),
+// XOR-swizzled so that lanes hit distinct banks.
 //
-// A tile takes 15.5 k cycles where its bytes take 5.9 k of the SM's share of
-// HBM: digits 3.6 k, MMAs 4.3 k, carries 3.7 k, store 2.8 k, one after the
-// other.  27 qubits: 1.63 ms per pass of up to five qubits, against 1.75 ms per
-// pass of three in double-float warp tiles; a 25-qubit brick circuit (10 layers)
-// went from 25.8 to 7.8 ms.  At 13 qubits a pass takes 15 us between events, a
-// warp-tile pass of three qubits 28 us.
+// 27 qubits: 1.49 ms per pass of up to five qubits (13.4 k cycles per tile;
+// its bytes take 5.9 k of the SM's share of HBM), against 1.75 ms per pass of
+// three in double-float warp tiles.  What bounds it is the threads' own work,
+// half of it integer arithmetic at half rate: digits 2.6 k cycles, carries and
+// joins 5 k, copies 3 k; the MMAs (3 k) run under it.  One tile after another
+// without the overlap took 1.61 ms.  Tried and slower: the digits' carries
+// before the next MMAs (1.60 ms), a warp of its own for the MMAs (five warps
+// on a scheduler leave 96 registers) with three that copy (1.85), bulk copies
+// of 2 KB runs (1.48 to 1.80).  At 13 qubits a pass takes 15 us between
+// events, a warp-tile pass of three qubits 28 us.
 //
-// Rows with an infinity or NaN are done in FP64 from the stage.
+// Rows with an infinity or NaN are done in FP64 as they come in.
 #include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "df64.cuh"
@@ -59,35 +68,30 @@ namespace {
 
 constexpr int kZThreads = 512;
 constexpr uint32_t kZTile = 4096;                       // amplitudes
-constexpr uint32_t kZStage = kZTile * 16;               // bytes
+constexpr uint32_t kZWarp = 256;                        // a warp's amplitudes
 constexpr uint32_t kZSlice = 8192;                      // one digit of R: 64 rows x 64 f16
-// shared memory: barrier and row maxima; B_0..B_4; scaled B_0..B_5; two stages
-constexpr uint32_t kZOffBar = 0, kZOffSlot = 8, kZOffAbort = 12, kZOffMax = 1024;
+constexpr uint32_t kZSliceA = 16384;                    // one digit of A: 128 rows x 64 f16
+// shared memory: barrier, tile offsets and row maxima; B_0..B_5; A_4 and A_5;
+// the tile coming in; the tile going out
+constexpr uint32_t kZOffBar = 0, kZOffSlot = 8, kZOffAbort = 12, kZOffBase = 64, kZOffMax = 1024;
 constexpr uint32_t kZOffB = 4096;
-constexpr uint32_t kZOffBs = kZOffB + 5 * kZSlice;
-constexpr uint32_t kZOffStage = kZOffBs + 6 * kZSlice;
-constexpr uint32_t kZSmem = kZOffStage + 2 * kZStage;
+constexpr uint32_t kZOffA = kZOffB + 6 * kZSlice;
+constexpr uint32_t kZOffIn = kZOffA + 2 * kZSliceA;
+constexpr uint32_t kZOffOut = kZOffIn + kZTile * 16;
+constexpr uint32_t kZSmem = kZOffOut + kZTile * 16;
 constexpr uint32_t kZSmemAlloc = kZSmem + 1024;         // alignment slack
-static_assert(kZOffMax + 4 * 128 * 4 <= kZOffB && kZOffB % 1024 == 0 && kZOffStage % 1024 == 0, "layout");
+constexpr uint32_t kZBases = 8;                         // ring of tile offsets
+static_assert(kZOffBase + kZBases * 8 <= kZOffMax && kZOffMax + 4 * 128 * 4 <= kZOffB && kZOffB % 1024 == 0 &&
+                  kZOffIn % 1024 == 0,
+              "layout");
 static_assert(kZSmemAlloc <= 227 * 1024, "fits the SM's shared memory");
-constexpr uint32_t kZColD = 192;                        // accumulators' first TMEM column
+constexpr uint32_t kZColD = 128;                        // accumulators' first TMEM column
 
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t* v)
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* v)
 {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
-                 "r"(v[2]), "r"(v[3])
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]),
+                 "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v)
-{
-    uint32_t r[8];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-        : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 __device__ __forceinline__ float2 splat(float v) { return make_float2(v, v); }
@@ -200,15 +204,30 @@ __device__ __forceinline__ void sts_amp(uint32_t addr, double re, double im)
     asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(addr), "d"(re), "d"(im) : "memory");
 }
 
-// Eight outputs of a row (rows of the matrix at mat) from its inputs at xa.
+__device__ __forceinline__ void sts_u32x4(uint32_t addr, const uint32_t* v)
+{
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+__device__ __forceinline__ void sts_raw(uint32_t addr, float2 h, float2 l)
+{
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(h.x), "f"(h.y), "f"(l.x), "f"(l.y)
+                 : "memory");
+}
+
+// Eight outputs of a row (rows of the matrix at mat) from its inputs, which the
+// four warps of its parts hold at xa + 4 (warps) * 4 KB * part.
 __device__ __noinline__ void row_fp64(uint32_t xa, uint32_t rslot, const ZPass& p, const double2* mat, double2* y)
 {
 #pragma unroll 1
     for (int j = 0; j < 8; ++j) {
         double re = 0.0, im = 0.0;
 #pragma unroll 1
-        for (int s = 0; s < 32; ++s) {
-            const ulonglong2 b = lds_amp(xa + (rslot ^ p.gate[s]) * 16u);
+        for (uint32_t s = 0; s < 32; ++s) {
+            uint32_t slot = rslot;
+            for (int k = 0; k < 3; ++k)
+                if ((s >> k) & 1u) slot ^= p.slot[p.gate_of[k]];
+            const ulonglong2 b = lds_amp(xa + ((s >> 3) * 4u * kZWarp + slot) * 16u);
             const double vr = __longlong_as_double((long long)b.x), vi = __longlong_as_double((long long)b.y);
             const double2 c = mat[32 * j + s];
             re = fma(c.x, vr, fma(-c.y, vi, re));
@@ -218,10 +237,69 @@ __device__ __noinline__ void row_fp64(uint32_t xa, uint32_t rslot, const ZPass& 
     }
 }
 
+// v (|v| < 2) in units of 2^-53, rounded
+__device__ __forceinline__ int64_t fixed53(double v)
+{
+    const uint64_t b = (uint64_t)__double_as_longlong(v);
+    const int e = (int)((b >> 52) & 2047u) - 1022;          // shift of the 53-bit mantissa
+    const uint64_t m = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+    const uint64_t u = e >= 0 ? m << min(e, 1) : e < -53 ? 0ull : (m + (1ull << (-e - 1))) >> -e;
+    return (int64_t)b < 0 ? -(int64_t)u : (int64_t)u;
+}
+
+// The 64x64 real embedding of the matrix in digits B_0..B_5.  Digits in -256..255 (the top one up to 257) from the
+// low end.
+__device__ __forceinline__ void build_operands(const double2* __restrict__ mat, uint8_t* smem, int tid)
+{
+    const __half2 bias = __float2half2_rn(1536.0f);
+    for (int e = tid; e < 1024; e += kZThreads) {
+        const double2 c = mat[e];
+        int64_t re = fixed53(c.x), im = fixed53(c.y);
+        const uint32_t row = 2u * (uint32_t)(e >> 5), k = 2u * (uint32_t)(e & 31);
+        const uint32_t at0 = tc_sw128_offset(row, k), at1 = tc_sw128_offset(row + 1, k);
+#pragma unroll
+        for (int t = 5; t >= 0; --t) {
+            int r, i;
+            if (t > 0) {
+                r = (int)((uint32_t)(re + 256) & 511u) - 256;
+                i = (int)((uint32_t)(im + 256) & 511u) - 256;
+                re = (re - r) >> 9;
+                im = (im - i) >> 9;
+            } else {
+                r = (int)re;
+                i = (int)im;
+            }
+            // 1024 + field as f16 bits, minus the bias: row (re, -im), row (im, re)
+            const uint32_t w0 = 0x64006400u + (uint32_t)(512 + r) + ((uint32_t)(512 - i) << 16);
+            const uint32_t w1 = 0x64006400u + (uint32_t)(512 + i) + ((uint32_t)(512 + r) << 16);
+            const __half2 h0 = __hsub2(*reinterpret_cast<const __half2*>(&w0), bias);
+            const __half2 h1 = __hsub2(*reinterpret_cast<const __half2*>(&w1), bias);
+            *reinterpret_cast<__half2*>(smem + kZOffB + t * kZSlice + at0) = h0;
+            *reinterpret_cast<__half2*>(smem + kZOffB + t * kZSlice + at1) = h1;
+        }
+    }
+}
+
+// K step ks of a tile's products, by one thread.
+__device__ __forceinline__ void issue_step(uint32_t ks, uint32_t tmem, uint32_t sbase, uint32_t mbar)
+{
+    const uint32_t D = tmem + kZColD, A = tmem + ks * 8u;
+    const uint32_t B = sbase + kZOffB + ks * 32u, As = sbase + kZOffA + ks * 32u;
+    const uint32_t acc = ks > 0 ? 1u : 0u;      // A_0 [B_0 .. B_5]: every accumulator's first product
+    mma_f16_ts(D, A, desc_sw128(B), idesc_f16(192), acc);
+    mma_f16_ts(D + 192u, A, desc_sw128(B + 3 * kZSlice), idesc_f16(192), acc);
+    mma_f16_ts(D + 64u, A + 32u, desc_sw128(B), idesc_f16(160), 1u);
+    mma_f16_ts(D + 224u, A + 32u, desc_sw128(B + 160u * 128u), idesc_f16(160), 1u);
+    mma_f16_ts(D + 128u, A + 64u, desc_sw128(B), idesc_f16(256), 1u);
+    mma_f16_ts(D + 192u, A + 96u, desc_sw128(B), idesc_f16(192), 1u);
+    mma_f16_ss(D + 256u, desc_sw128(As), desc_sw128(B), idesc_f16(128), 1u);
+    mma_f16_ss(D + 320u, desc_sw128(As + kZSliceA), desc_sw128(B), idesc_f16(64), 1u);
+    if (ks == 3) mma_commit(mbar);
+}
+
 __global__ void __launch_bounds__(kZThreads, 1)
 k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant__ ZPass p,
-                const uint4* __restrict__ image, const double2* __restrict__ mat, int* __restrict__ err,
-                uint64_t wait_ns)
+                const double2* __restrict__ mat, int* __restrict__ err, uint64_t wait_ns)
 {
     extern __shared__ uint8_t z_raw[];
     uint8_t* smem = z_raw + ((1024u - (smem_addr(z_raw) & 1023u)) & 1023u);
@@ -231,22 +309,13 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
     const uint32_t t = 32u * q + (uint32_t)lane;           // row = TMEM lane
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + kZOffAbort);
     uint32_t* rowmax = reinterpret_cast<uint32_t*>(smem + kZOffMax);
+    // offsets of this CTA's tiles, the i-th at i % 8: written by the last warp
+    // a barrier before their first use
+    uint64_t* bases = reinterpret_cast<uint64_t*>(smem + kZOffBase);
     const uint32_t mbar = sbase + kZOffBar;
+    const uint64_t count = (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
 
-    // B_0..B_4, and B_0..B_5 times 2^-9 (exact)
-    {
-        uint4* B = reinterpret_cast<uint4*>(smem + kZOffB);
-        uint4* Bs = reinterpret_cast<uint4*>(smem + kZOffBs);
-        const __half2 down = __float2half2_rn(1.0f / 512.0f);
-        for (int e = tid; e < (int)(6 * kZSlice / 16); e += kZThreads) {
-            uint4 v = image[e];
-            if (e < (int)(5 * kZSlice / 16)) B[e] = v;
-            __half2* h = reinterpret_cast<__half2*>(&v);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) h[k] = __hmul2(h[k], down);
-            Bs[e] = v;
-        }
-    }
+    build_operands(mat, smem, tid);
     if (tid == 0) {
         *abort_flag = 0;
         mbar_init(mbar, 1);
@@ -258,179 +327,238 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
+    auto put_base = [&](uint64_t i) {
+        bases[i % kZBases] = expand_index(blockIdx.x + i * gridDim.x, p.tilemap);
+    };
+    if (warp == 15 && lane < 2) put_base((uint64_t)lane);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(smem + kZOffSlot);
-    const uint32_t tl = tmem + ((32u * q) << 16);          // this warp's lanes
+    bool failed = false;
+    uint64_t it = 0;
 
-    // copies: thread's amplitude x = tid + 512 k at slot cslot ^ cstep[k]
-    uint64_t cown = 0;
+    const uint32_t tl = tmem + ((32u * q) << 16);          // this warp's lanes
+    const uint32_t in = sbase + kZOffIn + (uint32_t)warp * kZWarp * 16u;
+    const uint32_t out = sbase + kZOffOut + (uint32_t)warp * kZWarp * 16u;
+    // the warp's amplitudes: element lane + 32 k at offset own + (bits of k)
+    // and slot cslot ^ (bits of k)
+    uint64_t own = 0;
     uint32_t cslot = 0;
 #pragma unroll
-    for (int b = 0; b < 9; ++b)
-        if ((tid >> b) & 1) {
-            cown |= p.off[b];
+    for (int b = 0; b < 4; ++b)
+        if ((warp >> b) & 1) own |= p.warp[b];
+    const uint64_t wown = own;
+#pragma unroll
+    for (int b = 0; b < 5; ++b)
+        if ((lane >> b) & 1) {
+            own |= p.off[b];
             cslot ^= p.slot[b];
         }
-    auto copy_at = [&](int k, uint64_t& g, uint32_t& s) {
-        g = cown;
+    auto element = [&](int k, uint64_t& g, uint32_t& s) {
+        g = own;
         s = cslot;
 #pragma unroll
         for (int b = 0; b < 3; ++b)
             if ((k >> b) & 1) {
-                g |= p.off[9 + b];
-                s ^= p.slot[9 + b];
+                g |= p.off[5 + b];
+                s ^= p.slot[5 + b];
             }
     };
-    auto load_tile = [&](uint64_t tile, uint32_t stage) {
-        const double2* src = a + expand_index(tile, p.tilemap);
-        double2* dst = reinterpret_cast<double2*>(smem + kZOffStage + stage * kZStage);
+    auto load_tile = [&](uint64_t base) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             uint64_t g;
             uint32_t s;
-            copy_at(k, g, s);
-            cp_async16(dst + s, src + g);
+            element(k, g, s);
+            cp_async16(smem + (in - sbase) + s * 16u, a + base + g);
         }
         cp_async_commit();
     };
-    // the thread's 8 amplitudes: row t, gate states 8 part + j at byte
-    // rbyte ^ (gate bits of j)
+    // the thread's 8 amplitudes: states 8 part + j of row t at byte
+    // rbyte ^ (bits of j)
     uint32_t rslot = 0;
 #pragma unroll
-    for (int r = 0; r < 7; ++r)
-        if ((t >> r) & 1u) rslot ^= p.row[r];
-    const uint32_t rbyte = (rslot ^ p.gate[8 * part]) * 16u;
-    const uint32_t g0 = p.gate[1] * 16u, g1 = p.gate[2] * 16u, g2 = p.gate[4] * 16u;
-    auto at = [&](uint32_t stage_addr, int j) {
-        return stage_addr + (rbyte ^ ((j & 1) ? g0 : 0u) ^ ((j & 2) ? g1 : 0u) ^ ((j & 4) ? g2 : 0u));
+    for (int b = 0; b < 5; ++b)
+        if ((lane >> b) & 1) rslot ^= p.slot[p.row_of[b]];
+    const uint32_t g0 = p.slot[p.gate_of[0]] * 16u, g1 = p.slot[p.gate_of[1]] * 16u,
+                   g2 = p.slot[p.gate_of[2]] * 16u;
+    auto at = [&](uint32_t region, int j) {
+        return region + ((rslot * 16u) ^ ((j & 1) ? g0 : 0u) ^ ((j & 2) ? g1 : 0u) ^ ((j & 4) ? g2 : 0u));
+    };
+    // and their offsets (rows with infinities or NaN only)
+    auto offset_of = [&](int j) {
+        uint64_t g = wown;
+        for (int b = 0; b < 5; ++b)
+            if ((lane >> b) & 1) g |= p.off[p.row_of[b]];
+        for (int b = 0; b < 3; ++b)
+            if ((j >> b) & 1) g |= p.off[p.gate_of[b]];
+        return g;
     };
 
-    if (blockIdx.x < ntiles) load_tile(blockIdx.x, 0);
-    uint32_t it = 0;
-    bool failed = false;
-    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
-        const uint32_t stage = it & 1u;
-        const double2* X = reinterpret_cast<const double2*>(smem + kZOffStage + stage * kZStage);
-        const uint32_t xa = sbase + kZOffStage + stage * kZStage;
+    // its digits of A_4 and A_5 in shared memory: two 16-byte chunks each
+    const uint32_t a_own = sbase + kZOffA + tc_sw128_offset(t, 16u * part);
+
+    uint32_t dg[6][8];
+    uint32_t m = 0, m_prev = 0;           // the row's largest exponent
+    // Reads tile i, which is on its way, asks for the one after it, and splits.
+    auto read_split = [&](uint64_t i) {
         cp_async_wait_group<0>();
-        __syncthreads();
+        __syncwarp();
         ulonglong2 x[8];
-        uint32_t m = 0;
+        m = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            x[j] = lds_amp(at(xa, j));
+            x[j] = lds_amp(at(in, j));
             m = max(m, (uint32_t)(x[j].x >> 32) & 0x7FFFFFFFu);
             m = max(m, (uint32_t)(x[j].y >> 32) & 0x7FFFFFFFu);
         }
         rowmax[part * 128 + t] = m;
-        const bool special = __syncthreads_or(m >= 0x7FF00000u) != 0;    // an infinity or NaN in the tile
+        asm volatile("bar.sync %0, 128;" ::"r"(1u + q) : "memory");      // the four parts of these rows
         m = max(max(rowmax[t], rowmax[128 + t]), max(rowmax[256 + t], rowmax[384 + t])) & 0x7FF00000u;
-        const bool row_special = m == 0x7FF00000u;
-        // the row's largest exponent becomes that of 2^7 .. 2^8; a row below
-        // 2^-968 counts as zero
+        if (__any_sync(0xFFFFFFFFu, m == 0x7FF00000u)) {
+            // (the same lanes in each of the four warps)
+            if (m == 0x7FF00000u) {
+                double2 y[8];
+                row_fp64(sbase + kZOffIn + q * kZWarp * 16u, rslot, p, mat + 256 * part, y);
+                for (int j = 0; j < 8; ++j) a[bases[i % kZBases] + offset_of(j)] = y[j];
+            }
+            asm volatile("bar.sync %0, 128;" ::"r"(1u + q) : "memory");
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = lds_amp(at(in, j));    // (not kept across the call)
+            __syncwarp();
+        }
+        const bool more = i + 1 < count;
+        const double2* src = a + bases[(i + 1) % kZBases];
+        // the row's largest exponent becomes that of 2^7 .. 2^8; a row
+        // below 2^-968 counts as zero
         const uint32_t shift20 = (1030u << 20) - m;
         const uint32_t least = m <= (54u << 20) ? 0xFFFFFFFFu : m - (54u << 20);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            uint32_t v[6][4];
+        for (int j = 0; j < 8; ++j) {
+            uint64_t g;
+            uint32_t s;
+            element(j, g, s);
+            if (more) cp_async16(smem + (in - sbase) + s * 16u, src + g);
+            uint32_t d[6];
+            digits(scaled_split(x[j].x, shift20, least), scaled_split(x[j].y, shift20, least), d);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                uint32_t d[6];
-                digits(scaled_split(x[4 * half + j].x, shift20, least),
-                       scaled_split(x[4 * half + j].y, shift20, least), d);
-#pragma unroll
-                for (int s = 0; s < 6; ++s) v[s][j] = d[s];
-            }
-#pragma unroll
-            for (int s = 0; s < 6; ++s) tmem_st4(tl + 32u * s + 8u * part + 4u * half, v[s]);
+            for (int s = 0; s < 6; ++s) dg[s][j] = d[s];
         }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
+        cp_async_commit();
+    };
+
+    load_tile(bases[0]);
+    read_split(0);
+    // Step `it`: tile it's digits go to the tensor cores (if any), tile it - 1
+    // out (if any).  False: a wait ran out.
+    auto step = [&](auto has_tile, auto has_last) {
+        constexpr bool kTile = decltype(has_tile)::value, kLast = decltype(has_last)::value;
+        bool ok = true;
+        float acc[5][16];
+        if (warp == 15 && lane == 0) put_base(it + 2);
+        if (kLast) {
+            ok = wait_phase(mbar, (uint32_t)(it - 1) & 1u, abort_flag, wait_ns);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t D = tmem + kZColD;
+        }
+        if (kTile) {
 #pragma unroll
-            for (uint32_t ks = 0; ks < 4; ++ks) {
-                const uint32_t kb = ks * 32u, ka = ks * 8u;
-                const uint32_t B = sbase + kZOffB + kb, Bs = sbase + kZOffBs + kb;
-                const uint32_t acc = ks > 0 ? 1u : 0u;
-                // A_0 [B_0 .. B_4]: every accumulator's first product
-                mma_f16_ts(D, tmem + ka, desc_sw128(B), idesc_f16(160), acc);
-                mma_f16_ts(D + 160u, tmem + ka, desc_sw128(B + 160u * 128u), idesc_f16(160), acc);
-                mma_f16_ts(D + 64u, tmem + 32u + ka, desc_sw128(B), idesc_f16(256), 1u);
-                mma_f16_ts(D + 128u, tmem + 64u + ka, desc_sw128(B), idesc_f16(192), 1u);
-                mma_f16_ts(D + 192u, tmem + 96u + ka, desc_sw128(B), idesc_f16(128), 1u);
-                mma_f16_ts(D + 256u, tmem + 128u + ka, desc_sw128(B), idesc_f16(64), 1u);
+            for (int s = 0; s < 4; ++s) tmem_st8(tl + 32u * s + 8u * part, dg[s]);
 #pragma unroll
-                for (uint32_t s = 0; s < 6; ++s)
-                    mma_f16_ts(D + 256u, tmem + 32u * s + ka, desc_sw128(Bs + (5u - s) * kZSlice), idesc_f16(64), 1u);
+            for (int s = 0; s < 2; ++s) {
+                sts_u32x4(a_own + s * kZSliceA, dg[4 + s]);
+                sts_u32x4((a_own ^ 16u) + s * kZSliceA, dg[4 + s] + 4);
             }
-            mma_commit(mbar);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         }
-        // the other stage's last tile was read out before this tile's first
-        // barrier
-        if (tile + gridDim.x < ntiles) load_tile(tile + gridDim.x, stage ^ 1u);
-        const bool ok = wait_phase(mbar, it & 1u, abort_flag, wait_ns);
-        if (__syncthreads_or(!ok)) {
-            failed = true;
-            break;
-        }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (special) {
-            // rows with infinities or NaN: in FP64 from the stage, every
-            // input read before any output is written
-            double2 y[8];
-            if (row_special) row_fp64(xa, rslot, p, mat + 256 * part, y);
-            __syncthreads();
-            if (row_special)
+        if (kLast) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) sts_amp(at(xa, j), y[j].x, y[j].y);
-        }
-        // D_0 is in units of 2^-8 of the scaled row.  Outputs lie within
-        // 2^-60 .. 2^3 of the row's maximum (or are zero)
-        const int32_t back20 = (int32_t)m - (1038 << 20);
-        const bool mid = m > (100u << 20) && m < (1900u << 20);
+            for (int d = 4; d >= 0; --d) {
+                if (d == 4) {
+                    // D_4 + 2^-9 D_5: what this rounds off is far below the result's last digit
+                    float low[16];
+                    tmem_ld16(tl + kZColD + 64u * 5u + 16u * part, reinterpret_cast<uint32_t*>(low));
+                    tmem_ld16(tl + kZColD + 64u * 4u + 16u * part, reinterpret_cast<uint32_t*>(acc[4]));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float acc[5][8];
-#pragma unroll
-            for (int d = 0; d < 5; ++d) tmem_ld8(tl + kZColD + 64u * d + 16u * part + 8u * half, acc[d]);
+                    for (int i = 0; i < 16; ++i) acc[4][i] = fmaf(low[i], 1.0f / 512.0f, acc[4][i]);
+                } else {
+                    tmem_ld16(tl + kZColD + 64u * d + 16u * part, reinterpret_cast<uint32_t*>(acc[d]));
+                }
+            }
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (__syncthreads_or(!ok)) return false;
+        const bool issue = kTile && tid == 0;
+        if (issue) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!kLast && issue)
+            for (uint32_t ks = 0; ks < 4; ++ks) issue_step(ks, tmem, sbase, mbar);
+        if (kLast) {
+            // D_0 is in units of 2^-8 of the scaled row.  Outputs lie within
+            // 2^-60 .. 2^3 of the row's maximum (or are zero)
+            const int32_t back20 = (int32_t)m_prev - (1038 << 20);
+            const bool mid = m_prev > (100u << 20) && m_prev < (1900u << 20);
+            double2* dst = a + bases[(it - 1) % kZBases];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < 8; ++j) {
+                if (issue && (j & 3) == 0) issue_step((uint32_t)j >> 2, tmem, sbase, mbar);
                 float2 c[5], h, l;
 #pragma unroll
                 for (int d = 0; d < 5; ++d) c[d] = make_float2(acc[d][2 * j], acc[d][2 * j + 1]);
                 carry(c, h, l);
-                const uint32_t to = at(xa, 4 * half + j);
+                const uint32_t to = at(out, j);
                 if (mid) {
                     const uint32_t up20 = (uint32_t)back20 + (896u << 20);
                     sts_amp(to, scaled_join_mid(h.x, l.x, up20), scaled_join_mid(h.y, l.y, up20));
-                } else if (!row_special) {
-                    sts_amp(to, scaled_join(h.x, l.x, back20), scaled_join(h.y, l.y, back20));
+                } else {
+                    sts_raw(to, h, l);
                 }
             }
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        double2* dst = a + expand_index(tile, p.tilemap);
+            if (!mid) {
+#pragma unroll 1
+                for (int j = 0; j < 8; ++j) {
+                    const uint32_t to = at(out, j);
+                    const ulonglong2 v = lds_amp(to);
+                    if (m_prev == 0x7FF00000u) {
+                        const double2 y = dst[offset_of(j)];      // written by read_split
+                        sts_amp(to, y.x, y.y);
+                    } else {
+                        sts_amp(to, scaled_join(__uint_as_float((uint32_t)v.x), __uint_as_float((uint32_t)v.y), back20),
+                                scaled_join(__uint_as_float((uint32_t)(v.x >> 32)),
+                                            __uint_as_float((uint32_t)(v.y >> 32)), back20));
+                    }
+                }
+            }
+            if (issue) issue_step(2u, tmem, sbase, mbar);
+            __syncwarp();
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            uint64_t g;
-            uint32_t s;
-            copy_at(k, g, s);
-            dst[g] = X[s];
+            for (int k = 0; k < 8; ++k) {
+                uint64_t g;
+                uint32_t s;
+                element(k, g, s);
+                const ulonglong2 v = lds_amp(out + s * 16u);
+                dst[g] = make_double2(__longlong_as_double((long long)v.x), __longlong_as_double((long long)v.y));
+            }
         }
-    }
+        if (kLast && issue) issue_step(3u, tmem, sbase, mbar);
+        m_prev = m;
+        if (kTile && it + 1 < count) read_split(it + 1);
+        ++it;
+        return true;
+    };
+    using Yes = std::integral_constant<bool, true>;
+    using No = std::integral_constant<bool, false>;
+    step(Yes(), No());
+    while (!failed && it < count) failed = !step(Yes(), Yes());
+    if (!failed) failed = !step(No(), Yes());
     if (failed) {
         // what is in flight lands before the CTA's memory is given up
         cp_async_wait_group<0>();
         if (tid == 0) {
-            drain_phase(mbar, it & 1u);
+            drain_phase(mbar, (uint32_t)(it - 1) & 1u);
             atomicExch(err, 1);
         }
     }
@@ -442,66 +570,46 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
 
 }  // namespace
 
-void z_pass_layout(ZPass& p, const int* tile_pos, uint32_t gate_bits, const int* gate_of)
+void z_pass_layout(ZPass& p, const int* tile_pos, const int* gate_of)
 {
     std::memset(&p, 0, sizeof p);
     p.tilemap.nz = 12;
-    for (int j = 0; j < 12; ++j) {
-        p.tilemap.zpos[j] = tile_pos[j];
-        p.off[j] = uint64_t(1) << tile_pos[j];
-        p.slot[j] = 1u << j;
-    }
-    // rows: the non-gate tile bits, ascending; the three lowest vary within
-    // a phase of 8 lanes and take the three column bits, their own or those
-    // that gate bits leave
-    int r = 0;
-    uint32_t used = 0;
-    int rows[7];
+    uint32_t gate_bits = 0;
+    for (int j = 0; j < 12; ++j) p.tilemap.zpos[j] = tile_pos[j];
+    for (int k = 0; k < 5; ++k) gate_bits |= 1u << gate_of[k];
+    // rows: the non-gate tile bits, ascending.  A warp: the five lowest of
+    // them and the three lowest gates
+    int rows[7], r = 0, wb[8], w = 0;
     for (int j = 0; j < 12; ++j)
         if (!((gate_bits >> j) & 1u)) rows[r++] = j;
+    for (int j = 0; j < 12; ++j)
+        if (j == gate_of[0] || j == gate_of[1] || j == gate_of[2] || std::find(rows, rows + 5, j) != rows + 5)
+            wb[w++] = j;
+    for (int i = 0; i < 8; ++i) {
+        p.off[i] = uint64_t(1) << tile_pos[wb[i]];
+        p.slot[i] = 1u << i;
+    }
+    for (int i = 0; i < 5; ++i) p.row_of[i] = (uint8_t)(std::find(wb, wb + 8, rows[i]) - wb);
+    for (int i = 0; i < 3; ++i) p.gate_of[i] = (uint8_t)(std::find(wb, wb + 8, gate_of[i]) - wb);
+    for (int i = 0; i < 2; ++i) {
+        p.warp[i] = uint64_t(1) << tile_pos[rows[5 + i]];
+        p.warp[2 + i] = uint64_t(1) << tile_pos[gate_of[3 + i]];
+    }
+    // the three lowest rows vary within a phase of 8 lanes and take the three
+    // column bits, their own or those that gate bits leave
+    uint32_t used = 0;
     for (int i = 0; i < 3; ++i)
-        if (rows[i] < 3) used |= 1u << rows[i];
+        if (p.row_of[i] < 3) used |= 1u << p.row_of[i];
     for (int i = 0; i < 3; ++i)
-        if (rows[i] >= 3) {
+        if (p.row_of[i] >= 3) {
             int c = 0;
             while ((used >> c) & 1u) ++c;
             used |= 1u << c;
-            p.slot[rows[i]] ^= 1u << c;
+            p.slot[p.row_of[i]] ^= 1u << c;
         }
-    for (int i = 0; i < 7; ++i) p.row[i] = p.slot[rows[i]];
-    for (int g = 0; g < 32; ++g)
-        for (int k = 0; k < 5; ++k)
-            if ((g >> k) & 1) p.gate[g] ^= (uint16_t)p.slot[gate_of[k]];
 }
 
-void z_pass_image(const double* m, unsigned char* out)
-{
-    uint16_t* img = reinterpret_cast<uint16_t*>(out);
-    auto put = [&](int n, int k, const uint16_t (&d)[6], uint16_t flip) {
-        for (int t = 0; t < 6; ++t)
-            img[(t * kZSlice + tc_sw128_offset((uint32_t)n, (uint32_t)k)) / 2] = d[t] & 0x7FFFu ? d[t] ^ flip : 0;
-    };
-    for (int gp = 0; gp < 32; ++gp)
-        for (int g = 0; g < 32; ++g) {
-            uint16_t d[2][6];
-            for (int c = 0; c < 2; ++c) {
-                double v = m[2 * (gp * 32 + g) + c] * 256.0;
-                for (int t = 0; t < 6; ++t) {
-                    const double q = std::nearbyint(v);
-                    double rounded;
-                    d[c][t] = host_f16_bits(q, &rounded);    // an integer of at most 257: exact
-                    v = (v - q) * 512.0;
-                }
-            }
-            put(2 * gp, 2 * g, d[0], 0);
-            put(2 * gp, 2 * g + 1, d[1], 0x8000u);
-            put(2 * gp + 1, 2 * g, d[1], 0);
-            put(2 * gp + 1, 2 * g + 1, d[0], 0);
-        }
-    std::memcpy(out + 6 * kZSlice, m, 2048 * sizeof(double));
-}
-
-cudaError_t launch_fused_tc_c128(double2* amps, uint64_t total, const ZPass& p, const void* d_image, int* d_err,
+cudaError_t launch_fused_tc_c128(double2* amps, uint64_t total, const ZPass& p, const void* d_mat, int* d_err,
                                  int sm_count, cudaStream_t st, uint64_t wait_ns)
 {
     static std::mutex mu;
@@ -521,9 +629,7 @@ cudaError_t launch_fused_tc_c128(double2* amps, uint64_t total, const ZPass& p, 
     const uint64_t ntiles = total / kZTile;
     if (ntiles == 0) return cudaErrorInvalidValue;
     const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sm_count, ntiles);
-    const auto* img = static_cast<const unsigned char*>(d_image);
-    k_fused_tc_c128<<<grid, kZThreads, kZSmemAlloc, st>>>(amps, ntiles, p, reinterpret_cast<const uint4*>(img),
-                                                         reinterpret_cast<const double2*>(img + 6 * kZSlice), d_err,
+    k_fused_tc_c128<<<grid, kZThreads, kZSmemAlloc, st>>>(amps, ntiles, p, static_cast<const double2*>(d_mat), d_err,
                                                          wait_ns ? wait_ns : kTcDefaultWaitNs);
     return cudaGetLastError();
 }

@@ -272,7 +272,7 @@ bool tc_chain_layout(TcOffsets& offs, bool tma_ok, int conflict_slack, int (*gbi
 void tc_split_map(TcOffsets& offs, int* gbit0);
 // Byte offset of operand element (row r, K index k) in a K-major,
 // SWIZZLE_128B f16 matrix of 128-byte rows (8-row groups of 1024 B).
-inline uint32_t tc_sw128_offset(uint32_t r, uint32_t k)
+constexpr uint32_t tc_sw128_offset(uint32_t r, uint32_t k)
 {
     return (r >> 3) * 1024u + (r & 7u) * 128u + ((((k >> 3) ^ r) & 7u) << 4) + (k & 7u) * 2u;
 }
@@ -300,23 +300,22 @@ void tc_operand_scales(double max_norm, TcOffsets& offs);
 bool tc_block_bounded(const std::complex<double>* m, int dim);
 
 // ---- fused_tc_c128.cu: the same contraction on complex128 states
-// One block per pass.  Tile coordinate x (bit j: the tile's j-th position)
-// lies at amplitude offset OR off[j] and staged slot XOR slot[j].
+// One block per pass.  Element e of a warp's 256 amplitudes (of the warp's
+// part of a tile) lies at the OR of off[i], slot XOR of slot[i], over e's bits i;
+// bit b of a row is bit row_of[b] of e, bit k of a gate state gate_of[k]; bit b
+// of the warp's number (two more row bits, two more gate bits) adds warp[b].
 struct ZPass {
     IndexMap tilemap;
-    uint64_t off[12];
-    uint32_t slot[12];
-    uint32_t row[7];         // slot of row bit r
-    uint16_t gate[32];       // slot of gate state g
+    uint64_t off[8];
+    uint64_t warp[4];
+    uint32_t slot[8];
+    uint8_t row_of[5];
+    uint8_t gate_of[3];
 };
-// gate_bits: the five tile bits that are gates; gate_of[k]: the tile bit of
-// matrix index bit k.
-void z_pass_layout(ZPass& p, const int* tile_pos /* 12, ascending */, uint32_t gate_bits, const int* gate_of);
-// Device data of a pass with the 32x32 complex matrix m (rows of 2-norm <= 1):
-// six digits of the 64x64 real embedding, then m itself.
-constexpr size_t kZImageBytes = 6 * 8192 + 2048 * sizeof(double);
-void z_pass_image(const double* m, unsigned char* out);
-cudaError_t launch_fused_tc_c128(double2* amps, uint64_t total, const ZPass& p, const void* d_image, int* d_err,
+// gate_of[k]: the tile bit of matrix index bit k, ascending.
+void z_pass_layout(ZPass& p, const int* tile_pos /* 12, ascending */, const int* gate_of);
+// d_mat: the pass's 32x32 complex matrix (rows of 2-norm <= 1).
+cudaError_t launch_fused_tc_c128(double2* amps, uint64_t total, const ZPass& p, const void* d_mat, int* d_err,
                                  int sm_count, cudaStream_t st, uint64_t wait_ns);
 
 // ---- state_kernels.cu: construction, conversion, collapse

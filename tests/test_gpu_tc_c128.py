@@ -39,7 +39,7 @@ def _run(amps, m, qubits, n):
 @pytest.mark.parametrize("n,qubits", [
     (12, [0, 1, 2, 3, 4]), (12, [11, 10, 9, 8, 7]), (12, [5, 0, 11, 6, 3]), (12, [11, 2, 9]), (13, [12, 1, 11, 0]),
     (14, [13, 12, 11, 10, 9]), (16, [0, 4, 8, 12, 15]), (17, [1, 0, 2, 16, 15]), (20, [19, 18, 0, 1, 10]),
-    (21, [3, 20, 7, 19, 11])])
+    (21, [3, 20, 7, 19, 11]), (23, [22, 0, 9, 4, 17]), (23, [18, 19, 20, 21, 22])])
 def test_block_matches_numpy(n, qubits):
     rng = np.random.default_rng(n * 100 + len(qubits) + qubits[0])
     amps, m = rand_state(n, rng), rand_unitary(1 << len(qubits), rng)
