@@ -1180,34 +1180,85 @@ static void lower_z_block(q1g_state* s, const std::vector<cd>& mat, const std::v
     });
 }
 
-// Consecutive pair and phase updates (every one run_takes) as tile passes
-// (gate_run.h).  A pass of one op, or one whose ops together touch less than
-// the state where that is what costs (a state beyond the L2: two CX read and
-// write half of it each), goes gate by gate.
-template <typename Stage, typename Emit>
-static void lower_plain_gates(q1g_state* s, const std::vector<GateOp>& ops, Stage&& stage, Emit&& emit)
+// A plain gate (a pair or phase update that run_takes) with its matrix.
+struct PlainGate {
+    GateOp op;
+    SeqGate gate;
+};
+
+// Microseconds of a complex128 tensor-core pass (6.9 per tile of an SM: 0.75 ms
+// at 26 qubits), or of a block's matrix on the host where that is longer.
+static double z_pass_us(uint64_t total)
+{
+    return std::max(5.0 + 6.9 * std::ceil((double)(total >> 12) / 152.0), 100.0);
+}
+
+// A run of plain gates: as tile passes (gate_run.h), or, on complex128
+// states where that is faster by both paths' models, multiplied into blocks of
+// up to five qubits (in FP64 on the host) for the tensor cores.  10 brick
+// layers in us, tile passes and tensor cores: 20 qubits 965 / 412, 22 qubits
+// 3680 / 1101, 24 qubits 15205 / 4758; but with new matrices, which the host
+// multiplies first, 1175 / 1900, 3864 / 2486 and 15453 / 6337, so the line lies
+// at 21 to 22 qubits.  A tile pass of one op, or one whose ops together touch
+// less than the state where that is what costs (a state beyond the L2: two CX
+// read and write half of it each), goes gate by gate.
+template <typename Stage, typename Emit, typename Tc>
+static void lower_plain_gates(q1g_plan* p, q1g_state* s, const std::vector<PlainGate>& run, Stage&& stage, Emit&& emit,
+                              Tc&& tensor_cores)
 {
     const uint64_t total = s->total();
-    std::vector<const GateOp*> list;
-    for (const GateOp& op : ops) list.push_back(&op);
     auto one = [&](const GateOp& op) {
         emit([op](q1g_state* x) { x->apply_op(op, x->amps.as<char>(), x->total()); });
     };
-    if (ops.size() < 2) {
-        for (const GateOp& op : ops) one(op);
+    if (run.size() < 2) {
+        for (const PlainGate& g : run) one(g.op);
         return;
+    }
+    std::vector<const GateOp*> list;
+    for (const PlainGate& g : run) list.push_back(&g.op);
+    double cost = 0.0;
+    const std::vector<RunPass> passes = group_runs(list, s->nbits, total, s->prec, s->fp64_exact, &cost);
+    if (s->prec == kC128 && !s->fp64_exact && p->tensor_cores && s->nbits >= 12 &&
+        cost > 2.0 * z_pass_us(total)) {
+        std::vector<std::vector<int>> bits;
+        for (const PlainGate& g : run) bits.push_back(g.gate.bits);
+        const std::vector<FusedBlock> blocks = fuse(bits, s->nbits, 5);
+        bool faster = (double)blocks.size() * z_pass_us(total) < cost;
+        for (const FusedBlock& b : blocks) faster = faster && b.qubits.size() <= 5;
+        if (faster) {
+            std::vector<SeqGate> gates;
+            for (const PlainGate& g : run) gates.push_back(g.gate);
+            std::vector<std::vector<cd>> mats;
+            for (const FusedBlock& b : blocks) {
+                mats.push_back(block_matrix(b, gates));
+                faster = faster && tc_block_bounded(mats.back().data(), 1 << b.qubits.size());
+            }
+            if (faster) {
+                for (size_t i = 0; i < blocks.size(); ++i) {
+                    const std::vector<int>& q = blocks[i].qubits;
+                    const GateOp op = classify(mats[i].data(), (int)q.size(), q.data(), s->nbits);
+                    if (op.kind == GateOp::Dense) {
+                        tensor_cores();
+                        lower_z_block(s, mats[i], q, stage, emit);
+                    } else if (op.kind != GateOp::Noop) {
+                        one(op);
+                    }
+                }
+                return;
+            }
+        }
     }
     const char* name = s->prec == kC64 ? "gate_run_c64" : s->fp64_exact ? "gate_run_c128_fp64" : "gate_run_c128";
     std::vector<RunOp> table;
-    for (const RunPass& pass : group_runs(list, s->nbits, total, s->prec, s->fp64_exact)) {
+    for (const RunPass& pass : passes) {
         uint64_t touched = 0;
-        for (int i : pass.ops) touched += ops[i].touched(total);
+        for (int i : pass.ops) touched += run[i].op.touched(total);
         if (pass.ops.size() < 2 || (touched <= total && total * s->bsz() > (uint64_t(64) << 20))) {
-            for (int i : pass.ops) one(ops[i]);
+            for (int i : pass.ops) one(run[i].op);
             continue;
         }
         table.clear();
-        for (int i : pass.ops) table.push_back(make_run_op(ops[i], pass.tile));
+        for (int i : pass.ops) table.push_back(make_run_op(run[i].op, pass.tile));
         const RunOp* d = static_cast<const RunOp*>(stage(table.data(), table.size() * sizeof(RunOp)));
         emit([name, tile = pass.tile, d, n = (int)table.size()](q1g_state* x) {
             x->launch(name, 2.0 * x->total() * x->bsz(), [&] {
@@ -1391,9 +1442,9 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
         L.tensor_cores = true;
     };
     // Staging: every pass uploads its matrix or tensor-core image from its own
-    // slice of one pinned buffer into its own slice of L's device buffer.
-    // Nothing may still read that buffer: earlier launches on this stream
-    // precede the copies, those on others are waited for.
+    // slice of a pinned chunk into its own slice of L's chunk of that number.
+    // Nothing may still read those: earlier launches on this stream precede
+    // the copies, those on others are waited for.
     if (p->staged) check_cuda(cudaEventSynchronize(p->staged), "plan staging wait");
     else check_cuda(cudaEventCreateWithFlags(&p->staged, cudaEventDisableTiming), "cudaEventCreate");
     if (L.several_streams || (L.stream && L.stream != s->stream)) check_cuda(cudaDeviceSynchronize(), "plan upload wait");
@@ -1403,13 +1454,22 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
     L.tensor_cores = false;
     size_t staging = 256;
     for (const auto& b : p->blocks) staging += staging_bytes(b);
-    p->hmats.ensure(staging);
-    L.dmats.ensure(staging);
-    size_t staged = 0;
+    size_t chunk = 0, room = 0, staged = 0;      // chunks begun; the last one's size, and its bytes in use
     auto stage = [&](const void* src, size_t sz) -> const void* {
-        if (staged + sz > staging) throw Error(Q1G_ERR_DEVICE, "plan staging buffer too small");
-        char* h = p->hmats.as<char>() + staged;
-        char* d = L.dmats.as<char>() + staged;
+        if (staged + sz > room) {
+            // the first chunk takes what the blocks themselves need; further
+            // ones are for plain gates that became tensor-core blocks
+            const size_t want = std::max(sz, chunk == 0 ? staging : size_t(1) << 18);
+            if (p->hmats.size() == chunk) p->hmats.emplace_back();
+            if (L.dmats.size() == chunk) L.dmats.emplace_back();
+            p->hmats[chunk].ensure(want);
+            L.dmats[chunk].ensure(want);
+            room = std::min(p->hmats[chunk].bytes, L.dmats[chunk].bytes);
+            staged = 0;
+            ++chunk;
+        }
+        char* h = p->hmats[chunk - 1].as<char>() + staged;
+        char* d = L.dmats[chunk - 1].as<char>() + staged;
         std::memcpy(h, src, sz);
         s->h2d(d, h, sz, "upload plan matrix");
         staged += (sz + 255) & ~size_t(255);
@@ -1422,10 +1482,10 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
     };
     // plain gates (pairs and phases) gathered until another kind of block
     // comes, then grouped into tile passes
-    std::vector<GateOp> plain;
+    std::vector<PlainGate> plain;
     auto flush_plain = [&] {
         if (plain.empty()) return;
-        lower_plain_gates(s, plain, stage, emit);
+        lower_plain_gates(p, s, plain, stage, emit, tensor_cores);
         plain.clear();
     };
     for (size_t i = first; i < nb; ++i) {
@@ -1434,7 +1494,7 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
                 GateOp op = classify(gates[g].mat.data(), (int)gates[g].bits.size(), gates[g].bits.data(), s->nbits);
                 if (op.kind == GateOp::Noop) continue;
                 if (run_takes(op)) {
-                    plain.push_back(std::move(op));
+                    plain.push_back({std::move(op), gates[g]});
                 } else {
                     flush_plain();
                     emit([op](q1g_state* x) { x->apply_op(op, x->amps.as<char>(), x->total()); });
@@ -1446,16 +1506,16 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
             prepare(i);
             if (ops[i].kind == GateOp::Noop) continue;
             if (run_takes(ops[i])) {
-                plain.push_back(ops[i]);
+                plain.push_back({ops[i], {bbits[i], bmats[i]}});
                 continue;
             }
         }
         if (p->blocks[i].phase_run) {
             // an uncontrolled gate just before (a Fourier transform's first
             // Hadamard) is the group's first step
-            const GateOp* before = plain.size() == 1 && plain[0].kind == GateOp::Pair && plain[0].map.nz == 1 &&
-                                           plain[0].map.zpos[0] >= 2
-                                       ? &plain[0]
+            const GateOp* before = plain.size() == 1 && plain[0].op.kind == GateOp::Pair &&
+                                           plain[0].op.map.nz == 1 && plain[0].op.map.zpos[0] >= 2
+                                       ? &plain[0].op
                                        : nullptr;
             size_t count = before ? lower_phase_group(p, s, i, before, gates, stage, emit) : 0;
             if (count) {

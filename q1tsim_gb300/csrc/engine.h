@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <deque>
 #include <exception>
 #include <functional>
 #include <utility>
@@ -247,7 +248,7 @@ struct q1g_plan {
     int tc_pairs = 4;
     int tc_max_high = 8;
     int tc_slack = 4;
-    q1g::HostBuf hmats;            // pinned staging of dense matrices
+    std::deque<q1g::HostBuf> hmats;   // pinned staging of what the launches read, in chunks
     cudaEvent_t staged = nullptr;  // last upload of hmats finished
     // The launches of a run, kept with the matrices that they were made from
     // and uploaded: a run with the same matrices (compared byte by byte) on a
@@ -261,7 +262,7 @@ struct q1g_plan {
         size_t first = 0;
         int tiling[4] = {0, 0, 0, 0};     // tensor_cores, tc_pairs, tc_max_high, tc_slack
         std::vector<double> mats;
-        q1g::DevBuf dmats;                // what the launches read
+        std::deque<q1g::DevBuf> dmats;    // what the launches read, in chunks
         bool tensor_cores = false;        // some launch runs on them
         cudaStream_t stream = nullptr;    // of the last run
         bool several_streams = false;     // since the upload

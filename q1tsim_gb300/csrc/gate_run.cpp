@@ -103,7 +103,7 @@ RunTile make_tile(uint64_t S, int bits)
 }  // namespace
 
 std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits, uint64_t total, int prec,
-                                bool fp64_exact)
+                                bool fp64_exact, double* cost_us)
 {
     const int m = (int)ops.size();
     std::vector<Item> items(m);
@@ -199,6 +199,7 @@ std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits
             best.swap(passes);
         }
     }
+    if (cost_us) *cost_us = best_cost;
     return best;
 }
 

@@ -64,8 +64,9 @@ bool run_takes(const GateOp& op);
 // Groups `ops` (in order; every one run_takes and not a Noop) into passes on
 // a state of nbits qubits.  Ops on disjoint positions may change places.
 // prec / fp64_exact choose the cost model's arithmetic rates.
+// *cost_us: the model's time for them.
 std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits, uint64_t total, int prec,
-                                bool fp64_exact);
+                                bool fp64_exact, double* cost_us = nullptr);
 // The op in the tile's local coordinates.
 RunOp make_run_op(const GateOp& op, const RunTile& tile);
 

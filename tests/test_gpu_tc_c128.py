@@ -8,7 +8,7 @@ and roundings far below: 2^-45 of it."""
 import numpy as np
 import pytest
 
-from q1tsim_gb300 import Plan, VectorState
+from q1tsim_gb300 import Plan, Rng, VectorState
 from test_gpu_parity import rand_state, rand_unitary
 
 pytestmark = pytest.mark.gpu
@@ -105,3 +105,34 @@ def test_block_on_several_columns():
     for c in range(after.shape[1]):
         want, top = _apply(np.ascontiguousarray(before[:, c]), m, qubits, n)
         assert np.all(np.abs(after[:, c] - want) <= ROW_TOL * top)
+
+
+@pytest.mark.parametrize("n,shots,depth", [(22, 1, 3), (22, 1, 6), (21, 5, 4)])
+def test_plain_gates_as_blocks(n, shots, depth):
+    """Gates of a plan without fusion, multiplied into blocks where that is
+    faster, against the same plan on the CUDA cores.  Tolerance: 2^-45 per pass
+    of either (both are some 20 passes of 1e-15)."""
+    rng = np.random.default_rng(n + depth)
+    bits, mats = [], []
+    for layer in range(depth):
+        for q in range(n):
+            bits.append([q])
+            mats.append(rand_unitary(2, rng))
+        for q in range(layer % 2, n - 1, 2):
+            bits.append([q, q + 1] if q % 3 else [q + 1, q])
+            kind = rng.integers(3)
+            mats.append(np.eye(4)[[0, 1, 3, 2]] if kind == 0 else np.diag([1, 1, 1, -1]) if kind == 1
+                        else np.diag([1, 1, 1, np.exp(1j * rng.uniform(0, 6))]))
+    flat = np.concatenate([np.ascontiguousarray(m, dtype=np.complex128).ravel().view(np.float64) for m in mats])
+    out = []
+    for tc in (True, False):
+        s = VectorState(n, shots, "c128")
+        s.fill_random_normal(7)
+        if shots > 1:                       # several columns
+            s.measure(3, rng=Rng(1))
+        s.profile(True)
+        s.profile_report(reset=True)
+        s.apply_plan(Plan(n, bits, 0, tensor_cores=tc), flat)
+        assert ("fused_tc_c128" in s.profile_report()) == tc
+        out.append(s.states())
+    assert np.linalg.norm(out[0] - out[1]) <= 40 * 2.0 ** -45 * np.linalg.norm(out[1])
