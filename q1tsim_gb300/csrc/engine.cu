@@ -134,6 +134,11 @@ q1g_state::~q1g_state()
     compact.reset();   // it runs on this state's stream: free it while the stream exists
     unary_plan.reset();
     if (stream) cudaStreamSynchronize(stream);
+    if (copy_stream) {
+        cudaStreamSynchronize(copy_stream);
+        cudaEventDestroy(copy_event);
+        cudaStreamDestroy(copy_stream);
+    }
     for (auto& p : pending) {
         cudaEventDestroy(p.a);
         cudaEventDestroy(p.b);
@@ -535,47 +540,88 @@ void q1g_state::measure_all(const size_t* cbits, size_t ncbits, uint64_t* res, s
         return w;
     };
 
-    // per-run outcome indices: the pinned download of the dense sampler, or
-    // the basis columns of a sparse state
-    std::vector<uint64_t> outc;
-    const uint64_t* h_outc = nullptr;
     if (sparse) {
-        outc.resize(nshots);
-        h_outc = outc.data();
+        // basis columns stay as they are
         uint64_t off = 0;
         for (uint64_t c = 0; c < ncols; ++c) {
-            for (uint64_t r = 0; r < counts[c]; ++r) outc[off + r] = basis[c];
+            const uint64_t w = word_of(basis[c]);
+            for (uint64_t r = off; r < off + counts[c]; ++r) res[r] = (res[r] & mask) | w;
             if (!uniforms) rng->counter += counts[c] + 1;
             off += counts[c];
         }
-        for (uint64_t r = 0; r < nshots; ++r) res[r] = (res[r] & mask) | word_of(outc[r]);
-    } else if (nshots > 0) {
+        if (!collapse) return;
+        // (columns without runs go)
+        std::vector<uint64_t> nb, nc;
+        for (uint64_t c = 0; c < ncols; ++c) {
+            if (counts[c] == 0) continue;
+            nb.push_back(basis[c]);
+            nc.push_back(counts[c]);
+        }
+        basis.swap(nb);
+        counts.swap(nc);
+        norm_pending = false;
+        ncols = basis.size();
+        norms.assign(ncols, 1.0);
+        return;
+    }
+    // Results of 32 bits where they fit: half the download.  Many words (from
+    // 2^17) join the caller's on the device instead: the copies there and back
+    // take 80 + 50 us for 10^6, the first one under the chunk sums, the same loop
+    // on the host 300 to 400.
+    const bool narrow = nbits <= 32;
+    const bool join = nshots >= (uint64_t(1) << 17);
+    const bool narrow_word = !join && (~mask >> 32) == 0;
+    const size_t osz = narrow ? 4 : 8, wsz = narrow_word ? 4 : 8;
+    const std::vector<uint64_t> runs(counts.begin(), counts.end());
+    const char* h_word = nullptr;
+    const char* h_outc = nullptr;
+    if (nshots > 0) {
         const uint64_t chunk = std::min<uint64_t>(N, 256);
         const uint64_t ncc = N / chunk;  // chunks per column
         uint64_t mmax = 0;
         for (auto c : counts) mmax = std::max(mmax, c);
-        const uint64_t scan_tmp = scan_tmp_doubles(ncc) + 1;
-        const uint64_t spc_tmp = 2 * (mmax + 1) + scan_tmp_doubles(mmax + 1) + 1;
-        const uint64_t nd = ncols * ncc + ncols + scan_tmp + nshots + spc_tmp;
+        const uint64_t scan_tmp = scan_tmp_doubles(ncc) + scan_tmp_doubles(mmax + 1) + 1;
+        const uint64_t nspc = uniforms ? 0 : nshots + ncols;
+        // The group sums (1/16 of a complex64 state, 1/16 of a complex128 one)
+        // pay where the shots would read more than that from whole chunks:
+        // from one shot per 32 chunks on; up to 1 GiB of scratch.
+        const uint64_t group_doubles = prec == kC64 ? ncols * ncc * 16 : ncols * ncc * 32;
+        const bool groups = chunk == 256 && nshots * 32 >= ncols * ncc && group_doubles <= (uint64_t(1) << 27);
+        const uint64_t nd = ncols * ncc + ncols + scan_tmp + nshots + 2 * nspc + (groups ? group_doubles : 0) + 16;
         dscratch.ensure(nd * sizeof(double));
         double* d_sums = dscratch.as<double>();
-        double* d_tot = d_sums + ncols * ncc;
+        double* d_group = d_sums + ((ncols * ncc + 15) & ~uint64_t(15));     // 128-byte lines
+        double* d_tot = d_group + (groups ? group_doubles : 0);
         double* d_stmp = d_tot + ncols;
         double* d_u = d_stmp + scan_tmp;
-        double* d_spc = d_u + nshots;
-        uscratch.ensure((2 * nshots + 64 + nshots / 2 + 1) * sizeof(uint64_t));
-        uint64_t* d_out = uscratch.as<uint64_t>();
-        uint64_t* d_word = d_out + nshots;
-        uint64_t* d_cpos = d_word + nshots;
-        uint32_t* d_chunk = reinterpret_cast<uint32_t*>(d_cpos + 64);   // each shot's chunk
+        double* d_e = d_u + nshots;
+        double* d_excl = d_e + nspc;
+        const size_t out_off = (nshots * wsz + 255) & ~size_t(255);
+        const size_t out_bytes = (nshots * osz + 255) & ~size_t(255);
+        uscratch.ensure(out_off + out_bytes + 64 * sizeof(uint64_t));
+        char* d_word = uscratch.as<char>();
+        char* d_out = d_word + out_off;
+        uint64_t* d_cpos = reinterpret_cast<uint64_t*>(d_out + out_bytes);
         h2d(d_cpos, cbit_of_pos.data(), 64 * sizeof(uint64_t), "upload cbits");
+        Spacings sp{};
+        if (!uniforms) {
+            sp = {rng->seed, rng->counter, nspc, d_e, d_excl};
+            rng->counter += nspc;
+        }
+        const bool upload = join && mask != 0;
+        if (upload) {
+            if (!copy_stream) {
+                check_cuda(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking), "cudaStreamCreate");
+                check_cuda(cudaEventCreateWithFlags(&copy_event, cudaEventDisableTiming), "cudaEventCreate");
+            }
+            // (the buffer is free once what is on the stream now has run)
+            check_cuda(cudaEventRecord(copy_event, stream), "copy event");
+            check_cuda(cudaStreamWaitEvent(copy_stream, copy_event, 0), "copy wait");
+        }
         launch("chunk_sums", double(ncols * N * bsz()), [&] {
-            return launch_chunk_sums_dense(amps.p, prec, ncols * N, chunk, d_sums, stream);
+            return launch_chunk_sums_dense(amps.p, prec, ncols * N, chunk, d_sums, groups ? d_group : nullptr, sp,
+                                           stream);
         });
-        for (uint64_t c = 0; c < ncols; ++c)
-            launch("prefix_scan", 2.0 * ncc * sizeof(double), [&] {
-                return launch_exclusive_scan(d_sums + c * ncc, ncc, d_stmp, d_tot + c, stream);
-            });
         std::vector<double> hu;
         if (uniforms) {
             hu.assign(uniforms, uniforms + nshots);
@@ -585,76 +631,91 @@ void q1g_state::measure_all(const size_t* cbits, size_t ncbits, uint64_t* res, s
                 off += counts[c];
             }
             h2d(d_u, hu.data(), nshots * sizeof(double), "upload uniforms");
-        } else {
-            uint64_t off = 0;
-            for (uint64_t c = 0; c < ncols; ++c) {
-                const uint64_t m = counts[c];
-                launch("sorted_uniforms", 0.0, [&] {
-                    return launch_sorted_uniforms(rng->seed, rng->counter, m, d_u + off, d_spc, stream);
-                });
-                rng->counter += m + 1;
-                off += m;
-            }
+        }
+        if (upload) {
+            check_cuda(cudaMemcpyAsync(d_word, res, nshots * wsz, cudaMemcpyHostToDevice, copy_stream), "upload words");
+            h2d_bytes += nshots * wsz;
+            check_cuda(cudaEventRecord(copy_event, copy_stream), "copy event");
+            check_cuda(cudaStreamWaitEvent(stream, copy_event, 0), "copy wait");
         }
         uint64_t off = 0;
         for (uint64_t c = 0; c < ncols; ++c) {
+            // column c's spacings: counts + 1 of them, behind the earlier columns'
+            launch("scans", 2.0 * ncc * sizeof(double), [&] {
+                return launch_scans(d_sums + c * ncc, ncc, d_tot + c, d_excl + off + c, d_e + off + c,
+                                    uniforms ? 0 : counts[c], d_u + off, d_stmp, stream);
+            });
             SampleArgs a{};
             a.amps = col_ptr(c);
             a.prec = prec;
-            a.col_len = N;
             a.chunk = chunk;
             a.excl = d_sums + c * ncc;
             a.nchunks = ncc;
+            a.groups = groups ? d_group + c * (group_doubles / ncols) : nullptr;
             a.total = d_tot + c;
             a.u = d_u + off;
             a.nruns = counts[c];
-            a.outcome = d_out + off;
-            a.word = d_word + off;
+            a.narrow = narrow;
+            a.narrow_word = narrow_word;
+            a.keep = upload ? mask : 0;
+            a.outcome = collapse ? d_out + off * osz : nullptr;
+            a.word = d_word + off * wsz;
             a.nbits = nbits;
             a.d_cbit_of_pos = d_cpos;
-            a.chunk_of = d_chunk + off;
             launch("sample", double(counts[c] * chunk * bsz()), [&] { return launch_sample(a, stream); });
             off += counts[c];
         }
-        hstage.ensure(2 * nshots * sizeof(uint64_t));
-        d2h(hstage.p, d_out, 2 * nshots * sizeof(uint64_t), "download outcomes");
-        sync();
-        h_outc = hstage.as<uint64_t>();
-        if (!collapse) {
-            const uint64_t* h_word = h_outc + nshots;
-            for (uint64_t r = 0; r < nshots; ++r) res[r] = (res[r] & mask) | h_word[r];
-            return;
+        if (join) {
+            if (collapse) {
+                hstage.ensure(out_bytes);
+                d2h(hstage.p, d_out, nshots * osz, "download outcomes");
+            }
+            d2h(res, d_word, nshots * wsz, "download words");
+        } else {
+            hstage.ensure(out_off + out_bytes);
+            d2h(hstage.p, d_word, collapse ? out_off + nshots * osz : nshots * wsz, "download outcomes");
         }
+        sync();
+        h_word = hstage.as<char>();
+        h_outc = join ? h_word : h_word + out_off;
+    }
+    if (!join) {
+        if (narrow_word)
+            for (uint64_t r = 0; r < nshots; ++r)
+                res[r] = (res[r] & mask) | reinterpret_cast<const uint32_t*>(h_word)[r];
+        else
+            for (uint64_t r = 0; r < nshots; ++r)
+                res[r] = (res[r] & mask) | reinterpret_cast<const uint64_t*>(h_word)[r];
     }
     if (!collapse) return;
     // one basis column per distinct (column, outcome), in order: outcomes are
     // sorted within a column, so a column's distinct outcomes are its runs of
     // equal ones (about 10^6 at 30 qubits and 10^6 shots, two for a GHZ
-    // state).  One pass writes the words and appends the runs to
-    // basis/counts, whose capacity carries over between runs: no second
-    // pass, and no zero fill of a resize.  The reservation is capped (2^20
+    // state), appended to basis/counts, whose capacity carries over between
+    // runs (no zero fill of a resize).  The reservation is capped (2^20
     // entries, 8 MB each): many shots of few outcomes keep no large buffer,
     // and more distinct outcomes grow the vectors as they come.
-    const uint64_t* h_word = sparse ? nullptr : h_outc + nshots;
-    const std::vector<uint64_t> runs(counts.begin(), counts.end());
+    auto columns = [&](auto* outc) {
+        uint64_t off = 0;
+        for (uint64_t c = 0; c < runs.size(); ++c) {
+            const uint64_t end = off + runs[c];
+            for (uint64_t r = off; r < end; ++r) {
+                if (r == off || outc[r] != outc[r - 1]) {
+                    basis.push_back(outc[r]);
+                    counts.push_back(1);
+                } else {
+                    ++counts.back();
+                }
+            }
+            off = end;
+        }
+    };
     basis.clear();
     counts.clear();
     basis.reserve(std::min<uint64_t>(nshots, uint64_t(1) << 20));
     counts.reserve(std::min<uint64_t>(nshots, uint64_t(1) << 20));
-    uint64_t off = 0;
-    for (uint64_t c = 0; c < runs.size(); ++c) {
-        const uint64_t end = off + runs[c];
-        for (uint64_t r = off; r < end; ++r) {
-            if (h_word) res[r] = (res[r] & mask) | h_word[r];
-            if (r == off || h_outc[r] != h_outc[r - 1]) {
-                basis.push_back(h_outc[r]);
-                counts.push_back(1);
-            } else {
-                ++counts.back();
-            }
-        }
-        off = end;
-    }
+    if (narrow) columns(reinterpret_cast<const uint32_t*>(h_outc));
+    else columns(reinterpret_cast<const uint64_t*>(h_outc));
     sparse = true;
     norm_pending = false;
     ncols = basis.size();
@@ -1724,7 +1785,7 @@ std::vector<double> q1g_state::measure_norms()
     double* d_sums = s->dscratch.as<double>();
     double* d_norm = d_sums + s->ncols * nch;
     s->launch("column_norms", double(total * s->bsz()), [&] {
-        return launch_chunk_sums_dense(s->amps.p, s->prec, total, chunk, d_sums, s->stream);
+        return launch_chunk_sums_dense(s->amps.p, s->prec, total, chunk, d_sums, nullptr, Spacings{}, s->stream);
     });
     check_cuda(launch_segment_sums(d_sums, s->ncols, nch, d_norm, d_norm + 2 * s->ncols, s->stream),
                "segment_sums");

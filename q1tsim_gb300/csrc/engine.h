@@ -113,6 +113,8 @@ struct q1g_state {
     q1g::HostBuf hstage;    // pinned staging for results
     cudaStream_t stream = nullptr;
     bool own_stream = false;
+    cudaStream_t copy_stream = nullptr;    // of the words' upload in measure_all, made on first use
+    cudaEvent_t copy_event = nullptr;
 
     bool prof = false;
     struct Pending {

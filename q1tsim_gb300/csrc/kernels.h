@@ -360,8 +360,15 @@ cudaError_t launch_chunk_sums(const void* amps, int prec, uint64_t units, uint64
                               const IndexMap& map, double* out, cudaStream_t st);
 // Chunk sums for shot sampling: `chunk` = min(2^n, 256) consecutive
 // amplitudes per chunk, reduced as described in measure_kernels.cu.
+// groups (or null): the chunks' 32 group sums each, in the state's precision.
+// sp: spacings drawn by the same launch.
+struct Spacings {
+    uint64_t seed, counter0, n;    // n draws of the SplitMix64 stream, from counter0
+    double* e;                     // -log1p(-u) of each, twice
+    double* copy;
+};
 cudaError_t launch_chunk_sums_dense(const void* amps, int prec, uint64_t total, uint64_t chunk, double* out,
-                                    cudaStream_t st);
+                                    void* groups, const Spacings& sp, cudaStream_t st);
 // Deterministic per-segment reduction: out[s] = sum of in[s*len .. (s+1)*len).
 // tmp: segment_sums_tmp_doubles(nseg, len) doubles (none for short segments).
 uint64_t segment_sums_tmp_doubles(uint64_t nseg, uint64_t len);
@@ -372,34 +379,33 @@ cudaError_t launch_segment_sums(const double* in, uint64_t nseg, uint64_t len, d
 uint64_t scan_tmp_doubles(uint64_t n);
 cudaError_t launch_exclusive_scan(double* data, uint64_t n, double* tmp, double* total_out,
                                   cudaStream_t st);
-// Ascending uniforms by normalised exponential spacings from the SplitMix64
-// stream (seed, counter0): out[j] = S_j / S_m, S_j = sum_{k<=j} -log1p(-u_k),
-// for j < m, drawing m+1 uniforms.
-// tmp: 2*(m+1) + scan_tmp_doubles(m+1) + 1 doubles.
-cudaError_t launch_sorted_uniforms(uint64_t seed, uint64_t counter0, uint64_t m, double* out,
-                                   double* tmp, cudaStream_t st);
-// One warp per run: outcome[r] = first index i of the column with inclusive
-// prefix > u[r] * total, found through the chunk prefix (excl), a warp scan
-// of the chunk's group sums and a scan of the group; word[r] = classical
-// word of the outcome.  `chunk` must be the one used for the chunk sums.
+// A column's chunk sums to their exclusive prefix and total, and, for m > 0, its
+// m + 1 spacings (twice: e, and excl, which is overwritten) to m ascending
+// uniforms: u[j] = S_j / S_m, S_j = the sum of e[0..j].
+// tmp: scan_tmp_doubles(nchunks) + scan_tmp_doubles(m + 1) + 1 doubles.
+cudaError_t launch_scans(double* sums, uint64_t nchunks, double* total_out, double* excl, const double* e, uint64_t m,
+                         double* u, double* tmp, cudaStream_t st);
+// outcome[r] = first index i of the column with inclusive prefix > u[r] *
+// total, found through the chunk prefix (excl), a warp scan of the chunk's group
+// sums and a scan of the group; word[r] = classical word of the outcome.
+// `chunk` must be the one used for the chunk sums.
 struct SampleArgs {
     const void* amps;       // the column
     int prec;
-    uint64_t col_len;       // 2^n
     uint64_t chunk;
     const double* excl;     // exclusive chunk prefix, nchunks entries
     uint64_t nchunks;
+    const void* groups;     // the column's group sums (launch_chunk_sums_dense), or null
     const double* total;    // device scalar
-    const double* u;        // sorted uniforms of the column's runs
+    const double* u;        // the column's runs' uniforms
     uint64_t nruns;
-    uint64_t* outcome;      // per run
-    uint64_t* word;         // per run
+    bool narrow;            // 32-bit outcomes
+    bool narrow_word;       // 32-bit words
+    uint64_t keep;          // bits of a (64-bit) word's old value that stay
+    void* outcome;          // per run, or null
+    void* word;             // per run
     int nbits;
     const uint64_t* d_cbit_of_pos;  // classical bit mask for each bit position
-    // nruns device words for each shot's chunk: with it the shots' chunks
-    // come from one merge of the sorted targets with the prefix (a
-    // separate launch) instead of a search per shot; nullptr: the search
-    uint32_t* chunk_of;
 };
 cudaError_t launch_sample(const SampleArgs& a, cudaStream_t st);
 // ---- batch.cu: many circuits in one persistent launch (complex64)

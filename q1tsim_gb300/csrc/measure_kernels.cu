@@ -161,13 +161,13 @@ k_scan_tiles(double* data, uint64_t n, const double* offsets)
 
 // ------------------------------------------------- sorted uniforms
 
-__global__ void k_exp_spacings(uint64_t seed, uint64_t counter0, uint64_t n, double* e, double* copy)
+// Blocks `first`, first + step, ..: spacing k of the stream for k < sp.n.
+__device__ void exp_spacings(const Spacings& sp, uint64_t first, uint64_t step)
 {
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    for (uint64_t k = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride) {
-        const double v = -log1p(-stream_uniform(seed, counter0 + k));
-        e[k] = v;
-        copy[k] = v;
+    for (uint64_t k = first * blockDim.x + threadIdx.x; k < sp.n; k += step * blockDim.x) {
+        const double v = -log1p(-stream_uniform(sp.seed, sp.counter0 + k));
+        sp.e[k] = v;
+        sp.copy[k] = v;
     }
 }
 
@@ -180,6 +180,71 @@ __global__ void k_normalise_spacings(const double* excl, const double* e, const 
         out[j] = (excl[j] + e[j]) / t;
 }
 
+// A column's two scans in common launches, each in the order of the kernels
+// above: its chunk sums (in place, with their total) and its spacings, which are
+// normalised to u on the way out.  Both have at most kScanTile tiles.
+struct ScanPair {
+    double* sums;
+    uint64_t nchunks;
+    double* total;
+    double* excl;
+    const double* e;
+    uint64_t m;
+    double* u;
+    double* tmp;          // tile sums: those of the chunk sums, the spacings', the spacings' total
+    uint32_t sum_tiles, spc_tiles;
+};
+
+__device__ void normalise_spacings(const ScanPair& s, uint64_t j0, uint64_t n, double total)
+{
+    for (uint64_t j = j0 + threadIdx.x; j < min(j0 + n, s.m); j += blockDim.x) s.u[j] = (s.excl[j] + s.e[j]) / total;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_pair_small(ScanPair s)
+{
+    __shared__ double tot;
+    if (blockIdx.x == 0) {
+        tile_scan(s.sums, s.nchunks, 0, 0.0, &tot);
+        if (threadIdx.x == 0) *s.total = tot;
+    } else {
+        tile_scan(s.excl, s.m + 1, 0, 0.0, &tot);
+        normalise_spacings(s, 0, s.m, tot);
+    }
+}
+
+__device__ double tile_total(const double* data, uint64_t n, uint64_t t0)
+{
+    __shared__ double red[32];
+    double acc = 0.0;
+    for (uint64_t j = threadIdx.x; j < kScanTile; j += blockDim.x)
+        if (t0 + j < n) acc += data[t0 + j];
+    return block_sum(acc, red);
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_pair_tile_sums(ScanPair s)
+{
+    const bool sums = blockIdx.x < s.sum_tiles;
+    const uint64_t t0 = uint64_t(sums ? blockIdx.x : blockIdx.x - s.sum_tiles) * kScanTile;
+    const double v = sums ? tile_total(s.sums, s.nchunks, t0) : tile_total(s.excl, s.m + 1, t0);
+    if (threadIdx.x == 0) s.tmp[blockIdx.x] = v;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_pair_scan_sums(ScanPair s)
+{
+    __shared__ double tot;
+    const bool sums = blockIdx.x == 0;
+    tile_scan(sums ? s.tmp : s.tmp + s.sum_tiles, sums ? s.sum_tiles : s.spc_tiles, 0, 0.0, &tot);
+    if (threadIdx.x == 0) *(sums ? s.total : s.tmp + s.sum_tiles + s.spc_tiles) = tot;
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_pair_scan_tiles(ScanPair s)
+{
+    const bool sums = blockIdx.x < s.sum_tiles;
+    const uint64_t t0 = uint64_t(sums ? blockIdx.x : blockIdx.x - s.sum_tiles) * kScanTile;
+    tile_scan(sums ? s.sums : s.excl, sums ? s.nchunks : s.m + 1, t0, s.tmp[blockIdx.x], nullptr);
+    if (!sums) normalise_spacings(s, t0, kScanTile, s.tmp[s.sum_tiles + s.spc_tiles]);
+}
+
 // ----------------------------------------------------------- sampling
 //
 // Outcome probabilities are summed hierarchically, with the same arithmetic
@@ -190,88 +255,114 @@ __global__ void k_normalise_spacings(const double* excl, const double* e, const 
 // search on that prefix, its group by an FP64 warp scan of the chunk's 32
 // group sums, and its amplitude by a sequential scan of the group.
 
-// One warp per chunk of `chunk` (<= 256) amplitudes.
+// One warp per chunk of `chunk` (<= 256) amplitudes.  groups (or null): the 32
+// group sums of each chunk, for the sampler.  The first sp_blocks blocks draw
+// the spacings of the sorted uniforms instead: those are bound by the FP64
+// pipe (a log1p each; 10^6 of them 105 us alone), the sums by HBM, so they
+// hide under a large state's sums and cost a small one no launch.
 template <typename T>
 __global__ void __launch_bounds__(256)
-k_chunk_sums_dense(const T* __restrict__ a, uint64_t nchunks, uint64_t chunk, double* out)
+k_chunk_sums_dense(const T* __restrict__ a, uint64_t nchunks, uint64_t chunk, double* out,
+                   typename ProbT<T>::R* __restrict__ groups, Spacings sp, unsigned sp_blocks)
 {
     using R = typename ProbT<T>::R;
+    if (blockIdx.x < sp_blocks) {
+        exp_spacings(sp, blockIdx.x, sp_blocks);
+        return;
+    }
     const int lane = threadIdx.x & 31;
-    const uint64_t warps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
-    for (uint64_t c = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += warps) {
+    const uint64_t warps = (uint64_t(gridDim.x - sp_blocks) * blockDim.x) >> 5;
+    for (uint64_t c = (uint64_t(blockIdx.x - sp_blocks) * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += warps) {
         R p[8];
         group_probs(a, c * chunk, chunk, lane, p);
-        const double s = chunk_total(group_sum(p), lane);
+        const R g = group_sum(p);
+        if (groups) groups[c * 32 + lane] = g;
+        const double s = chunk_total(g, lane);
         if (lane == 0) out[c] = s;
     }
 }
 
-template <typename T>
+// A warp takes 32 consecutive shots.  Each lane finds its shot's chunk (the
+// largest c with excl[c] <= target) by a binary search: the shots are sorted, so
+// the lanes' probes share their cache lines.  Then the warp finds the shots'
+// groups one after the other by a scan of the chunk's 32 group sums, and each
+// lane its shot's amplitude in its group and its word.  With the group sums from
+// memory (kGroups) a shot reads 128 + 64 bytes of complex64 instead of the
+// chunk's 2 KB.  10^6 shots of 29 qubits: 627 us with one shot per warp at a
+// time (its amplitude and word found by one lane) and a merge for the chunks;
+// 113 us now.
+template <typename T, bool kGroups>
 __global__ void __launch_bounds__(256)
 k_sample(SampleArgs s)
 {
-    // one warp per shot, warps looping over the shots (a few blocks per SM
-    // rather than one short-lived block per eight shots)
-    const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
-    for (uint64_t r = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < s.nruns; r += nwarps) {
-        uint64_t idx;
-        if (sample_one((const T*)s.amps, s.chunk, s.excl, s.nchunks, *s.total, s.u[r], threadIdx.x & 31, &idx)) {
-            s.outcome[r] = idx;
-            s.word[r] = outcome_word(idx, s.nbits, s.d_cbit_of_pos);
-        }
-    }
-}
-
-// The chunk of every shot of a column: the largest c with excl[c] <=
-// target(u[r]), for sorted u, found by one merge of the targets with the
-// chunk prefix (excl first on ties).  The merge is cut into spans of
-// kMergeSpan steps (merge path): thread t finds where its span starts by a
-// binary search on its diagonal and walks it, so that every thread does the
-// same work whatever the distribution of the shots over the chunks.
-constexpr uint64_t kMergeSpan = 32;
-
-__global__ void k_locate_chunks(const double* __restrict__ excl, uint64_t nchunks, const double* __restrict__ u,
-                                const double* total_p, uint64_t nruns, uint32_t* __restrict__ chunk_of)
-{
-    const uint64_t d0 = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) * kMergeSpan;
-    const uint64_t len = nchunks + nruns;
-    if (d0 >= len) return;
-    const double total = *total_p;
-    // largest i in [max(0, d0 - nruns), min(d0, nchunks)] whose first i
-    // prefixes all precede the first d0 - i targets
-    uint64_t lo = d0 > nruns ? d0 - nruns : 0, hi = d0 < nchunks ? d0 : nchunks;
-    while (lo < hi) {
-        const uint64_t i = (lo + hi + 1) >> 1;     // candidate: excl[i-1] precedes target[d0-i]
-        const uint64_t j = d0 - i;
-        if (j >= nruns || excl[i - 1] <= shot_target(u[j], total)) lo = i;
-        else hi = i - 1;
-    }
-    uint64_t i = lo, j = d0 - lo;
-    const uint64_t end = d0 + kMergeSpan < len ? d0 + kMergeSpan : len;
-    double tj = j < nruns ? shot_target(u[j], total) : 0.0;
-    for (uint64_t d = d0; d < end; ++d) {
-        if (j < nruns && (i >= nchunks || excl[i] > tj)) {
-            chunk_of[j] = (uint32_t)(i - 1);   // excl[0] = 0 precedes every target
-            ++j;
-            if (j < nruns) tj = shot_target(u[j], total);
-        } else {
-            ++i;
-        }
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256)
-k_sample_located(SampleArgs s, const uint32_t* __restrict__ chunk_of)
-{
-    const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
+    using R = typename ProbT<T>::R;
+    constexpr int kAhead = kGroups ? 8 : 2;      // chunks read at once
+    const T* a = static_cast<const T*>(s.amps);
+    const R* groups = static_cast<const R*>(s.groups);
+    const int lane = threadIdx.x & 31;
+    const uint64_t warps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
     const double total = *s.total;
-    for (uint64_t r = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < s.nruns; r += nwarps) {
-        uint64_t idx;
-        const double target = shot_target(s.u[r], total);
-        if (sample_in_chunk((const T*)s.amps, s.chunk, s.excl, chunk_of[r], target, threadIdx.x & 31, &idx)) {
-            s.outcome[r] = idx;
-            s.word[r] = outcome_word(idx, s.nbits, s.d_cbit_of_pos);
+    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; b * 32 < s.nruns; b += warps) {
+        const uint64_t r = b * 32 + lane;
+        const int count = (int)min(s.nruns - b * 32, uint64_t(32));
+        const double target = lane < count ? shot_target(s.u[r], total) : 0.0;
+        uint64_t lo = 0, hi = s.nchunks;
+        while (hi - lo > 1) {
+            const uint64_t mid = (lo + hi) >> 1;
+            if (s.excl[mid] <= target) lo = mid;
+            else hi = mid;
+        }
+        // the target's offset into the chunk, in the state's precision (it is
+        // at most the chunk's mass)
+        const R offset = (R)(target - s.excl[lo]);
+        int group = 0;
+        R local = R(0);
+        for (int k0 = 0; k0 < count; k0 += kAhead) {
+            R gs[kAhead];
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                const uint64_t c = __shfl_sync(0xffffffffu, lo, k0 + k);
+                if (kGroups) {
+                    gs[k] = groups[c * 32 + lane];
+                } else {
+                    R p[8];
+                    group_probs(a, c * s.chunk, s.chunk, lane, p);
+                    gs[k] = group_sum(p);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) {
+                // the group sums scanned in the state's precision (the chunk
+                // sums add them in the same order, chunk_total)
+                const R t = __shfl_sync(0xffffffffu, offset, k0 + k);
+                const R incl = warp_incl_scan(gs[k], lane);
+                const unsigned hit = __ballot_sync(0xffffffffu, gs[k] > R(0) && incl > t);
+                const unsigned nz = __ballot_sync(0xffffffffu, gs[k] > R(0));
+                const int owner = hit ? __ffs(hit) - 1 : nz ? 31 - __clz(nz) : 0;
+                const R before = __shfl_sync(0xffffffffu, incl - gs[k], owner);
+                if (lane == k0 + k) {
+                    group = owner;
+                    // past the end: the group's last nonzero amplitude
+                    local = hit ? t - before : R(INFINITY);
+                }
+            }
+        }
+        if (lane >= count) continue;
+        const uint64_t i0 = lo * s.chunk + (uint64_t)group * 8;
+        R p[8];
+        group_probs(a, lo * s.chunk, s.chunk, group, p);
+        const int e = pick_in_group(p, local);
+        const uint64_t idx = i0 + (uint64_t)e;
+        const uint64_t word = outcome_word(idx, s.nbits, s.d_cbit_of_pos);
+        if (s.outcome) {
+            if (s.narrow) static_cast<uint32_t*>(s.outcome)[r] = (uint32_t)idx;
+            else static_cast<uint64_t*>(s.outcome)[r] = idx;
+        }
+        if (s.narrow_word) {
+            static_cast<uint32_t*>(s.word)[r] = (uint32_t)word;
+        } else {
+            uint64_t* w = static_cast<uint64_t*>(s.word) + r;
+            *w = s.keep ? (*w & s.keep) | word : word;
         }
     }
 }
@@ -362,14 +453,17 @@ cudaError_t launch_chunk_sums(const void* amps, int prec, uint64_t units, uint64
 }
 
 cudaError_t launch_chunk_sums_dense(const void* amps, int prec, uint64_t total, uint64_t chunk, double* out,
-                                    cudaStream_t st)
+                                    void* groups, const Spacings& sp, cudaStream_t st)
 {
     const uint64_t nchunks = total / chunk;
-    const unsigned grid = cap_grid((nchunks * 32 + 255) / 256);
+    const unsigned blocks = cap_grid((nchunks * 32 + 255) / 256);
+    const unsigned sp_blocks = (unsigned)std::min<uint64_t>((sp.n + 255) / 256, 152);
     if (prec == kC128)
-        k_chunk_sums_dense<double2><<<grid, 256, 0, st>>>((const double2*)amps, nchunks, chunk, out);
+        k_chunk_sums_dense<double2><<<sp_blocks + blocks, 256, 0, st>>>((const double2*)amps, nchunks, chunk, out,
+                                                                       (double*)groups, sp, sp_blocks);
     else
-        k_chunk_sums_dense<float2><<<grid, 256, 0, st>>>((const float2*)amps, nchunks, chunk, out);
+        k_chunk_sums_dense<float2><<<sp_blocks + blocks, 256, 0, st>>>((const float2*)amps, nchunks, chunk, out,
+                                                                      (float*)groups, sp, sp_blocks);
     return cudaGetLastError();
 }
 
@@ -424,22 +518,27 @@ cudaError_t launch_exclusive_scan(double* data, uint64_t n, double* tmp, double*
     return cudaGetLastError();
 }
 
-cudaError_t launch_sorted_uniforms(uint64_t seed, uint64_t counter0, uint64_t m, double* out,
-                                   double* tmp, cudaStream_t st)
+cudaError_t launch_scans(double* sums, uint64_t nchunks, double* total_out, double* excl, const double* e, uint64_t m,
+                         double* u, double* tmp, cudaStream_t st)
 {
-    if (m == 0) return cudaSuccess;
-    const uint64_t n = m + 1;
-    double* e = tmp;                 // n doubles: the spacings
-    double* work = tmp + n;          // n doubles: scanned copy
-    double* stmp = tmp + 2 * n;      // scan scratch, last slot = total
-    const unsigned grid = cap_grid((n + 255) / 256);
-    k_exp_spacings<<<grid, 256, 0, st>>>(seed, counter0, n, e, work);
-    cudaError_t err = cudaGetLastError();
+    const uint64_t ta = (nchunks + kScanTile - 1) / kScanTile, tb = (m + kScanTile) / kScanTile;
+    if (m > 0 && ta <= kScanTile && tb <= kScanTile) {
+        const ScanPair s{sums, nchunks, total_out, excl, e, m, u, tmp, (uint32_t)ta, (uint32_t)tb};
+        if (ta == 1 && tb == 1) {
+            k_pair_small<<<2, kScanThreads, 0, st>>>(s);
+            return cudaGetLastError();
+        }
+        k_pair_tile_sums<<<(unsigned)(ta + tb), kScanThreads, 0, st>>>(s);
+        k_pair_scan_sums<<<2, kScanThreads, 0, st>>>(s);
+        k_pair_scan_tiles<<<(unsigned)(ta + tb), kScanThreads, 0, st>>>(s);
+        return cudaGetLastError();
+    }
+    cudaError_t err = launch_exclusive_scan(sums, nchunks, tmp, total_out, st);
+    if (err != cudaSuccess || m == 0) return err;
+    double* total = tmp + scan_tmp_doubles(m + 1);
+    err = launch_exclusive_scan(excl, m + 1, tmp, total, st);
     if (err != cudaSuccess) return err;
-    double* total = stmp + scan_tmp_doubles(n);
-    err = launch_exclusive_scan(work, n, stmp, total, st);
-    if (err != cudaSuccess) return err;
-    k_normalise_spacings<<<cap_grid((m + 255) / 256), 256, 0, st>>>(work, e, total, m, out);
+    k_normalise_spacings<<<cap_grid((m + 255) / 256), 256, 0, st>>>(excl, e, total, m, u);
     return cudaGetLastError();
 }
 
@@ -476,24 +575,18 @@ cudaError_t launch_scale_columns(void* amps, int prec, uint64_t col_len, uint64_
 cudaError_t launch_sample(const SampleArgs& a, cudaStream_t st)
 {
     if (a.nruns == 0) return cudaSuccess;
-    // 8 warps per block, 8 blocks per SM (64 warps): every SM full, each
-    // warp taking every nwarps-th shot
-    const uint64_t blocks = (a.nruns + 7) / 8;
-    const unsigned grid = (unsigned)std::min<uint64_t>(blocks, 152ull * 8);
-    if (a.chunk_of && a.nchunks < (uint64_t(1) << 32)) {
-        const uint64_t spans = (a.nchunks + a.nruns + kMergeSpan - 1) / kMergeSpan;
-        k_locate_chunks<<<(unsigned)((spans + 255) / 256), 256, 0, st>>>(a.excl, a.nchunks, a.u, a.total, a.nruns,
-                                                                          a.chunk_of);
-        if (a.prec == kC128)
-            k_sample_located<double2><<<grid, 256, 0, st>>>(a, a.chunk_of);
-        else
-            k_sample_located<float2><<<grid, 256, 0, st>>>(a, a.chunk_of);
-        return cudaGetLastError();
+    // 8 warps of 32 shots per block, at most 8 blocks per SM (64 warps); few
+    // shots go one warp to a block, over all SMs
+    const uint64_t warps = (a.nruns + 31) / 32;
+    const unsigned threads = warps <= 152 ? 32 : 256;
+    const unsigned grid = (unsigned)std::min<uint64_t>((warps * 32 + threads - 1) / threads, 152ull * 8);
+    if (a.prec == kC128) {
+        if (a.groups) k_sample<double2, true><<<grid, threads, 0, st>>>(a);
+        else k_sample<double2, false><<<grid, threads, 0, st>>>(a);
+    } else {
+        if (a.groups) k_sample<float2, true><<<grid, threads, 0, st>>>(a);
+        else k_sample<float2, false><<<grid, threads, 0, st>>>(a);
     }
-    if (a.prec == kC128)
-        k_sample<double2><<<grid, 256, 0, st>>>(a);
-    else
-        k_sample<float2><<<grid, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -110,12 +110,11 @@ void sample_shots_noalloc(const void* d_amps, int precision, size_t nr_bits, con
     // call is read; the chunk sums, prefix and total are rewritten too
     k_store_cbit_table<<<1, 64, 0, st>>>(d_cpos, table);
     check_cuda(cudaGetLastError(), "store classical-bit table");
-    check_cuda(launch_chunk_sums_dense(d_amps, precision, n, chunk, d_sums, st), "chunk_sums");
+    check_cuda(launch_chunk_sums_dense(d_amps, precision, n, chunk, d_sums, nullptr, Spacings{}, st), "chunk_sums");
     check_cuda(launch_exclusive_scan(d_sums, nchunks, d_stmp, d_total, st), "prefix_scan");
     SampleArgs a{};
     a.amps = d_amps;
     a.prec = precision;
-    a.col_len = n;
     a.chunk = chunk;
     a.excl = d_sums;
     a.nchunks = nchunks;

@@ -82,6 +82,24 @@ __device__ __forceinline__ R group_sum(const R p[8])
     return s;
 }
 
+// The first amplitude of a group whose inclusive prefix exceeds `local`, or the
+// last nonzero one.
+template <typename R>
+__device__ __forceinline__ int pick_in_group(const R p[8], R local)
+{
+    int e_pick = -1, e_last = 0;
+    R run = R(0);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        run = padd(run, p[e]);
+        if (p[e] > R(0)) {
+            e_last = e;
+            if (e_pick < 0 && run > local) e_pick = e;
+        }
+    }
+    return e_pick < 0 ? e_last : e_pick;
+}
+
 // Inclusive prefix of v over the warp's lanes, in v's precision: the order
 // in which the sampler adds a chunk's 32 group sums.
 template <typename R>
@@ -184,18 +202,7 @@ __device__ bool sample_in_chunk(const T* a, uint64_t chunk, const double* excl, 
         local = R(INFINITY);   // past the end: take the group's last nonzero amplitude
     }
     if (lane != owner) return false;
-    int e_pick = -1, e_last = 0;
-    R run = R(0);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        run = padd(run, p[e]);
-        if (p[e] > R(0)) {
-            e_last = e;
-            if (e_pick < 0 && run > local) e_pick = e;
-        }
-    }
-    if (e_pick < 0) e_pick = e_last;
-    *idx = i0 + (uint64_t)lane * 8 + (uint64_t)e_pick;
+    *idx = i0 + (uint64_t)lane * 8 + (uint64_t)pick_in_group(p, local);
     return true;
 }
 
