@@ -8,6 +8,10 @@
 //   complex128: 512-amplitude tiles of 16-byte amplitudes, double-float
 //               products as in the complex128 pair kernel (df64.cuh); a unit
 //               with an amplitude outside the split's range is done in FP64.
+// The matrix is a kernel parameter (3 KB at most): nothing is uploaded and the
+// host waits for nothing.  A small state's few tiles go one warp to a block,
+// over the SMs: a 3-qubit complex128 block at 13 qubits (16 tiles) took 27.9 us
+// between events with 16 warps in one CTA, 18.5 us so.
 #include <algorithm>
 #include <mutex>
 #include <set>
@@ -23,7 +27,18 @@ namespace {
 
 constexpr int kTiledThreads = 512;
 constexpr int kTiledWarps = kTiledThreads / 32;
-constexpr size_t kTiledStageBytes = size_t(kTiledWarps) * 8192;
+constexpr size_t kTiledWarpBytes = 8192;                 // a warp's stage
+constexpr size_t kTiledStageBytes = kTiledWarps * kTiledWarpBytes;
+
+template <int TB>
+struct TiledMatC64 {
+    float2 m[1 << (2 * TB)];
+};
+template <int TB>
+struct TiledMatC128 {
+    float4 terms[2 << (2 * TB)];
+    double2 m[1 << (2 * TB)];
+};
 
 __device__ __forceinline__ void copy_tile_words(WarpTile& dst, const WarpTile& src)
 {
@@ -35,18 +50,19 @@ __device__ __forceinline__ void copy_tile_words(WarpTile& dst, const WarpTile& s
 
 template <int TB>
 __global__ void __launch_bounds__(kTiledThreads, 1)
-k_dense_tiled_c64(float2* a, uint64_t total, const __grid_constant__ WarpTile tile, const float2* __restrict__ gmat)
+k_dense_tiled_c64(float2* a, uint64_t total, const __grid_constant__ WarpTile tile,
+                  const __grid_constant__ TiledMatC64<TB> gmat)
 {
     constexpr int D = 1 << TB;
     __shared__ WarpTile w;
     __shared__ float2 mat[D * D];
     extern __shared__ float2 stage_c64[];
     copy_tile_words(w, tile);
-    for (int e = threadIdx.x; e < D * D; e += blockDim.x) mat[e] = gmat[e];
+    for (int e = threadIdx.x; e < D * D; e += blockDim.x) mat[e] = gmat.m[e];
     __syncthreads();
     const int warp = threadIdx.x >> 5;
-    tiled_dense_c64<TB, false>(a, total, w, mat, stage_c64 + warp * 1024, (uint64_t)blockIdx.x * kTiledWarps + warp,
-                        (uint64_t)gridDim.x * kTiledWarps);
+    tiled_dense_c64<TB, false>(a, total, w, mat, stage_c64 + warp * 1024,
+                               ((uint64_t)blockIdx.x * blockDim.x >> 5) + warp, (uint64_t)gridDim.x * blockDim.x >> 5);
 }
 
 // Shared-memory load of one 16-byte term, kept at its use.
@@ -95,7 +111,7 @@ __device__ __forceinline__ void dot_terms(const float4* t, const float2* bh, con
 template <int TB>
 __global__ void __launch_bounds__(kTiledThreads, 1)
 k_dense_tiled_c128(double2* a, uint64_t total, const __grid_constant__ WarpTile tile,
-                   const float4* __restrict__ gterms, const double2* __restrict__ gmat)
+                   const __grid_constant__ TiledMatC128<TB> gmat)
 {
     constexpr int D = 1 << TB;
     constexpr int U = 16 >> TB;   // units per lane in a 512-amplitude tile
@@ -104,8 +120,8 @@ k_dense_tiled_c128(double2* a, uint64_t total, const __grid_constant__ WarpTile 
     __shared__ double2 mat[D * D];
     extern __shared__ ulonglong2 stage_c128[];
     copy_tile_words(w, tile);
-    for (int e = threadIdx.x; e < 2 * D * D; e += blockDim.x) terms[e] = gterms[e];
-    for (int e = threadIdx.x; e < D * D; e += blockDim.x) mat[e] = gmat[e];
+    for (int e = threadIdx.x; e < 2 * D * D; e += blockDim.x) terms[e] = gmat.terms[e];
+    for (int e = threadIdx.x; e < D * D; e += blockDim.x) mat[e] = gmat.m[e];
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     ulonglong2* stage = stage_c128 + warp * 512;
@@ -116,7 +132,8 @@ k_dense_tiled_c128(double2* a, uint64_t total, const __grid_constant__ WarpTile 
 #pragma unroll
     for (int b = 0; b < 5; ++b)
         if ((lane >> b) & 1) pl ^= w.wbit[b];
-    for (uint64_t t = (uint64_t)blockIdx.x * kTiledWarps + warp; t < tiles; t += (uint64_t)gridDim.x * kTiledWarps) {
+    const uint64_t warps = (uint64_t)gridDim.x * blockDim.x >> 5;
+    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x >> 5) + warp; t < tiles; t += warps) {
         uint32_t gb[4], sb[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
@@ -236,80 +253,62 @@ bool dense_tiled_applies(int prec, int nbits, int t, const IndexMap& map, bool f
     return t >= 1 && t <= 4 && nbits >= 10 && (t >= 3 || map.zpos[0] <= 1);
 }
 
-size_t dense_tiled_matrix_bytes(int prec, int t)
+template <int TB>
+static cudaError_t launch_tiled_c64(void* amps, uint64_t total, const WarpTile& w, const double* m, unsigned grid,
+                                    unsigned warps, cudaStream_t st)
 {
-    const size_t d2 = size_t(1) << (2 * t);
-    return prec == kC128 ? 2 * d2 * sizeof(float4) + d2 * sizeof(double2) : d2 * sizeof(float2);
+    const cudaError_t e = opt_in(k_dense_tiled_c64<TB>);
+    if (e != cudaSuccess) return e;
+    TiledMatC64<TB> g;
+    for (int i = 0; i < 1 << (2 * TB); ++i) g.m[i] = make_float2((float)m[2 * i], (float)m[2 * i + 1]);
+    k_dense_tiled_c64<TB><<<grid, 32 * warps, warps * kTiledWarpBytes, st>>>((float2*)amps, total, w, g);
+    return cudaGetLastError();
 }
 
-void dense_tiled_matrix(int prec, int t, const double* m, void* out)
+template <int TB>
+static cudaError_t launch_tiled_c128(void* amps, uint64_t total, const WarpTile& w, const double* m, unsigned grid,
+                                     unsigned warps, cudaStream_t st)
 {
-    const size_t d = size_t(1) << t;
-    if (prec != kC128) {
-        float2* f = static_cast<float2*>(out);
-        for (size_t e = 0; e < d * d; ++e) f[e] = make_float2((float)m[2 * e], (float)m[2 * e + 1]);
-        return;
+    const cudaError_t e = opt_in(k_dense_tiled_c128<TB>);
+    if (e != cudaSuccess) return e;
+    TiledMatC128<TB> g;
+    for (int i = 0; i < 1 << (2 * TB); ++i) {
+        const double re = m[2 * i], im = m[2 * i + 1];
+        const DF hr = host_split(re), hi = host_split(im);
+        g.terms[2 * i] = make_float4(hr.h, hr.h, hr.l, hr.l);
+        g.terms[2 * i + 1] = make_float4(-hi.h, hi.h, -hi.l, hi.l);
+        g.m[i] = make_double2(re, im);
     }
-    float4* terms = static_cast<float4*>(out);
-    double2* md = reinterpret_cast<double2*>(terms + 2 * d * d);
-    for (size_t r = 0; r < d; ++r)
-        for (size_t s = 0; s < d; ++s) {
-            const double re = m[2 * (r * d + s)], im = m[2 * (r * d + s) + 1];
-            const DF hr = host_split(re), hi = host_split(im);
-            terms[r * 2 * d + 2 * s] = make_float4(hr.h, hr.h, hr.l, hr.l);
-            terms[r * 2 * d + 2 * s + 1] = make_float4(-hi.h, hi.h, -hi.l, hi.l);
-            md[r * d + s] = make_double2(re, im);
-        }
+    k_dense_tiled_c128<TB><<<grid, 32 * warps, warps * kTiledWarpBytes, st>>>((double2*)amps, total, w, g);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_dense_tiled(void* amps, int prec, uint64_t total, int nbits, const IndexMap& map,
-                               const DenseOffsets& offs, int t, const void* dmat, int sm_count, cudaStream_t st)
+                               const DenseOffsets& offs, int t, const double* m, int sm_count, cudaStream_t st)
 {
     WarpTile w;
     const bool c128 = prec == kC128;
     warp_tile_layout(w, map.zpos, t, offs.off, nbits, c128 ? 9 : 10, c128 ? 3 : 4);
     if (!w.tiled) return cudaErrorInvalidValue;
     const uint64_t tiles = total >> w.tile_bits;
-    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sm_count, (tiles + kTiledWarps - 1) / kTiledWarps);
-    if (grid == 0) return cudaSuccess;
-    cudaError_t e = cudaSuccess;
-#define Q1G_TILED_C64(TBV)                                                                                    \
-    case TBV:                                                                                                 \
-        e = opt_in(k_dense_tiled_c64<TBV>);                                                                   \
-        if (e == cudaSuccess)                                                                                 \
-            k_dense_tiled_c64<TBV><<<grid, kTiledThreads, kTiledStageBytes, st>>>((float2*)amps, total, w,     \
-                                                                                  (const float2*)dmat);       \
-        break;
-#define Q1G_TILED_C128(TBV)                                                                                   \
-    case TBV:                                                                                                 \
-        e = opt_in(k_dense_tiled_c128<TBV>);                                                                  \
-        if (e == cudaSuccess)                                                                                 \
-            k_dense_tiled_c128<TBV><<<grid, kTiledThreads, kTiledStageBytes, st>>>(                           \
-                (double2*)amps, total, w, (const float4*)dmat,                                                \
-                (const double2*)((const float4*)dmat + 2 * (1 << (2 * TBV))));                                \
-        break;
-    if (c128) {
-        switch (t) {
-            Q1G_TILED_C128(1)
-            Q1G_TILED_C128(2)
-            Q1G_TILED_C128(3)
-            default:
-                return cudaErrorInvalidValue;
-        }
-    } else {
-        switch (t) {
-            Q1G_TILED_C64(1)
-            Q1G_TILED_C64(2)
-            Q1G_TILED_C64(3)
-            Q1G_TILED_C64(4)
-            default:
-                return cudaErrorInvalidValue;
-        }
+    if (tiles == 0) return cudaSuccess;
+    const unsigned warps = (unsigned)std::min<uint64_t>(kTiledWarps, (tiles + sm_count - 1) / sm_count);
+    const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sm_count, (tiles + warps - 1) / warps);
+    switch (t) {
+        case 1:
+            return c128 ? launch_tiled_c128<1>(amps, total, w, m, grid, warps, st)
+                        : launch_tiled_c64<1>(amps, total, w, m, grid, warps, st);
+        case 2:
+            return c128 ? launch_tiled_c128<2>(amps, total, w, m, grid, warps, st)
+                        : launch_tiled_c64<2>(amps, total, w, m, grid, warps, st);
+        case 3:
+            return c128 ? launch_tiled_c128<3>(amps, total, w, m, grid, warps, st)
+                        : launch_tiled_c64<3>(amps, total, w, m, grid, warps, st);
+        case 4:
+            return c128 ? cudaErrorInvalidValue : launch_tiled_c64<4>(amps, total, w, m, grid, warps, st);
+        default:
+            return cudaErrorInvalidValue;
     }
-#undef Q1G_TILED_C64
-#undef Q1G_TILED_C128
-    if (e != cudaSuccess) return e;
-    return cudaGetLastError();
 }
 
 }  // namespace q1g

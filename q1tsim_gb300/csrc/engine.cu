@@ -208,36 +208,16 @@ void q1g_state::apply_op(const GateOp& op, char* base, uint64_t total_amps)
             });
             return;
         case GateOp::Dense: {
-            const size_t d = size_t(1) << op.t;
-            std::vector<double> hm(2 * d * d);
-            for (size_t e = 0; e < d * d; ++e) {
-                hm[2 * e] = op.dense[e].real();
-                hm[2 * e + 1] = op.dense[e].imag();
-            }
+            const double* m = reinterpret_cast<const double*>(op.dense.data());
             if (dense_tiled_applies(prec, nbits, op.t, op.map, fp64_exact)) {
-                std::vector<unsigned char> img(dense_tiled_matrix_bytes(prec, op.t));
-                dense_tiled_matrix(prec, op.t, hm.data(), img.data());
-                matbuf.ensure(img.size());
-                h2d(matbuf.p, img.data(), img.size(), "upload matrix");
-                sync();
                 launch(prec == kC128 ? "dense_tiled_c128" : "dense_tiled_c64", b2 * op.touched(total_amps), [&] {
-                    return launch_dense_tiled(base, prec, total_amps, nbits, op.map, op.offs, op.t, matbuf.p,
-                                              sm_count(), stream);
+                    return launch_dense_tiled(base, prec, total_amps, nbits, op.map, op.offs, op.t, m, sm_count(),
+                                              stream);
                 });
                 return;
             }
-            if (prec == kC64) {
-                std::vector<float> hf(hm.begin(), hm.end());
-                matbuf.ensure(hf.size() * sizeof(float));
-                h2d(matbuf.p, hf.data(), hf.size() * sizeof(float), "upload matrix");
-                sync();
-            } else {
-                matbuf.ensure(hm.size() * sizeof(double));
-                h2d(matbuf.p, hm.data(), hm.size() * sizeof(double), "upload matrix");
-                sync();
-            }
             launch(prec == kC128 ? "dense_c128" : "dense_c64", b2 * op.touched(total_amps), [&] {
-                return launch_dense(base, prec, total_amps, op.map, op.offs, op.t, matbuf.p, stream);
+                return launch_dense(base, prec, total_amps, op.map, op.offs, op.t, m, stream);
             });
             return;
         }
@@ -1669,46 +1649,6 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
                 });
             });
             i += (size_t)(group - 1);   // the next blocks rode in this pass
-        } else if (op.kind == GateOp::Dense &&
-                   dense_tiled_applies(s->prec, s->nbits, op.t, op.map, s->fp64_exact)) {
-            const size_t d2 = op.dense.size();
-            std::vector<double> v(2 * d2);
-            for (size_t e = 0; e < d2; ++e) {
-                v[2 * e] = op.dense[e].real();
-                v[2 * e + 1] = op.dense[e].imag();
-            }
-            std::vector<unsigned char> img(dense_tiled_matrix_bytes(s->prec, op.t));
-            dense_tiled_matrix(s->prec, op.t, v.data(), img.data());
-            const void* dm = stage(img.data(), img.size());
-            emit([map = op.map, offs = op.offs, t = op.t, touched = op.touched(s->total()), dm](q1g_state* x) {
-                x->launch(x->prec == kC128 ? "dense_tiled_c128" : "dense_tiled_c64", 2.0 * x->bsz() * touched, [&] {
-                    return launch_dense_tiled(x->amps.p, x->prec, x->total(), x->nbits, map, offs, t, dm,
-                                              x->sm_count(), x->stream);
-                });
-            });
-        } else if (op.kind == GateOp::Dense) {
-            const size_t d2 = op.dense.size();
-            const void* dm;
-            if (s->prec == kC128) {
-                std::vector<double> v(2 * d2);
-                for (size_t e = 0; e < d2; ++e) {
-                    v[2 * e] = op.dense[e].real();
-                    v[2 * e + 1] = op.dense[e].imag();
-                }
-                dm = stage(v.data(), v.size() * sizeof(double));
-            } else {
-                std::vector<float> v(2 * d2);
-                for (size_t e = 0; e < d2; ++e) {
-                    v[2 * e] = (float)op.dense[e].real();
-                    v[2 * e + 1] = (float)op.dense[e].imag();
-                }
-                dm = stage(v.data(), v.size() * sizeof(float));
-            }
-            emit([map = op.map, offs = op.offs, t = op.t, touched = op.touched(s->total()), dm](q1g_state* x) {
-                x->launch(x->prec == kC128 ? "dense_c128" : "dense_c64", 2.0 * x->bsz() * touched, [&] {
-                    return launch_dense(x->amps.p, x->prec, x->total(), map, offs, t, dm, x->stream);
-                });
-            });
         } else {
             emit([op](q1g_state* x) { x->apply_op(op, x->amps.as<char>(), x->total()); });
         }

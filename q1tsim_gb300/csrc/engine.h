@@ -107,7 +107,6 @@ struct q1g_state {
     q1g::DevBuf amps, spare;
     q1g::DevBuf dscratch;   // doubles
     q1g::DevBuf uscratch;   // uint64
-    q1g::DevBuf matbuf;     // one dense matrix
     q1g::DevBuf colbuf;     // CollapseCol table
     q1g::DevBuf errbuf;     // error flag of bounded device waits
     q1g::HostBuf hstage;    // pinned staging for results

@@ -346,13 +346,21 @@ k_phase_c128x(double2* __restrict__ a, uint64_t units, IndexMap map, DF pr, DF p
 
 // One thread per group of 2^TB amplitudes at i | off[s]; the matrix sits in
 // shared memory (row-major, complex R).
+// The matrix as a kernel parameter (16 KB at most): no upload, and no wait for
+// one.
+template <typename T, int TB>
+struct DenseMat {
+    T m[1 << (2 * TB)];
+};
+
 template <typename T, int TB>
 __global__ void __launch_bounds__(128)
-k_dense(T* __restrict__ a, uint64_t units, IndexMap map, DenseOffsets offs, const T* __restrict__ gmat)
+k_dense(T* __restrict__ a, uint64_t units, IndexMap map, const __grid_constant__ DenseOffsets offs,
+        const __grid_constant__ DenseMat<T, TB> gmat)
 {
     constexpr int D = 1 << TB;
     __shared__ T mat[D * D];
-    for (int e = threadIdx.x; e < D * D; e += blockDim.x) mat[e] = gmat[e];
+    for (int e = threadIdx.x; e < D * D; e += blockDim.x) mat[e] = gmat.m[e];
     __syncthreads();
     const uint64_t u = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (u >= units) return;
@@ -481,21 +489,29 @@ cudaError_t launch_phase(void* amps, int prec, uint64_t total, const IndexMap& m
     return cudaGetLastError();
 }
 
+template <typename T, int TB>
+static cudaError_t dense_launch(void* amps, uint64_t units, const IndexMap& map, const DenseOffsets& offs,
+                                const double* m, cudaStream_t st)
+{
+    using R = decltype(T::x);
+    DenseMat<T, TB> g;
+    for (int e = 0; e < 1 << (2 * TB); ++e) {
+        g.m[e].x = (R)m[2 * e];
+        g.m[e].y = (R)m[2 * e + 1];
+    }
+    k_dense<T, TB><<<grid_for(units, 128), 128, 0, st>>>((T*)amps, units, map, offs, g);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_dense(void* amps, int prec, uint64_t total, const IndexMap& map,
-                         const DenseOffsets& offs, int tb, const void* dmat, cudaStream_t st)
+                         const DenseOffsets& offs, int tb, const double* m, cudaStream_t st)
 {
     const uint64_t units = total >> map.nz;
     if (units == 0) return cudaSuccess;
-    const unsigned grid = grid_for(units, 128);
 #define Q1G_DENSE_CASE(TBV)                                                                  \
     case TBV:                                                                                \
-        if (prec == kC128)                                                                   \
-            k_dense<double2, TBV><<<grid, 128, 0, st>>>((double2*)amps, units, map, offs,    \
-                                                        (const double2*)dmat);               \
-        else                                                                                 \
-            k_dense<float2, TBV><<<grid, 128, 0, st>>>((float2*)amps, units, map, offs,      \
-                                                       (const float2*)dmat);                 \
-        break;
+        return prec == kC128 ? dense_launch<double2, TBV>(amps, units, map, offs, m, st)     \
+                             : dense_launch<float2, TBV>(amps, units, map, offs, m, st);
     switch (tb) {
         Q1G_DENSE_CASE(1)
         Q1G_DENSE_CASE(2)
@@ -506,7 +522,6 @@ cudaError_t launch_dense(void* amps, int prec, uint64_t total, const IndexMap& m
             return cudaErrorInvalidValue;
     }
 #undef Q1G_DENSE_CASE
-    return cudaGetLastError();
 }
 
 }  // namespace q1g

@@ -31,9 +31,9 @@ cudaError_t launch_pair(void* amps, int prec, uint64_t total, const IndexMap& ma
                         cudaStream_t st, bool fp64_exact = false);
 cudaError_t launch_phase(void* amps, int prec, uint64_t total, const IndexMap& map,
                          double ph_re, double ph_im, cudaStream_t st, bool fp64_exact = false);
-// dmat: device matrix 2^tb x 2^tb, complex in the state's precision.
+// m: the 2^tb x 2^tb matrix, interleaved doubles (host).
 cudaError_t launch_dense(void* amps, int prec, uint64_t total, const IndexMap& map,
-                         const DenseOffsets& offs, int tb, const void* dmat, cudaStream_t st);
+                         const DenseOffsets& offs, int tb, const double* m, cudaStream_t st);
 
 // ---- phase_run.cu: a run of diagonal gates as one pass (complex64, <= 32 qubits)
 // out: the 2048 complex factors of phi = c + L0 + x_pivot L1, lin0/lin1 the
@@ -99,13 +99,9 @@ cudaError_t launch_swap_run(void* amps, int amp_bytes, uint64_t total, const voi
 // (higher 1-2 qubit blocks are coalesced, and faster, per unit); complex128
 // on >= 9 qubits with t <= 3 (double-float pairs).
 bool dense_tiled_applies(int prec, int nbits, int t, const IndexMap& map, bool fp64_exact);
-// The kernel's matrix image of a 2^t x 2^t complex matrix m (interleaved
-// doubles): complex64 entries, or complex128 double-float terms followed by
-// the FP64 matrix.
-size_t dense_tiled_matrix_bytes(int prec, int t);
-void dense_tiled_matrix(int prec, int t, const double* m, void* out);
+// m: the 2^t x 2^t matrix, interleaved doubles (host).
 cudaError_t launch_dense_tiled(void* amps, int prec, uint64_t total, int nbits, const IndexMap& map,
-                               const DenseOffsets& offs, int t, const void* dmat, int sm_count, cudaStream_t st);
+                               const DenseOffsets& offs, int t, const double* m, int sm_count, cudaStream_t st);
 
 // ---- fused_tc.cu: 5-qubit fused blocks on the tensor cores (complex64)
 // Geometry of one tensor-core pass over tiles of 2^12 amplitudes.  Tile
