@@ -172,13 +172,20 @@ void q1g_state::ensure_dense()
 {
     if (!sparse) return;
     amps.ensure(ncols * N * bsz());
-    uscratch.ensure(ncols * sizeof(uint64_t));
-    h2d(uscratch.p, basis.data(), ncols * sizeof(uint64_t), "upload basis");
+    const uint64_t* d_index = nullptr;
+    BasisList list;
+    if (ncols <= kMaxListCols && nbits >= 1) {
+        std::copy_n(basis.data(), ncols, list.index);
+    } else {
+        uscratch.ensure(ncols * sizeof(uint64_t));
+        h2d(uscratch.p, basis.data(), ncols * sizeof(uint64_t), "upload basis");
+        d_index = uscratch.as<uint64_t>();
+    }
     launch("fill_basis", double(ncols * N * bsz()), [&] {
-        return launch_fill_basis(amps.p, prec, ncols * N, uscratch.as<uint64_t>(), ncols, N, stream);
+        return launch_fill_basis(amps.p, prec, nbits, d_index ? nullptr : &list, d_index, ncols, stream);
     });
-    // The basis list must stay alive until the copy ran: wait here.
-    sync();
+    // an uploaded list must stay alive until the copy ran: wait here
+    if (d_index) sync();
     sparse = false;
     basis.clear();
 }
@@ -313,6 +320,10 @@ struct CondRange {
     bool apply;
 };
 
+// A split's old columns are kept for the next one up to this size: allocating
+// 1 GB and freeing it again takes longer (1 to 2 ms) than the split itself.
+constexpr size_t kKeptSpareBytes = size_t(4) << 30;
+
 static std::vector<CondRange> conditional_ranges(const std::vector<uint64_t>& counts,
                                                  const uint8_t* control)
 {
@@ -357,14 +368,9 @@ void q1g_state::apply_conditional(const uint8_t* control, size_t ncontrol, const
         std::vector<CollapseCol> cols(nr);
         for (uint64_t j = 0; j < nr; ++j) cols[j] = {ranges[j].col, -1, 1.0};
         spare.ensure(nr * N * bsz());
-        colbuf.ensure(nr * sizeof(CollapseCol));
-        h2d(colbuf.p, cols.data(), nr * sizeof(CollapseCol), "upload columns");
-        launch("column_copy", 2.0 * nr * N * bsz(), [&] {
-            return launch_collapse_copy(spare.p, amps.p, prec, N, 0, colbuf.as<CollapseCol>(), nr, stream);
-        });
-        sync();
+        copy_columns("column_copy", 2.0 * nr, spare.p, 0, cols);
         amps.swap(spare);
-        if (spare.bytes > (size_t(1) << 30)) spare.release();
+        if (spare.bytes > kKeptSpareBytes) spare.release();
         ncols = nr;
     }
     if (!same_layout) {
@@ -376,6 +382,25 @@ void q1g_state::apply_conditional(const uint8_t* control, size_t ncontrol, const
     for (size_t j = 0; j < ranges.size(); ++j) counts[j] = ranges[j].len;
     for (size_t j = 0; j < ranges.size(); ++j)
         if (ranges[j].apply) apply_op(op, col_ptr(j), N);
+}
+
+// New columns `cols` of amps into dst (launch_collapse_copy); moved: columns'
+// worth of bytes.
+void q1g_state::copy_columns(const char* name, double moved, void* dst, int pos, const std::vector<CollapseCol>& cols)
+{
+    const CollapseCol* d_cols = nullptr;
+    CollapseList list;
+    if (cols.size() <= kMaxListCols) {
+        std::copy(cols.begin(), cols.end(), list.col);
+    } else {
+        colbuf.ensure(cols.size() * sizeof(CollapseCol));
+        h2d(colbuf.p, cols.data(), cols.size() * sizeof(CollapseCol), "upload columns");
+        d_cols = colbuf.as<CollapseCol>();
+    }
+    launch(name, moved * N * bsz(), [&] {
+        return launch_collapse_copy(dst, amps.p, prec, N, pos, list, d_cols, cols.size(), stream);
+    });
+    if (d_cols) sync();      // the uploaded table must stay alive until the copy ran
 }
 
 std::vector<double> q1g_state::zero_weights(size_t qbit)
@@ -468,22 +493,14 @@ void q1g_state::measure(size_t qbit, size_t cbit, uint64_t* res, size_t res_len,
     norms.assign(new_nr, 1.0);
     const int pos = nbits - 1 - (int)qbit;
     const bool split = new_nr != ncols;
-    colbuf.ensure(new_nr * sizeof(CollapseCol));
-    h2d(colbuf.p, cols.data(), new_nr * sizeof(CollapseCol), "upload columns");
+    // each column's kept half is read
     if (!split) {
-        launch("collapse", 2.0 * ncols * N * bsz(), [&] {
-            return launch_collapse_copy(amps.p, amps.p, prec, N, pos, colbuf.as<CollapseCol>(), new_nr, stream);
-        });
+        copy_columns("collapse", 1.5 * ncols, amps.p, pos, cols);
     } else {
         spare.ensure(new_nr * N * bsz());
-        launch("collapse", double(new_nr + ncols) * N * bsz(), [&] {
-            return launch_collapse_copy(spare.p, amps.p, prec, N, pos, colbuf.as<CollapseCol>(), new_nr, stream);
-        });
-    }
-    sync();
-    if (split) {
+        copy_columns("collapse", 1.5 * new_nr, spare.p, pos, cols);
         amps.swap(spare);
-        if (spare.bytes > (size_t(1) << 30)) spare.release();
+        if (spare.bytes > kKeptSpareBytes) spare.release();
     }
     ncols = new_nr;
     counts = nc;

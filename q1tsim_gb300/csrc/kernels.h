@@ -315,8 +315,16 @@ cudaError_t launch_fused_tc_c128(double2* amps, uint64_t total, const ZPass& p, 
                                  int sm_count, cudaStream_t st, uint64_t wait_ns);
 
 // ---- state_kernels.cu: construction, conversion, collapse
-cudaError_t launch_fill_basis(void* amps, int prec, uint64_t n_amps, const uint64_t* d_col_index,
-                              uint64_t ncols, uint64_t col_len, cudaStream_t st);
+// Tables of up to this many columns go as kernel parameters: no upload, and no
+// wait for one.
+constexpr uint64_t kMaxListCols = 64;
+struct BasisList {
+    uint64_t index[kMaxListCols];
+};
+// Column c of 2^nbits amplitudes is the basis state list->index[c], or, where
+// there are more, d_col_index[c].
+cudaError_t launch_fill_basis(void* amps, int prec, int nbits, const BasisList* list, const uint64_t* d_col_index,
+                              uint64_t ncols, cudaStream_t st);
 // Bit positions of a subspace: bit k of a compact index is position pos[k].
 struct SubspacePositions {
     int n;
@@ -344,8 +352,12 @@ struct CollapseCol {
     int keep;       // 0 or 1: the measured value this column keeps; -1: plain copy
     double scale;
 };
+struct CollapseList {
+    CollapseCol col[kMaxListCols];
+};
+// d_cols: the columns where they are more than the list holds, else null.
 cudaError_t launch_collapse_copy(void* dst, const void* src, int prec, uint64_t col_len, int pos,
-                                 const CollapseCol* d_cols, uint64_t ncols, cudaStream_t st);
+                                 const CollapseList& list, const CollapseCol* d_cols, uint64_t ncols, cudaStream_t st);
 
 // ---- measure_kernels.cu
 // Per-chunk FP64 sums of |a|^2.  The kernel walks `units` virtual indices j,
