@@ -16,7 +16,7 @@ struct q1g_batch {
     uint64_t arena_amps = 0;
     uint64_t scratch_per_cta = 0;
     int sms = 0;
-    q1g::DevBuf arena, results, dcircuits, dops, dmats, dtables, scratch, queue, traffic;
+    q1g::DevBuf arena, results, dcircuits, dops, dmats, dtables, lfact, scratch, queue, traffic;
     q1g::HostBuf hresults, htraffic;
     cudaStream_t stream = nullptr;
     cudaGraph_t graph = nullptr;
@@ -32,6 +32,21 @@ void batch_add_circuit(q1g_batch* b, size_t nr_bits, size_t nr_shots, uint64_t s
                        const size_t* nbits_per_op, const size_t* bits_flat, const double* mats_flat,
                        const size_t* args);
 void batch_run(q1g_batch* b, uint64_t* results, size_t len);
+// How a batch's largest circuits run: the first `circuits` of the queue on
+// `count` teams of `size` CTAs.
+struct TeamPlan {
+    int circuits = 0, size = 1, count = 0;
+};
+// Teams of `size` CTAs, of which `count` run at once; us: each circuit's time on
+// one, in queue order.
+struct TeamChoice {
+    int size = 1, count = 0;
+    std::vector<double> us;
+};
+// alone, able: per circuit in queue order, its time on one CTA and whether a
+// team may run it.
+TeamPlan plan_teams(const std::vector<double>& alone, const std::vector<char>& able, int sms,
+                    const std::vector<TeamChoice>& choices);
 // warp-tile layout of a dense op on nbits qubits, gate positions pos[0..tb)
 void batch_tile_layout(BatchOp& op, const int* pos, int tb, int nbits);
 }  // namespace q1g

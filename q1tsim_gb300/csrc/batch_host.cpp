@@ -3,7 +3,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <numeric>
+#include <queue>
 #include <string>
 
 #include "batch.h"
@@ -165,45 +167,113 @@ static void upload(DevBuf& d, const void* h, size_t bytes, cudaStream_t st)
     if (bytes) check_cuda(cudaMemcpyAsync(d.p, h, bytes, cudaMemcpyHostToDevice, st), "batch upload");
 }
 
+// Microseconds of a circuit on a team of `size` CTAs, from one-circuit batches
+// of 8 to 18 qubits (within 15 %): a round of tiles (one per warp) 3 us, and 5 for
+// a 4-qubit block's arithmetic; 2.5 us per pass; the draws of a measurement and
+// the shots.
+static double circuit_us(const q1g_batch* b, const BatchCircuit& C, int size)
+{
+    const double n = std::ldexp(1.0, C.nbits), rounds = std::ceil(n / 1024.0 / (16.0 * size));
+    double us = 10.0, cols = 1.0;
+    for (uint32_t oi = C.op_begin; oi < C.op_end; ++oi) {
+        const BatchOp& op = b->ops[oi];
+        if (op.kind == kBatchDense) {
+            us += 2.5 + (op.cond >= 0 ? 1.0 : cols) * rounds * (C.nbits < 10 ? 0.5 : 3.0 + 5.0 / 16.0 * (1 << op.t));
+        } else if (op.kind == kBatchMeasure) {
+            us += cols * (20.0 + 3e-4 * n / size);
+            cols = std::min(2.0 * cols, (double)C.maxcols);
+        } else {
+            us += cols * (30.0 + 1e-4 * n / size) + 0.05 * C.nshots / size;
+        }
+    }
+    return us;
+}
+
+TeamPlan plan_teams(const std::vector<double>& alone, const std::vector<char>& able, int sms,
+                    const std::vector<TeamChoice>& choices)
+{
+    const size_t nc = alone.size();
+    // Finish time with the first k circuits on the teams of c, the others alone
+    // on the CTAs of the teams as these come free.
+    auto finish = [&](size_t k, const TeamChoice& c) {
+        std::priority_queue<double, std::vector<double>, std::greater<double>> teams, ctas;
+        for (int t = 0; t < c.count; ++t) teams.push(0.0);
+        for (size_t i = 0; i < k; ++i) {
+            const double t = teams.top();
+            teams.pop();
+            teams.push(t + c.us[i]);
+        }
+        double last = 0.0;
+        for (; !teams.empty(); teams.pop()) {
+            last = std::max(last, teams.top());
+            for (int r = 0; r < c.size; ++r) ctas.push(teams.top());
+        }
+        for (size_t i = k; i < nc; ++i) {
+            const double t = ctas.top() + alone[i];
+            ctas.pop();
+            ctas.push(t);
+            last = std::max(last, t);
+        }
+        return last;
+    };
+    TeamPlan best;
+    if (nc == 0 || nc > 16 * (size_t)sms) return best;      // many circuits fill the SMs alone
+    // (the estimate is good to some 10 %)
+    double best_us = 0.9 * finish(0, {1, sms, alone});
+    for (const TeamChoice& c : choices) {
+        if (c.count < 1) continue;
+        for (size_t k = 1; k <= nc; k += 1 + k / 8) {
+            if (!std::all_of(able.begin(), able.begin() + k, [](char v) { return v != 0; })) break;
+            const double us = finish(k, c);
+            if (us < best_us) {
+                best_us = us;
+                best = {(int)k, c.size, c.count};
+            }
+        }
+    }
+    return best;
+}
+
 static void batch_build(q1g_batch* b)
 {
     if (!b->stream) check_cuda(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     int dev = 0;
     check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
     check_cuda(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev), "sm count");
-    // queue order: most work first (longest-processing-time order), so the
-    // long circuits start early and the short ones fill in at the end.  The
-    // work estimate counts amplitude reads and writes: every gate pass over
-    // every column (their number at most doubling at each measurement), the
-    // measurements, and the sampling's chunk sums and searched chunks.
+    // queue order: the longest first (longest-processing-time order), so the
+    // long circuits start early and the short ones fill in at the end
     const size_t nc = b->circuits.size();
-    std::vector<double> work(nc, 0.0);
-    for (size_t i = 0; i < nc; ++i) {
-        const BatchCircuit& C = b->circuits[i];
-        const double N = std::ldexp(1.0, C.nbits);
-        double w = N, cols = 1.0;
-        for (uint32_t oi = C.op_begin; oi < C.op_end; ++oi) {
-            const BatchOp& op = b->ops[oi];
-            if (op.kind == kBatchDense) {
-                w += 2.0 * N * (op.cond >= 0 ? 1.0 : cols);
-            } else if (op.kind == kBatchMeasure) {
-                w += 4.0 * N * cols;
-                cols = std::min(2.0 * cols, (double)C.maxcols);
-            } else {
-                w += N * cols + (double)C.nshots * std::min(N, 256.0);
-            }
-        }
-        work[i] = w;
-    }
+    std::vector<double> time(nc, 0.0);
+    for (size_t i = 0; i < nc; ++i) time[i] = circuit_us(b, b->circuits[i], 1);
     std::vector<size_t> order(nc);
     std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return work[x] > work[y]; });
+    std::stable_sort(order.begin(), order.end(), [&](size_t x, size_t y) { return time[x] > time[y]; });
     uint64_t res = 0;
     for (auto& C : b->circuits) {
         C.res_off = res;
         res += C.nshots;
     }
     b->total_runs = res;
+    check_cuda(setup_batch_kernel(), "batch kernel attributes");
+    std::vector<TeamChoice> choices;
+    for (int size = 2; size <= 8; size *= 2) {
+        TeamChoice c;
+        c.size = size;
+        if (batch_clusters(size, b->sms, &c.count) != cudaSuccess) {
+            (void)cudaGetLastError();
+            c.count = 0;
+        }
+        c.count = std::min(c.count, b->sms / size);
+        for (size_t i : order) c.us.push_back(circuit_us(b, b->circuits[i], size));
+        choices.push_back(std::move(c));
+    }
+    std::vector<double> alone;
+    std::vector<char> able;
+    for (size_t i : order) {
+        alone.push_back(time[i]);
+        able.push_back(b->circuits[i].nbits >= kBatchTeamBits);
+    }
+    const TeamPlan teams = plan_teams(alone, able, b->sms, choices);
     std::vector<BatchCircuit> queue;
     uint64_t off = 0, per_cta = 16;
     for (size_t i : order) {
@@ -223,9 +293,17 @@ static void batch_build(q1g_batch* b)
     upload(b->dops, b->ops.data(), b->ops.size() * sizeof(BatchOp), b->stream);
     upload(b->dmats, b->mats.data(), b->mats.size() * sizeof(float2), b->stream);
     upload(b->dtables, b->cbit_tables.data(), b->cbit_tables.size() * sizeof(uint64_t), b->stream);
-    const int grid = std::min<int>(b->sms, (int)std::max<size_t>(nc, 1));
+    // log k! for the draws of measurements with at most 2^20 runs
+    uint64_t nlfact = 0;
+    for (const BatchCircuit& C : b->circuits)
+        for (uint32_t oi = C.op_begin; oi < C.op_end; ++oi)
+            if (b->ops[oi].kind == kBatchMeasure)
+                nlfact = std::max(nlfact, std::min<uint64_t>(C.nshots + 1, (uint64_t(1) << 20) + 1));
+    b->lfact.ensure(std::max<uint64_t>(nlfact, 2) * sizeof(double));
+    check_cuda(launch_log_factorials(b->lfact.as<double>(), nlfact, b->stream), "log factorials");
+    const int grid = teams.circuits ? teams.size * teams.count : std::min<int>(b->sms, (int)std::max<size_t>(nc, 1));
     b->scratch.ensure((size_t)grid * b->scratch_per_cta * sizeof(double));
-    b->queue.ensure(sizeof(unsigned));
+    b->queue.ensure(2 * sizeof(unsigned));
     b->traffic.ensure(sizeof(unsigned long long));
     b->htraffic.ensure(sizeof(unsigned long long));
     check_cuda(cudaStreamSynchronize(b->stream), "batch upload");
@@ -235,20 +313,22 @@ static void batch_build(q1g_batch* b)
     a.results = b->results.as<uint64_t>();
     a.circuits = b->dcircuits.as<BatchCircuit>();
     a.ncircuits = (int)nc;
+    a.nteam = teams.circuits;
     a.ops = b->dops.as<BatchOp>();
     a.mats = b->dmats.as<float2>();
     a.cbit_tables = b->dtables.as<uint64_t>();
+    a.lfact = b->lfact.as<double>();
+    a.nlfact = nlfact;
     a.scratch = b->scratch.as<double>();
     a.scratch_per_cta = b->scratch_per_cta;
     a.queue = b->queue.as<unsigned>();
     a.traffic = b->traffic.as<unsigned long long>();
-    check_cuda(setup_batch_kernel(), "batch kernel attributes");
     // one execution = reset queue and results, the persistent launch, results out
     check_cuda(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-    cudaError_t e = cudaMemsetAsync(b->queue.p, 0, sizeof(unsigned), b->stream);
+    cudaError_t e = cudaMemsetAsync(b->queue.p, 0, 2 * sizeof(unsigned), b->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->traffic.p, 0, sizeof(unsigned long long), b->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->results.p, 0, std::max<uint64_t>(res, 1) * sizeof(uint64_t), b->stream);
-    if (e == cudaSuccess) e = launch_batch(a, b->sms, b->stream);
+    if (e == cudaSuccess) e = launch_batch(a, nc ? (unsigned)grid : 0u, teams.size, b->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(b->hresults.p, b->results.p, res * sizeof(uint64_t), cudaMemcpyDeviceToHost, b->stream);
     if (e == cudaSuccess)

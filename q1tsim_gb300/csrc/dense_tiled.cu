@@ -62,7 +62,7 @@ k_dense_tiled_c64(float2* a, uint64_t total, const __grid_constant__ WarpTile ti
     __syncthreads();
     const int warp = threadIdx.x >> 5;
     tiled_dense_c64<TB, false>(a, total, w, mat, stage_c64 + warp * 1024,
-                               ((uint64_t)blockIdx.x * blockDim.x >> 5) + warp, (uint64_t)gridDim.x * blockDim.x >> 5);
+                               (blockIdx.x * blockDim.x >> 5) + warp, [] { return gridDim.x * blockDim.x >> 5; });
 }
 
 // Shared-memory load of one 16-byte term, kept at its use.

@@ -452,16 +452,24 @@ struct BatchArgs {
     uint64_t* results;
     const BatchCircuit* circuits;   // in queue order
     int ncircuits;
+    int nteam;                      // the first of them, run by whole clusters
     const BatchOp* ops;
     const float2* mats;
     const uint64_t* cbit_tables;
+    const double* lfact;            // log k! for k < nlfact
+    uint64_t nlfact;
     double* scratch;
     uint64_t scratch_per_cta;
-    unsigned* queue;
+    unsigned* queue;                // taken so far: of the teams' circuits, of the others
     unsigned long long* traffic;    // algorithmic bytes the launch moves in device memory (summed)
 };
 cudaError_t setup_batch_kernel();   // opt the batch kernel in to its shared-memory stage
-cudaError_t launch_batch(const BatchArgs& a, int sm_count, cudaStream_t st);
+// grid: a multiple of `cluster`, the CTAs of a team (1: no teams).
+cudaError_t launch_batch(const BatchArgs& a, unsigned grid, int cluster, cudaStream_t st);
+cudaError_t launch_log_factorials(double* out, uint64_t n, cudaStream_t st);
+// Clusters of that size that run at the same time.
+cudaError_t batch_clusters(int cluster, int sm_count, int* count);
+constexpr int kBatchTeamBits = 12;      // qubits of a team's circuit at least (whole tiles for every CTA)
 
 // Per-block partials (6 doubles per block) comparing two states; wa and wb
 // weight the probabilities in the total-variation term.

@@ -251,9 +251,9 @@ __global__ void __launch_bounds__(kScanThreads) k_pair_scan_tiles(ScanPair s)
 // in the reduction and in the search so the two agree: p_i = |a_i|^2 in the
 // state's precision, groups of 8 consecutive p_i summed sequentially in that
 // precision, chunks of 32 groups (256 amplitudes) summed in FP64, and the
-// FP64 exclusive prefix over chunks.  A shot finds its chunk by a 32-ary warp
-// search on that prefix, its group by an FP64 warp scan of the chunk's 32
-// group sums, and its amplitude by a sequential scan of the group.
+// FP64 exclusive prefix over chunks.  A shot finds its chunk by a search on that
+// prefix, its group by a warp scan of the chunk's 32 group sums, and its
+// amplitude by a sequential scan of the group.
 
 // One warp per chunk of `chunk` (<= 256) amplitudes.  groups (or null): the 32
 // group sums of each chunk, for the sampler.  The first sp_blocks blocks draw
@@ -282,77 +282,26 @@ k_chunk_sums_dense(const T* __restrict__ a, uint64_t nchunks, uint64_t chunk, do
     }
 }
 
-// A warp takes 32 consecutive shots.  Each lane finds its shot's chunk (the
-// largest c with excl[c] <= target) by a binary search: the shots are sorted, so
-// the lanes' probes share their cache lines.  Then the warp finds the shots'
-// groups one after the other by a scan of the chunk's 32 group sums, and each
-// lane its shot's amplitude in its group and its word.  With the group sums from
+// A warp takes `per` consecutive shots, at most 32 (sample_warp).  With the group sums from
 // memory (kGroups) a shot reads 128 + 64 bytes of complex64 instead of the
 // chunk's 2 KB.  10^6 shots of 29 qubits: 627 us with one shot per warp at a
 // time (its amplitude and word found by one lane) and a merge for the chunks;
 // 113 us now.
 template <typename T, bool kGroups>
 __global__ void __launch_bounds__(256)
-k_sample(SampleArgs s)
+k_sample(SampleArgs s, uint32_t per)
 {
     using R = typename ProbT<T>::R;
-    constexpr int kAhead = kGroups ? 8 : 2;      // chunks read at once
-    const T* a = static_cast<const T*>(s.amps);
-    const R* groups = static_cast<const R*>(s.groups);
     const int lane = threadIdx.x & 31;
     const uint64_t warps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
     const double total = *s.total;
-    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; b * 32 < s.nruns; b += warps) {
-        const uint64_t r = b * 32 + lane;
-        const int count = (int)min(s.nruns - b * 32, uint64_t(32));
+    for (uint64_t b = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; b * per < s.nruns; b += warps) {
+        const uint64_t r = b * per + lane;
+        const int count = (int)min(s.nruns - b * per, uint64_t(per));
         const double target = lane < count ? shot_target(s.u[r], total) : 0.0;
-        uint64_t lo = 0, hi = s.nchunks;
-        while (hi - lo > 1) {
-            const uint64_t mid = (lo + hi) >> 1;
-            if (s.excl[mid] <= target) lo = mid;
-            else hi = mid;
-        }
-        // the target's offset into the chunk, in the state's precision (it is
-        // at most the chunk's mass)
-        const R offset = (R)(target - s.excl[lo]);
-        int group = 0;
-        R local = R(0);
-        for (int k0 = 0; k0 < count; k0 += kAhead) {
-            R gs[kAhead];
-#pragma unroll
-            for (int k = 0; k < kAhead; ++k) {
-                const uint64_t c = __shfl_sync(0xffffffffu, lo, k0 + k);
-                if (kGroups) {
-                    gs[k] = groups[c * 32 + lane];
-                } else {
-                    R p[8];
-                    group_probs(a, c * s.chunk, s.chunk, lane, p);
-                    gs[k] = group_sum(p);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < kAhead; ++k) {
-                // the group sums scanned in the state's precision (the chunk
-                // sums add them in the same order, chunk_total)
-                const R t = __shfl_sync(0xffffffffu, offset, k0 + k);
-                const R incl = warp_incl_scan(gs[k], lane);
-                const unsigned hit = __ballot_sync(0xffffffffu, gs[k] > R(0) && incl > t);
-                const unsigned nz = __ballot_sync(0xffffffffu, gs[k] > R(0));
-                const int owner = hit ? __ffs(hit) - 1 : nz ? 31 - __clz(nz) : 0;
-                const R before = __shfl_sync(0xffffffffu, incl - gs[k], owner);
-                if (lane == k0 + k) {
-                    group = owner;
-                    // past the end: the group's last nonzero amplitude
-                    local = hit ? t - before : R(INFINITY);
-                }
-            }
-        }
+        const uint64_t idx = sample_warp<kGroups>(static_cast<const T*>(s.amps), s.chunk, s.excl, s.nchunks,
+                                                  static_cast<const R*>(s.groups), target, count, lane);
         if (lane >= count) continue;
-        const uint64_t i0 = lo * s.chunk + (uint64_t)group * 8;
-        R p[8];
-        group_probs(a, lo * s.chunk, s.chunk, group, p);
-        const int e = pick_in_group(p, local);
-        const uint64_t idx = i0 + (uint64_t)e;
         const uint64_t word = outcome_word(idx, s.nbits, s.d_cbit_of_pos);
         if (s.outcome) {
             if (s.narrow) static_cast<uint32_t*>(s.outcome)[r] = (uint32_t)idx;
@@ -575,17 +524,20 @@ cudaError_t launch_scale_columns(void* amps, int prec, uint64_t col_len, uint64_
 cudaError_t launch_sample(const SampleArgs& a, cudaStream_t st)
 {
     if (a.nruns == 0) return cudaSuccess;
-    // 8 warps of 32 shots per block, at most 8 blocks per SM (64 warps); few
-    // shots go one warp to a block, over all SMs
-    const uint64_t warps = (a.nruns + 31) / 32;
-    const unsigned threads = warps <= 152 ? 32 : 256;
+    // 8 warps of 32 shots per block, at most 8 blocks per SM (64 warps).  Few
+    // shots go 8 to a warp (one round of reads), up to 8 warps per SM and one
+    // to a block: 1024 shots of 10 qubits 24.5 us between events with 32, 12.3
+    // us with 8.
+    const uint32_t per = a.nruns <= 152 * 8 * 8 ? 8 : 32;
+    const uint64_t warps = (a.nruns + per - 1) / per;
+    const unsigned threads = per == 8 ? 32 : 256;
     const unsigned grid = (unsigned)std::min<uint64_t>((warps * 32 + threads - 1) / threads, 152ull * 8);
     if (a.prec == kC128) {
-        if (a.groups) k_sample<double2, true><<<grid, threads, 0, st>>>(a);
-        else k_sample<double2, false><<<grid, threads, 0, st>>>(a);
+        if (a.groups) k_sample<double2, true><<<grid, threads, 0, st>>>(a, per);
+        else k_sample<double2, false><<<grid, threads, 0, st>>>(a, per);
     } else {
-        if (a.groups) k_sample<float2, true><<<grid, threads, 0, st>>>(a);
-        else k_sample<float2, false><<<grid, threads, 0, st>>>(a);
+        if (a.groups) k_sample<float2, true><<<grid, threads, 0, st>>>(a, per);
+        else k_sample<float2, false><<<grid, threads, 0, st>>>(a, per);
     }
     return cudaGetLastError();
 }

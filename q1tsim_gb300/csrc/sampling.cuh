@@ -7,9 +7,9 @@
 // state's precision, groups of 8 consecutive p_i summed sequentially in that
 // precision, chunks of 32 groups (256 amplitudes) summed in the state's
 // precision too (FP64 for complex128), and an FP64 exclusive prefix over
-// chunks.  A shot finds its chunk by a 32-ary warp
-// search on that prefix, its group by an FP64 warp scan of the chunk's 32
-// group sums, and its amplitude by a sequential scan of the group.
+// chunks.  A shot finds its chunk by a search on that prefix, its group by a
+// warp scan of the chunk's 32 group sums, and its amplitude by a sequential
+// scan of the group.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -134,9 +134,6 @@ __device__ __forceinline__ double chunk_sum(const T* a, uint64_t i0, uint64_t ch
     return chunk_total(group_sum(p), lane);
 }
 
-// One shot, executed by a whole warp: the basis index whose inclusive
-// probability prefix first exceeds u * total.  Returns true on the lane that
-// holds the result in *idx.
 // The shot's target u * total, kept strictly inside the mass if rounding
 // pushed it onto the total (u < 1): the shot then lands on the last nonzero
 // amplitude.
@@ -146,64 +143,64 @@ __device__ __forceinline__ double shot_target(double u, double total)
     return target < total ? target : nextafter(total, 0.0);
 }
 
-// One shot whose chunk lo is known (the largest chunk c with excl[c] <=
-// target), executed by a whole warp.  Returns true on the lane that holds
-// the result in *idx.
-template <typename T>
-__device__ bool sample_in_chunk(const T* a, uint64_t chunk, const double* excl, uint64_t lo, double target,
-                                int lane, uint64_t* idx);
-
-template <typename T>
-__device__ bool sample_one(const T* a, uint64_t chunk, const double* excl, uint64_t nchunks, double total,
-                           double u, int lane, uint64_t* idx)
-{
-    const double target = shot_target(u, total);
-    // Largest chunk c with excl[c] <= target (excl is non-decreasing and
-    // excl[0] = 0).  The warp searches 32-ary: lane j probes lo + j * step,
-    // and the last lane whose prefix is <= target narrows [lo, hi) to one
-    // step: 5 dependent rounds over 2^22 chunks instead of 22 for a binary
-    // search.
-    uint64_t lo = 0, hi = nchunks;
-    while (hi - lo > 1) {
-        const uint64_t step = (hi - lo + 31) >> 5;
-        const uint64_t pj = lo + (uint64_t)lane * step;
-        const unsigned ok = __ballot_sync(0xffffffffu, pj < hi && excl[pj] <= target);
-        lo += (uint64_t)(31 - __clz(ok)) * step;    // lane 0 always qualifies
-        hi = min(hi, lo + step);
-    }
-    return sample_in_chunk(a, chunk, excl, lo, target, lane, idx);
-}
-
-template <typename T>
-__device__ bool sample_in_chunk(const T* a, uint64_t chunk, const double* excl, uint64_t lo, double target,
-                                int lane, uint64_t* idx)
+// 32 shots of a column by a warp: lane r's has the target `target`; lanes from
+// `count` on have none.  Each lane finds its shot's chunk (the largest c with
+// excl[c] <= target; excl is non-decreasing, excl[0] = 0) by a binary search:
+// shots are sorted, so the lanes' probes share their cache lines.  Then the warp
+// finds the shots' groups one after the other by a scan of the chunk's 32 group
+// sums (from `groups`, or from the amplitudes), and each lane its shot's
+// amplitude in its group.  Returns the lane's basis index: the first whose
+// inclusive probability prefix exceeds the target.
+template <bool kGroups, typename T>
+__device__ __forceinline__ uint64_t sample_warp(const T* a, uint64_t chunk, const double* excl, uint64_t nchunks,
+                                                const typename ProbT<T>::R* groups, double target, int count, int lane)
 {
     using R = typename ProbT<T>::R;
-    const uint64_t i0 = lo * chunk;
-    const double tl = target - excl[lo];
-    R p[8];
-    group_probs(a, i0, chunk, lane, p);
-    // the chunk's group sums scanned in the state's precision (the chunk
-    // sums add them in the same order, chunk_total)
-    // and the target's offset into the chunk compared in that precision too
-    // (it is at most the chunk's mass)
-    const R gs = group_sum(p);
-    const R incl = warp_incl_scan(gs, lane);
-    const R tlr = (R)tl;
-    const unsigned hit = __ballot_sync(0xffffffffu, gs > R(0) && incl > tlr);
-    const unsigned nz = __ballot_sync(0xffffffffu, gs > R(0));
-    int owner;
-    R local;
-    if (hit) {
-        owner = __ffs(hit) - 1;
-        local = tlr - (incl - gs);
-    } else {
-        owner = nz ? 31 - __clz(nz) : 0;
-        local = R(INFINITY);   // past the end: take the group's last nonzero amplitude
+    constexpr int kAhead = kGroups ? 8 : 2;      // chunks read at once
+    uint64_t lo = 0, hi = nchunks;
+    while (hi - lo > 1) {
+        const uint64_t mid = (lo + hi) >> 1;
+        if (excl[mid] <= target) lo = mid;
+        else hi = mid;
     }
-    if (lane != owner) return false;
-    *idx = i0 + (uint64_t)lane * 8 + (uint64_t)pick_in_group(p, local);
-    return true;
+    // the target's offset into the chunk, in the state's precision (it is at
+    // most the chunk's mass)
+    const R offset = (R)(target - excl[lo]);
+    int group = 0;
+    R local = R(0);
+    for (int k0 = 0; k0 < count; k0 += kAhead) {
+        R gs[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            const uint64_t c = __shfl_sync(0xffffffffu, lo, k0 + k);
+            if (kGroups) {
+                gs[k] = groups[c * 32 + lane];
+            } else {
+                R p[8];
+                group_probs(a, c * chunk, chunk, lane, p);
+                gs[k] = group_sum(p);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            // the group sums scanned in the state's precision (the chunk
+            // sums add them in the same order, chunk_total)
+            const R t = __shfl_sync(0xffffffffu, offset, k0 + k);
+            const R incl = warp_incl_scan(gs[k], lane);
+            const unsigned hit = __ballot_sync(0xffffffffu, gs[k] > R(0) && incl > t);
+            const unsigned nz = __ballot_sync(0xffffffffu, gs[k] > R(0));
+            const int owner = hit ? __ffs(hit) - 1 : nz ? 31 - __clz(nz) : 0;
+            const R before = __shfl_sync(0xffffffffu, incl - gs[k], owner);
+            if (lane == k0 + k) {
+                group = owner;
+                // past the end: the group's last nonzero amplitude
+                local = hit ? t - before : R(INFINITY);
+            }
+        }
+    }
+    R p[8];
+    group_probs(a, lo * chunk, chunk, group, p);
+    return lo * chunk + (uint64_t)group * 8 + (uint64_t)pick_in_group(p, local);
 }
 
 // Classical word of outcome idx: bit position p of idx goes to the mask

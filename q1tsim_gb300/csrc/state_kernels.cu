@@ -195,9 +195,9 @@ template <> struct Quad<float2> {
 
 // Columns of a collapse, blockIdx.y-th and every gridDim.y-th: the amplitudes
 // that go are not read (half of each column).  dst may be src where every
-// column stays in its place.Four measurements of a
-// 23-qubit complex128 state (to up to 16 columns): 1.21 ms with every amplitude
-// read and a division for each, 0.92 ms so.
+// column stays in its place.  Four measurements of a 23-qubit complex128 state
+// (to up to 16 columns): 1.21 ms with every amplitude read and a division for
+// each, 0.92 ms so.
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_collapse_copy(T* dst, const T* src, uint64_t col_len, int pos, const __grid_constant__ CollapseList list,

@@ -66,7 +66,7 @@ __device__ __forceinline__ uint32_t lane_phys(const WarpTile& w, int lane)
     return p;
 }
 
-// Complex64 tile pass over tiles t0, t0 + tstride, ... of a state of
+// Complex64 tile pass over tiles t0, t0 + step(), ... of a state of
 // n_amps amplitudes (tile_bits 10: 1024 amplitudes, 8 KB of stage per warp).
 // w and mat (row-major 2^TB x 2^TB entries) are in shared memory.  A tile is
 // copied asynchronously into the warp's stage: 8 bytes per lane and slot, or,
@@ -77,16 +77,18 @@ __device__ __forceinline__ uint32_t lane_phys(const WarpTile& w, int lane)
 // to 32 / 2^TB units, KB units and RB rows at a time so that one matrix entry
 // read serves KB units and 2 KB RB FMA chains are in flight, and the tile is
 // stored back.  Warps never synchronise with one another.
-template <int TB, bool PAIRS_ANY_TB>
+// step(): the stride, worked out anew for each tile (held in registers it made
+// the batch's 4-qubit passes spill, 10 to 20 % of their time).
+template <int TB, bool PAIRS_ANY_TB, typename Step>
 __device__ void tiled_dense_c64(float2* a, uint64_t n_amps, const WarpTile& w, const float2* mat, float2* stage,
-                                uint64_t t0, uint64_t tstride)
+                                uint32_t t0, Step step)
 {
     constexpr int D = 1 << TB;
     constexpr int U = 32 >> TB;
     constexpr int KB = U < 2 ? U : 2;
     constexpr int RB = TB >= 3 ? 2 : 1;
     const int lane = threadIdx.x & 31;
-    const uint64_t tiles = n_amps >> 10;
+    const uint32_t tiles = (uint32_t)(n_amps >> 10);
     const uint32_t plane = lane_phys(w, lane);
     // 16-byte form: lane l moves amplitudes 2i, 2i+1 (i = l & 15) of slot 2mm + (l >> 4)
     uint32_t p16 = 0;
@@ -98,7 +100,7 @@ __device__ void tiled_dense_c64(float2* a, uint64_t n_amps, const WarpTile& w, c
     for (int b = 0; b < 5; ++b)
         if ((lane >> b) & 1) pl ^= w.wbit[b];
 
-    for (uint64_t t = t0; t < tiles; t += tstride) {
+    for (uint32_t t = t0; t < tiles; t += step()) {
         // slot offsets from the five basis values, read per tile (volatile)
         // so that the 64 derived offsets are not kept in registers across tiles
         uint32_t gb[5], sb[5];
