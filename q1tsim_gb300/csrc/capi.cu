@@ -104,26 +104,17 @@ int q1g_state_from_qubit_coefs(const double* coefs, size_t nr_bits, size_t nr_sh
         need(coefs, "coefs");
         check_new(nr_bits, precision);
         // normalise each qubit's (c0, c1) pair (src/vectorstate.rs:69-73)
-        std::vector<double> c(coefs, coefs + 4 * nr_bits);
+        ProductCoefs c{};
+        std::copy_n(coefs, 4 * nr_bits, c.c);
         for (size_t q = 0; q < nr_bits; ++q) {
-            double* p = c.data() + 4 * q;
+            double* p = c.c + 4 * q;
             const double norm = std::sqrt(p[0] * p[0] + p[1] * p[1] + p[2] * p[2] + p[3] * p[3]);
             for (int j = 0; j < 4; ++j) p[j] /= norm;
         }
         auto* s = new q1g_state((int)nr_bits, nr_shots, precision);
         try {
-            // the coefficients, then the kernel's table of the high qubits
-            const size_t cbytes = (c.size() * sizeof(double) + 255) & ~size_t(255);
-            s->dscratch.ensure(std::max<size_t>(cbytes + product_state_tmp_bytes((int)nr_bits), 256));
-            s->h2d(s->dscratch.p, c.data(), c.size() * sizeof(double), "upload coefs");
-            s->amps.ensure(s->N * s->bsz());
-            s->launch("product_state", double(s->N * s->bsz()), [&] {
-                return launch_product_state(s->amps.p, s->prec, (int)nr_bits, s->dscratch.as<double>(),
-                                            s->dscratch.as<char>() + cbytes, s->stream);
-            });
+            s->product_state(c);
             s->sync();
-            s->sparse = false;
-            s->basis.clear();
         } catch (...) {
             delete s;
             throw;

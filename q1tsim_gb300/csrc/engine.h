@@ -181,6 +181,7 @@ struct q1g_state {
     void collect_profile();
 
     void ensure_dense();
+    void product_state(const q1g::ProductCoefs& c);     // one column, that state
     void clear_error_flag();               // of the tensor-core passes
     void settle_norms();
     std::vector<double> measure_norms();   // each column's squared norm, FP64, now

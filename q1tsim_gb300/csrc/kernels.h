@@ -337,9 +337,14 @@ struct SubspacePositions {
 constexpr int kFillMaxExcluded = 8;
 cudaError_t launch_scatter_subspace(void* full, const void* compact, int prec, int nbits_full, int nbits_compact,
                                    const SubspacePositions& sp, uint64_t fixed, cudaStream_t st);
-// The product of nbits qubits' (c0, c1) pairs; tmp: product_state_tmp_bytes.
+// The product of nbits qubits' (c0, c1) pairs (re, im, re, im of qubit q at
+// c[4 q]), a kernel parameter; tmp: product_state_tmp_bytes.
+struct ProductCoefs {
+    double c[4 * 48];
+};
 uint64_t product_state_tmp_bytes(int nbits);
-cudaError_t launch_product_state(void* amps, int prec, int nbits, const double* d_coefs, void* tmp, cudaStream_t st);
+cudaError_t launch_product_state(void* amps, int prec, int nbits, const ProductCoefs& coefs, void* tmp,
+                                 cudaStream_t st);
 cudaError_t launch_convert_c128_to_c64(float2* dst, const double2* src, uint64_t n, cudaStream_t st);
 // total amplitudes with re, im i.i.d. N(0,1) from the SplitMix64 stream
 // `seed` (amplitude i: Box-Muller of uniforms 2i, 2i+1); not normalised.

@@ -27,7 +27,7 @@ __global__ void k_set_basis(T* a, const uint64_t* col_index, uint64_t ncols, uin
 // amp(i) = c_0[b_0] * c_1[b_1] * ... multiplied left to right, b_q the bit of
 // qubit q (position n-1-q) -- the kron chain of src/vectorstate.rs:68-74.
 template <typename T>
-__global__ void k_product_state(T* a, int nbits, const double* coefs)
+__global__ void k_product_state(T* a, int nbits, const __grid_constant__ ProductCoefs coefs)
 {
     const uint64_t n = uint64_t(1) << nbits;
     const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
@@ -35,7 +35,8 @@ __global__ void k_product_state(T* a, int nbits, const double* coefs)
         double re = 1.0, im = 0.0;
         for (int q = 0; q < nbits; ++q) {
             const int b = (i >> (nbits - 1 - q)) & 1;
-            const double cr = coefs[4 * q + 2 * b], ci = coefs[4 * q + 2 * b + 1];
+            const double* c = coefs.c + 4 * q;
+            const double cr = b ? c[2] : c[0], ci = b ? c[3] : c[1];
             const double nr = cr * re - ci * im;
             const double ni = cr * im + ci * re;
             re = nr;
@@ -84,7 +85,7 @@ __device__ __forceinline__ void product_store(float2* a, const DfAmp& h, const D
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 k_product_rows(T* __restrict__ a, uint64_t rows, const double2* __restrict__ high, int nbits,
-               const double* __restrict__ coefs)
+               const __grid_constant__ ProductCoefs coefs)
 {
     constexpr int N = 1 << kProductLow;
     __shared__ double2 low[N];
@@ -93,7 +94,7 @@ k_product_rows(T* __restrict__ a, uint64_t rows, const double2* __restrict__ hig
     // the last qubit is the lowest bit: entries of bits 0..b-1 give those of
     // bit b by its qubit's two coefficients
     for (int b = 0; b < kProductLow; ++b) {
-        const double* c = coefs + 4 * (nbits - 1 - b);
+        const double* c = coefs.c + 4 * (nbits - 1 - b);
         const double2 c0 = make_double2(c[0], c[1]), c1 = make_double2(c[2], c[3]);
         for (int j = threadIdx.x; j < (1 << b); j += kThreads) {
             const double2 v = low[j];
@@ -372,30 +373,32 @@ uint64_t product_state_tmp_bytes(int nbits)
 }
 
 template <typename T>
-static void product_direct(T* a, int nbits, const double* d_coefs, cudaStream_t st)
+static void product_direct(T* a, int nbits, const ProductCoefs& coefs, cudaStream_t st)
 {
     const uint64_t n = uint64_t(1) << nbits;
     const unsigned grid = blocks_for(n, kThreads) > 152 * 64 ? 152 * 64 : blocks_for(n, kThreads);
-    k_product_state<T><<<grid, kThreads, 0, st>>>(a, nbits, d_coefs);
+    k_product_state<T><<<grid, kThreads, 0, st>>>(a, nbits, coefs);
 }
 
-cudaError_t launch_product_state(void* amps, int prec, int nbits, const double* d_coefs, void* tmp, cudaStream_t st)
+cudaError_t launch_product_state(void* amps, int prec, int nbits, const ProductCoefs& coefs, void* tmp,
+                                 cudaStream_t st)
 {
+    if (nbits > 48) return cudaErrorInvalidValue;
     if (nbits < kProductTwoLevelBits) {
-        if (prec == kC128) product_direct((double2*)amps, nbits, d_coefs, st);
-        else product_direct((float2*)amps, nbits, d_coefs, st);
+        if (prec == kC128) product_direct((double2*)amps, nbits, coefs, st);
+        else product_direct((float2*)amps, nbits, coefs, st);
         return cudaGetLastError();
     }
     // qubits 0 .. n-1-kProductLow are the row's bits, in the same order
-    product_direct((double2*)tmp, nbits - kProductLow, d_coefs, st);
+    product_direct((double2*)tmp, nbits - kProductLow, coefs, st);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const uint64_t rows = uint64_t(1) << (nbits - kProductLow);
     const unsigned grid = (unsigned)(rows < 152 * 6 ? rows : 152 * 6);
     if (prec == kC128)
-        k_product_rows<double2><<<grid, kThreads, 0, st>>>((double2*)amps, rows, (const double2*)tmp, nbits, d_coefs);
+        k_product_rows<double2><<<grid, kThreads, 0, st>>>((double2*)amps, rows, (const double2*)tmp, nbits, coefs);
     else
-        k_product_rows<float2><<<grid, kThreads, 0, st>>>((float2*)amps, rows, (const double2*)tmp, nbits, d_coefs);
+        k_product_rows<float2><<<grid, kThreads, 0, st>>>((float2*)amps, rows, (const double2*)tmp, nbits, coefs);
     return cudaGetLastError();
 }
 
