@@ -107,9 +107,10 @@ def test_block_on_several_columns():
         assert np.all(np.abs(after[:, c] - want) <= ROW_TOL * top)
 
 
-@pytest.mark.parametrize("n,shots,depth", [(22, 1, 3), (22, 1, 6), (21, 5, 4)])
-def test_plain_gates_as_blocks(n, shots, depth):
-    """Gates of a plan without fusion, multiplied into blocks where that is
+@pytest.mark.parametrize("n,shots,depth,width", [(22, 1, 3, 0), (22, 1, 6, 0), (21, 5, 4, 0), (22, 1, 3, 3),
+                                                 (22, 1, 4, 2)])
+def test_plain_gates_as_blocks(n, shots, depth, width):
+    """Gates of a plan without fusion, or with narrow blocks, multiplied into blocks where that is
     faster, against the same plan on the CUDA cores.  Tolerance: 2^-45 per pass
     of either (both are some 20 passes of 1e-15)."""
     rng = np.random.default_rng(n + depth)
@@ -132,7 +133,7 @@ def test_plain_gates_as_blocks(n, shots, depth):
             s.measure(3, rng=Rng(1))
         s.profile(True)
         s.profile_report(reset=True)
-        s.apply_plan(Plan(n, bits, 0, tensor_cores=tc), flat)
+        s.apply_plan(Plan(n, bits, width, tensor_cores=tc), flat)
         assert ("fused_tc_c128" in s.profile_report()) == tc
         out.append(s.states())
     assert np.linalg.norm(out[0] - out[1]) <= 40 * 2.0 ** -45 * np.linalg.norm(out[1])
