@@ -222,7 +222,7 @@ struct TcPass {
 struct q1g_plan {
     int nbits = 0;
     int width = 0;
-    int tensor_cores = 1;          // 1: complex64 dense blocks on tcgen05; 0: CUDA cores
+    int tensor_cores = 1;          // 1: dense blocks on tcgen05; 0: CUDA cores
     std::vector<std::vector<int>> gate_bits;
     std::vector<size_t> mat_off;   // offset (doubles) of each gate's matrix
     size_t mat_doubles = 0;

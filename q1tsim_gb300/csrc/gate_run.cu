@@ -12,8 +12,9 @@
 // memory is read and written once per 40-60 gates), on small ones the
 // latency of a gate's chain, about 0.5 us.  Measured on one GB300 against one
 // launch and one HBM pass per gate: complex128 brick circuits of 10 qubits,
-// depth 8 (116 gates) 0.64 -> 0.25 ms, 16 qubits, depth 20 (470 gates)
-// 2.86 -> 0.76 ms, 26 qubits, depth 6 (231 gates) 59.9 -> 35.5 ms.
+// depth 8 (116 gates) 0.63 -> 0.12 ms (with the plan's launches kept), 16 qubits,
+// depth 20 (470 gates) 2.86 -> 0.40 ms, 26 qubits, depth 6 (231 gates) 59.9 ->
+// 35.5 ms (complex128 states of that size take the tensor cores now, 11.5 ms).
 #include <algorithm>
 #include <mutex>
 #include <set>
