@@ -1254,11 +1254,11 @@ struct PlainGate {
     SeqGate gate;
 };
 
-// Microseconds of a complex128 tensor-core pass (6.9 per tile of an SM: 0.75 ms
+// Microseconds of a complex128 tensor-core pass (6.2 to 6.9 per tile of an SM: 0.70 ms
 // at 26 qubits), or of a block's matrix on the host where that is longer.
 static double z_pass_us(uint64_t total)
 {
-    return std::max(5.0 + 6.9 * std::ceil((double)(total >> 12) / 152.0), 100.0);
+    return std::max(5.0 + 6.4 * std::ceil((double)(total >> 12) / 152.0), 100.0);
 }
 
 // A run of plain gates: as tile passes (gate_run.h), or, on complex128

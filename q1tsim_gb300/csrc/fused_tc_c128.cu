@@ -21,7 +21,8 @@
 // of the row's amplitudes, so a warp's 256 amplitudes lie in whole runs of at
 // least 8 (its rows' and states' low bits include the tile's three lowest): it
 // copies them in (cp.async) and, rearranged through shared memory, out by
-// itself.  TMEM has room for one tile only: 128 columns of A (digit s < 4 in
+// itself.  Where the lowest positions are rows (kDirect) a thread copies its own
+// amplitudes in, and writes them straight to memory.  TMEM has room for one tile only: 128 columns of A (digit s < 4 in
 // columns 32 s ..: one 32-bit column per amplitude; the other two digits are in
 // shared memory), 384 of accumulators.  So the next tile's digits wait in
 // registers while the MMAs of a tile run; when these are done every thread
@@ -35,9 +36,10 @@
 // (32 KB), the tile coming in and the tile going out (64 KB each),
 // XOR-swizzled so that lanes hit distinct banks.
 //
-// 27 qubits: 1.49 ms per pass of up to five qubits (13.4 k cycles per tile;
-// its bytes take 5.9 k of the SM's share of HBM), against 1.75 ms per pass of
-// three in double-float warp tiles.  What bounds it is the threads' own work,
+// 27 qubits: 1.30 ms per pass of up to five qubits, 1.49 where the lowest
+// positions are gates (11.8 k and 13.4 k cycles per tile; its bytes take 5.9 k of
+// the SM's share of HBM), against 1.75 ms per pass of three in double-float warp
+// tiles.  What bounds it is the threads' own work,
 // half of it integer arithmetic at half rate: digits 2.6 k cycles, carries and
 // joins 5 k, copies 3 k; the MMAs (3 k) run under it.  One tile after another
 // without the overlap took 1.61 ms.  Tried and slower: the digits' carries
@@ -297,6 +299,7 @@ __device__ __forceinline__ void issue_step(uint32_t ks, uint32_t tmem, uint32_t 
     if (ks == 3) mma_commit(mbar);
 }
 
+template <bool kDirect>
 __global__ void __launch_bounds__(kZThreads, 1)
 k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant__ ZPass p,
                 const double2* __restrict__ mat, int* __restrict__ err, uint64_t wait_ns)
@@ -512,7 +515,15 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
                 const uint32_t to = at(out, j);
                 if (mid) {
                     const uint32_t up20 = (uint32_t)back20 + (896u << 20);
-                    sts_amp(to, scaled_join_mid(h.x, l.x, up20), scaled_join_mid(h.y, l.y, up20));
+                    const double re = scaled_join_mid(h.x, l.x, up20), im = scaled_join_mid(h.y, l.y, up20);
+                    if (kDirect) {
+                        uint64_t g;
+                        uint32_t s;
+                        element(j, g, s);
+                        dst[g] = make_double2(re, im);
+                    } else {
+                        sts_amp(to, re, im);
+                    }
                 } else {
                     sts_raw(to, h, l);
                 }
@@ -533,14 +544,17 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
                 }
             }
             if (issue) issue_step(2u, tmem, sbase, mbar);
-            __syncwarp();
+            if (!kDirect || !__all_sync(0xFFFFFFFFu, mid)) {
+                __syncwarp();
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                uint64_t g;
-                uint32_t s;
-                element(k, g, s);
-                const ulonglong2 v = lds_amp(out + s * 16u);
-                dst[g] = make_double2(__longlong_as_double((long long)v.x), __longlong_as_double((long long)v.y));
+                for (int k = 0; k < 8; ++k) {
+                    uint64_t g;
+                    uint32_t s;
+                    element(k, g, s);
+                    const ulonglong2 v = lds_amp(out + s * 16u);
+                    if (!kDirect || !mid)
+                        dst[g] = make_double2(__longlong_as_double((long long)v.x), __longlong_as_double((long long)v.y));
+                }
             }
         }
         if (kLast && issue) issue_step(3u, tmem, sbase, mbar);
@@ -582,9 +596,19 @@ void z_pass_layout(ZPass& p, const int* tile_pos, const int* gate_of)
     int rows[7], r = 0, wb[8], w = 0;
     for (int j = 0; j < 12; ++j)
         if (!((gate_bits >> j) & 1u)) rows[r++] = j;
-    for (int j = 0; j < 12; ++j)
-        if (j == gate_of[0] || j == gate_of[1] || j == gate_of[2] || std::find(rows, rows + 5, j) != rows + 5)
-            wb[w++] = j;
+    // Straight to memory where that fills whole 32-byte sectors and at least
+    // half-lines: tile bit 0 and one of bits 1 and 2 are rows.  26 qubits, us,
+    // straight / staged: lowest gate position 3 or higher 660 / 745, 2 670 / 745, 1
+    // 708 / 745; 1 and 2 762 / 745.
+    p.direct = rows[0] == 0 && rows[1] <= 2;
+    if (p.direct) {
+        for (int i = 0; i < 5; ++i) wb[w++] = rows[i];
+        for (int i = 0; i < 3; ++i) wb[w++] = gate_of[i];
+    } else {
+        for (int j = 0; j < 12; ++j)
+            if (j == gate_of[0] || j == gate_of[1] || j == gate_of[2] || std::find(rows, rows + 5, j) != rows + 5)
+                wb[w++] = j;
+    }
     for (int i = 0; i < 8; ++i) {
         p.off[i] = uint64_t(1) << tile_pos[wb[i]];
         p.slot[i] = 1u << i;
@@ -621,7 +645,11 @@ cudaError_t launch_fused_tc_c128(double2* amps, uint64_t total, const ZPass& p, 
     {
         std::lock_guard<std::mutex> lock(mu);
         if (!done[dev]) {
-            e = cudaFuncSetAttribute(k_fused_tc_c128, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZSmemAlloc);
+            e = cudaFuncSetAttribute(k_fused_tc_c128<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kZSmemAlloc);
+            if (e != cudaSuccess) return e;
+            e = cudaFuncSetAttribute(k_fused_tc_c128<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kZSmemAlloc);
             if (e != cudaSuccess) return e;
             done[dev] = true;
         }
@@ -629,8 +657,9 @@ cudaError_t launch_fused_tc_c128(double2* amps, uint64_t total, const ZPass& p, 
     const uint64_t ntiles = total / kZTile;
     if (ntiles == 0) return cudaErrorInvalidValue;
     const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)sm_count, ntiles);
-    k_fused_tc_c128<<<grid, kZThreads, kZSmemAlloc, st>>>(amps, ntiles, p, static_cast<const double2*>(d_mat), d_err,
-                                                         wait_ns ? wait_ns : kTcDefaultWaitNs);
+    const auto kernel = p.direct ? k_fused_tc_c128<true> : k_fused_tc_c128<false>;
+    kernel<<<grid, kZThreads, kZSmemAlloc, st>>>(amps, ntiles, p, static_cast<const double2*>(d_mat), d_err,
+                                                 wait_ns ? wait_ns : kTcDefaultWaitNs);
     return cudaGetLastError();
 }
 

@@ -307,6 +307,7 @@ struct ZPass {
     uint32_t slot[8];
     uint8_t row_of[5];
     uint8_t gate_of[3];
+    bool direct;             // a lane's elements are its own row's, in the order of the states
 };
 // gate_of[k]: the tile bit of matrix index bit k, ascending.
 void z_pass_layout(ZPass& p, const int* tile_pos /* 12, ascending */, const int* gate_of);

@@ -1,8 +1,8 @@
 // CPU check of the complex128 tensor-core pass's layout (z_pass_layout in
 // libq1gpu.so): in each warp's part of a tile elements and (row, state) pairs
 // take every slot once and agree on the offsets, the 8 lanes of a phase hit
-// distinct bank groups in both, elements come in runs of 8 or more, and the
-// parts of all tiles cover the state.
+// distinct bank groups in both, elements come in runs of 8 or more (2 where
+// they are the lanes' own), and the parts of all tiles cover the state.
 // Prints "bad <count>"; exit status 1 on any failure.
 #include <algorithm>
 #include <cstdio>
@@ -42,7 +42,15 @@ int main()
                 if ((e >> i) & 1) s ^= p.slot[i], o |= p.off[i];
             if (s >= 256 || at[s] != ~0ull) ++bad;
             else at[s] = o;
-            bad += (o & 7) != (e & 7);
+            bad += (o ^ e) & (p.direct ? 1 : 7);
+            if (p.direct) {      // lane e % 32's own row, state e / 32
+                uint64_t own = 0;
+                for (int b = 0; b < 5; ++b)
+                    if ((e >> b) & 1) own |= uint64_t(1) << T[rows[b]];
+                for (int k = 0; k < 3; ++k)
+                    if ((e >> (5 + k)) & 1) own |= uint64_t(1) << g[k];
+                bad += o != own;
+            }
             if ((e & 7) == 0) {
                 uint32_t banks = 0;
                 for (uint32_t l = 0; l < 8; ++l) {
