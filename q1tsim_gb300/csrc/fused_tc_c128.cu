@@ -100,20 +100,18 @@ __device__ __forceinline__ float2 splat(float v) { return make_float2(v, v); }
 // 1.5 * 2^23: adding and subtracting it rounds |v| < 2^22 to an integer
 constexpr float kRound = 12582912.0f;
 
-// x scaled by 2^shift (exponent bits added), as h + l; zero where the high
-// word of |x| is below `least`: 2^-47 after scaling (a row's last digit is
-// 2^-45).  The scaled exponent is at most 1030: split_fast (df64.cuh) on the
-// scaled bits.
-__device__ __forceinline__ DF scaled_split(uint64_t bits, uint32_t shift20, uint32_t least)
+// x scaled by 2^shift (exponent bits added), as h + l.  High words of |x| below
+// `floor` count as it: 2^-74 after scaling, where a row's last digit is 2^-45.
+// The scaled exponent is 949 to 1030: split_fast (df64.cuh) on the scaled bits.
+__device__ __forceinline__ DF scaled_split(uint64_t bits, uint32_t shift20, uint32_t floor)
 {
-    const uint32_t hw = (uint32_t)(bits >> 32) + shift20, lw = (uint32_t)bits;
-    const uint32_t sign = hw & 0x80000000u;
+    const uint32_t top = (uint32_t)(bits >> 32), lw = (uint32_t)bits, sign = top & 0x80000000u;
+    const uint32_t hw = max(top & 0x7FFFFFFFu, floor) + shift20;
     const uint32_t t = __funnelshift_r(lw + (1u << 28), hw + (lw > 0xEFFFFFFFu ? 1u : 0u), 29);
     const float h = __uint_as_float((t - (896u << 23)) | sign);
     const float r = (float)((int32_t)(lw << 3) >> 3);
     const float l = r * __uint_as_float((((hw << 3) & 0xFF800000u) - (948u << 23)) | sign);
-    const bool zero = ((uint32_t)(bits >> 32) & 0x7FFFFFFFu) < least;
-    return zero ? DF{0.0f, 0.0f} : DF{h, l};
+    return DF{h, l};
 }
 
 // The six digits of an amplitude's components as f16 pairs.
@@ -435,9 +433,10 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
         const bool more = i + 1 < count;
         const double2* src = a + bases[(i + 1) % kZBases];
         // the row's largest exponent becomes that of 2^7 .. 2^8; a row
-        // below 2^-968 counts as zero
-        const uint32_t shift20 = (1030u << 20) - m;
-        const uint32_t least = m <= (54u << 20) ? 0xFFFFFFFFu : m - (54u << 20);
+        // below 2^-940 counts as zero
+        const bool tiny = m <= (82u << 20);
+        const uint32_t shift20 = tiny ? 0u : (1030u << 20) - m;
+        const uint32_t floor = tiny ? 949u << 20 : m - (81u << 20);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             uint64_t g;
@@ -445,7 +444,7 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
             element(j, g, s);
             if (more) cp_async16(smem + (in - sbase) + s * 16u, src + g);
             uint32_t d[6];
-            digits(scaled_split(x[j].x, shift20, least), scaled_split(x[j].y, shift20, least), d);
+            digits(scaled_split(x[j].x, shift20, floor), scaled_split(x[j].y, shift20, floor), d);
 #pragma unroll
             for (int s = 0; s < 6; ++s) dg[s][j] = d[s];
         }
@@ -462,7 +461,9 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
         float acc[5][16];
         if (warp == 15 && lane == 0) put_base(it + 2);
         if (kLast) {
+            __syncwarp();      // (lane 0 of warp 0 may be behind, issuing)
             ok = wait_phase(mbar, (uint32_t)(it - 1) & 1u, abort_flag, wait_ns);
+            __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
         if (kTile) {
