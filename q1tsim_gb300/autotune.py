@@ -4,8 +4,8 @@ tensor-core tiling.
 For one circuit structure (qubit count, precision and the qubits of each
 gate), every candidate is lowered to a plan and timed on a scratch state of
 the same shape; the fastest one is remembered for that structure.  A
-candidate is a fusion width, whether complex64 dense blocks run on the
-tensor cores or the CUDA cores, and for tensor-core plans the tiling of
+candidate is a fusion width, whether dense blocks run on the tensor cores
+or the CUDA cores, and for tensor-core plans the tiling of
 their passes (q1g_plan_set_tc_tiling): whether two blocks may share a pass,
 how many tile positions of a pair may lie at large-page strides, and how
 many bank conflicts an unpadded one-box tile may take before it is padded.
@@ -24,11 +24,14 @@ DEFAULT_TILING = Plan.DEFAULT_TC_TILING
 # pairs; pairs over fewer large pages; a tighter conflict slack
 TC_TILINGS = (DEFAULT_TILING, (5, 8, 4), (1, 8, 2), (2, 8, 2), (3, 8, 2), (0, 8, 2), (4, 5, 4), (4, 8, 2))
 
-# (fusion width, dense complex64 blocks on tensor cores, tiling)
+# (fusion width, dense blocks on tensor cores, tiling)
 CANDIDATES_C64 = tuple((5, True, t) for t in TC_TILINGS) + (
     (4, True, DEFAULT_TILING), (3, True, DEFAULT_TILING),
     (4, False, DEFAULT_TILING), (3, False, DEFAULT_TILING), (2, False, DEFAULT_TILING), (0, False, DEFAULT_TILING))
 CANDIDATES_C128 = tuple((w, False, DEFAULT_TILING) for w in (0, 1, 2, 3))
+# from 12 qubits on (the tensor cores' tile): 24 qubits, 8 layers, 2.0 ms with
+# width 5 and 3.1 with 0, 9.9 the best without them
+CANDIDATES_C128_TC = ((5, True, DEFAULT_TILING), (0, True, DEFAULT_TILING))
 
 _cache = {}
 
@@ -52,6 +55,8 @@ def tune(nr_bits, precision, gate_bits, mats_flat, reps=2, candidates=None, kind
         return _cache[key]
     if candidates is None:
         candidates = CANDIDATES_C64 if precision == "c64" else CANDIDATES_C128
+        if precision != "c64" and nr_bits >= 12:
+            candidates = CANDIDATES_C128_TC + candidates
     scratch = VectorState(nr_bits, 1, precision)
     timings = []
     for width, tc, tiling in candidates:
