@@ -117,6 +117,7 @@ def load():
     _proto(L, "q1g_last_error_args", None, [_u64p, _u64p])
     _proto(L, "q1g_version", _int, [])
     _proto(L, "q1g_device_info", _int, [ctypes.POINTER(_int), _szp, _szp])
+    _proto(L, "q1g_release_cached_memory", _int, [])
     _proto(L, "q1g_state_new", _int, [_sz, _sz, _int, ctypes.POINTER(_vp)])
     _proto(L, "q1g_state_from_qubit_coefs", _int, [_dp, _sz, _sz, _int, ctypes.POINTER(_vp)])
     _proto(L, "q1g_state_from_amplitudes", _int, [_dp, _sz, _sz, _int, ctypes.POINTER(_vp)])

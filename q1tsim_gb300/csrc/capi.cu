@@ -82,9 +82,14 @@ int q1g_device_info(int* sm_count, size_t* free_bytes, size_t* total_bytes)
         if (sm_count) check_cuda(cudaDeviceGetAttribute(sm_count, cudaDevAttrMultiProcessorCount, dev), "attr");
         size_t f = 0, t = 0;
         check_cuda(cudaMemGetInfo(&f, &t), "cudaMemGetInfo");
-        if (free_bytes) *free_bytes = f;
+        if (free_bytes) *free_bytes = f + cached_device_bytes();
         if (total_bytes) *total_bytes = t;
     });
+}
+
+int q1g_release_cached_memory(void)
+{
+    return guarded([&] { release_cached_memory(); });
 }
 
 int q1g_state_new(size_t nr_bits, size_t nr_shots, int precision, q1g_state** out)

@@ -45,10 +45,17 @@ struct DevBuf {
     {
         std::swap(p, o.p);
         std::swap(bytes, o.bytes);
+        std::swap(dev, o.dev);
     }
     ~DevBuf() { release(); }
     template <typename T> T* as() const { return static_cast<T*>(p); }
+
+private:
+    int dev = -1;
 };
+// Device memory that released buffers left for new ones, and its return.
+size_t cached_device_bytes();
+void release_cached_memory();
 
 // Grow-only pinned host allocation.
 struct HostBuf {

@@ -404,6 +404,12 @@ def device_info():
     return {"sm_count": sm.value, "free_bytes": free.value, "total_bytes": total.value}
 
 
+def release_cached_memory():
+    """Return the device memory that freed states left for new ones (up to
+    4 GiB) to the device (q1g_release_cached_memory)."""
+    check(_lib.load().q1g_release_cached_memory())
+
+
 def device_histogram(words, stream=None, sort=True):
     """Distinct values of a uint64 array and their counts, counted on the
     GPU (q1g_histogram): the classical-word histogram of a circuit with many
