@@ -8,7 +8,7 @@ and roundings far below: 2^-45 of it."""
 import numpy as np
 import pytest
 
-from q1tsim_gb300 import Plan, Rng, VectorState
+from q1tsim_gb300 import DeviceTimeout, Plan, Rng, VectorState
 from test_gpu_parity import rand_state, rand_unitary
 
 pytestmark = pytest.mark.gpu
@@ -137,3 +137,23 @@ def test_plain_gates_as_blocks(n, shots, depth, width):
         assert ("fused_tc_c128" in s.profile_report()) == tc
         out.append(s.states())
     assert np.linalg.norm(out[0] - out[1]) <= 40 * 2.0 ** -45 * np.linalg.norm(out[1])
+
+
+@pytest.mark.parametrize("n", [12, 16, 22])
+def test_expired_wait_is_reported_and_the_state_usable(n):
+    """A limit that every wait for the MMAs exceeds: an error, nothing left
+    behind, and the same plan runs with the default limit."""
+    rng = np.random.default_rng(n)
+    amps, m, qubits = rand_state(n, rng), rand_unitary(32, rng), [n - 1, 3, 0, 7, 5]
+    s = VectorState.from_amplitudes(amps, 1, "c128")
+    s.set_wait_limit(1e-9)
+    plan, flat = Plan(n, [qubits], 5), np.ascontiguousarray(m).ravel().view(np.float64)
+    with pytest.raises(DeviceTimeout):
+        s.apply_plan(plan, flat)
+    s.set_wait_limit(0)
+    s.reset_all()
+    s.apply_plan(plan, flat)
+    start = np.zeros(1 << n, dtype=np.complex128)
+    start[0] = 1.0
+    assert np.linalg.norm(s.states()[:, 0] - _apply(start, m, qubits, n)[0]) <= 1e-14
+    np.testing.assert_allclose(_run(amps, m, qubits, n), _apply(amps, m, qubits, n)[0], rtol=0, atol=1e-14)
