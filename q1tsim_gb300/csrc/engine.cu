@@ -9,7 +9,6 @@
 
 #include <algorithm>
 #include <array>
-#include <map>
 #include <memory>
 #include <mutex>
 #include <set>
@@ -28,49 +27,65 @@ void check_cuda(cudaError_t e, const char* what)
 
 // Released device memory, kept per device for the next buffers: cudaMalloc and
 // cudaFree of a 27-qubit complex128 state (2 GiB) take 1.7 ms, its product
-// state 1.0.  Bounded (kPoolBytes a device); returned when an allocation fails
-// and by q1g_release_cached_memory.  A block enters only after the device
-// has finished everything (as cudaFree waits, too), so any stream or thread may
-// have it next.
+// state 1.0.  Bounded (kPoolBytes a device, the oldest blocks make room);
+// returned when an allocation fails and by q1g_release_cached_memory.  A block
+// enters only after the device has finished everything (as cudaFree waits, too),
+// so any stream or thread may have it next.
 namespace {
 
 constexpr size_t kPoolBytes = size_t(4) << 30;
+constexpr size_t kPoolBlocks = 256;
 constexpr int kPoolDevices = 64;
 
 struct DevicePool {
+    struct Block {
+        size_t size;
+        void* p;
+    };
     std::mutex mu;
-    std::multimap<size_t, void*> blocks;
+    std::deque<Block> blocks;      // oldest first
     size_t bytes = 0;
 
-    // A block of at least `size` bytes and not much more, or null.
+    // The smallest block of at least `size` bytes and not much more, or null.
     void* take(size_t size, size_t* got)
     {
         std::lock_guard<std::mutex> lock(mu);
-        const auto it = blocks.lower_bound(size);
-        if (it == blocks.end() || it->first > std::max(size + size / 8, size_t(1) << 16)) return nullptr;
-        void* q = it->second;
-        *got = it->first;
-        bytes -= it->first;
-        blocks.erase(it);
+        const size_t most = std::max(size + size / 8, size_t(1) << 16);
+        auto best = blocks.end();
+        for (auto it = blocks.begin(); it != blocks.end(); ++it)
+            if (it->size >= size && it->size <= most && (best == blocks.end() || it->size < best->size)) best = it;
+        if (best == blocks.end()) return nullptr;
+        void* q = best->p;
+        *got = best->size;
+        bytes -= best->size;
+        blocks.erase(best);
         return q;
     }
-    bool put(void* q, size_t size)
+    // Keeps a block; the oldest ones make room.
+    void put(void* q, size_t size)
     {
-        std::lock_guard<std::mutex> lock(mu);
-        if (bytes + size > kPoolBytes) return false;
-        blocks.emplace(size, q);
-        bytes += size;
-        return true;
+        std::vector<void*> out;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            while (!blocks.empty() && (bytes + size > kPoolBytes || blocks.size() >= kPoolBlocks)) {
+                out.push_back(blocks.front().p);
+                bytes -= blocks.front().size;
+                blocks.pop_front();
+            }
+            blocks.push_back({size, q});
+            bytes += size;
+        }
+        for (void* o : out) cudaFree(o);
     }
     void trim()
     {
-        std::multimap<size_t, void*> all;
+        std::deque<Block> all;
         {
             std::lock_guard<std::mutex> lock(mu);
             all.swap(blocks);
             bytes = 0;
         }
-        for (auto& b : all) cudaFree(b.second);
+        for (const Block& o : all) cudaFree(o.p);
     }
 };
 
@@ -144,8 +159,12 @@ void DevBuf::release()
         int device;
         DevicePool* pool = bytes <= kPoolBytes ? current_pool(&device) : nullptr;
         const bool idle = pool && device == dev && cudaDeviceSynchronize() == cudaSuccess;
-        if (!idle) (void)cudaGetLastError();
-        if (!idle || !pool->put(p, bytes)) cudaFree(p);
+        if (idle) {
+            pool->put(p, bytes);
+        } else {
+            (void)cudaGetLastError();
+            cudaFree(p);
+        }
     }
     p = nullptr;
     bytes = 0;
