@@ -1727,7 +1727,7 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
             // A narrow plan's blocks on a large state: a pass takes the same
             // time for three qubits as for five, so their gates are grouped
             // anew with the plain ones (30 qubits, depth 24, plan of width 3:
-            // 1.84 s for its 169 passes, 0.66 s so).
+            // 1.84 s for its 169 passes, 0.58 s so).
             std::vector<PlainGate> again;
             for (int g : p->blocks[i].gates) {
                 GateOp o = classify(gates[g].mat.data(), (int)gates[g].bits.size(), gates[g].bits.data(), s->nbits);
