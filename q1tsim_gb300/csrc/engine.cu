@@ -1274,6 +1274,16 @@ static int group_position(const q1g_plan* p, const FusedBlock& b)
     return t >= 2 ? t : -1;
 }
 
+// Whether every angle is a number (a NaN has no fraction of a turn: such a run
+// goes alone, where its tables carry it to the amplitudes that it turns).
+static bool finite_phases(const PhaseFunction& f)
+{
+    auto all = [](const std::vector<double>& v) {
+        return std::all_of(v.begin(), v.end(), [](double x) { return std::isfinite(x); });
+    };
+    return std::isfinite(f.c) && all(f.lin0) && all(f.lin1);
+}
+
 // Blocks i .. as one group as far as they go (two at least), after the plain
 // gate `before` when the group starts with one (an uncontrolled 1-qubit
 // gate).  Returns the number of blocks taken, 0 for none.
@@ -1286,9 +1296,13 @@ static size_t lower_phase_group(q1g_plan* p, q1g_state* s, size_t i, const GateO
     auto taken = [&](int t) { return std::find(g.t, g.t + g.nsteps, t) != g.t + g.nsteps; };
     if (before) g.t[g.nsteps++] = before->map.zpos[0];
     size_t count = 0;
+    std::vector<PhaseFunction> phases;
     while (g.nsteps < kPhaseGroupMax && i + count < p->blocks.size()) {
-        const int t = group_position(p, p->blocks[i + count]);
+        const FusedBlock& b = p->blocks[i + count];
+        const int t = group_position(p, b);
         if (t < 0 || taken(t)) break;
+        phases.push_back(phase_function(p, n, b, gates));
+        if (!finite_phases(phases.back())) break;
         g.t[g.nsteps++] = t;
         ++count;
     }
@@ -1302,9 +1316,9 @@ static size_t lower_phase_group(q1g_plan* p, q1g_state* s, size_t i, const GateO
             f.lin0 = f.lin1 = none;
             std::copy(before->m2, before->m2 + 8, m2);
         } else {
-            const FusedBlock& b = p->blocks[i + k - (before ? 1 : 0)];
-            f = phase_function(p, n, b, gates);
-            const SeqGate& t = gates[b.gates.back()];
+            const size_t at = (size_t)k - (before ? 1 : 0);
+            f = phases[at];
+            const SeqGate& t = gates[p->blocks[i + at].gates.back()];
             for (int e = 0; e < 4; ++e) {
                 m2[2 * e] = t.mat[e].real();
                 m2[2 * e + 1] = t.mat[e].imag();
