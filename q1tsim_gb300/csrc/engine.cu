@@ -11,6 +11,7 @@
 #include <array>
 #include <memory>
 #include <mutex>
+#include <numeric>
 #include <set>
 #include <cmath>
 #include <cstdlib>
@@ -1405,9 +1406,11 @@ static double z_pass_us(uint64_t total)
 // layers in us, tile passes and tensor cores: 20 qubits 965 / 412, 22 qubits
 // 3680 / 1101, 24 qubits 15205 / 4758; but with new matrices, which the host
 // multiplies first, 1175 / 1900, 3864 / 2486 and 15453 / 6337, so the line lies
-// at 21 to 22 qubits.  A tile pass of one op, or one whose ops together touch
-// less than the state where that is what costs (a state beyond the L2: two CX
-// read and write half of it each), goes gate by gate.
+// at 21 to 22 qubits.  Blocks without a gate that rounds every amplitude
+// (controlled gates, phases, permutations alone) stay tile passes: those leave
+// the bits of what no arithmetic touches.  A tile pass of one op, or one whose
+// ops together touch less than the state where that is what costs (a state
+// beyond the L2: two CX read and write half of it each), goes gate by gate.
 template <typename Stage, typename Emit, typename Tc>
 static void lower_plain_gates(q1g_plan* p, q1g_state* s, const std::vector<PlainGate>& run, Stage&& stage, Emit&& emit,
                               Tc&& tensor_cores)
@@ -1420,32 +1423,101 @@ static void lower_plain_gates(q1g_plan* p, q1g_state* s, const std::vector<Plain
         for (const PlainGate& g : run) one(g.op);
         return;
     }
-    std::vector<const GateOp*> list;
-    for (const PlainGate& g : run) list.push_back(&g.op);
+    // tile passes of the gates `at` of the run
+    auto group = [&](const std::vector<int>& at, double* cost) {
+        std::vector<const GateOp*> list;
+        for (int i : at) list.push_back(&run[i].op);
+        return group_runs(list, s->nbits, total, s->prec, s->fp64_exact, cost);
+    };
+    const bool pairs = s->prec == kC128 && !s->fp64_exact;
+    std::vector<RunOp> table;
+    auto emit_passes = [&](const std::vector<int>& at, const std::vector<RunPass>& passes) {
+        for (const RunPass& pass : passes) {
+            uint64_t touched = 0;
+            bool units = true, rounded = false;
+            for (int i : pass.ops) {
+                const GateOp& op = run[at[i]].op;
+                touched += op.touched(total);
+                units = units && is_unit(op);
+                rounded = rounded || rounds_all(op);
+            }
+            if (pass.ops.size() < 2 || (touched <= total && total * s->bsz() > (uint64_t(64) << 20))) {
+                for (int i : pass.ops) one(run[at[i]].op);
+                continue;
+            }
+            table.clear();
+            for (int i : pass.ops) table.push_back(make_run_op(run[at[i]].op, pass.tile));
+            const RunArith arith = !pairs || units ? RunArith::kPlain
+                                   : rounded       ? RunArith::kPairs
+                                                   : RunArith::kPairsPartly;
+            const char* name = s->prec == kC64 ? "gate_run_c64" : s->fp64_exact ? "gate_run_c128_fp64" : "gate_run_c128";
+            const RunOp* d = static_cast<const RunOp*>(stage(table.data(), table.size() * sizeof(RunOp)));
+            emit([name, arith, tile = pass.tile, d, n = (int)table.size()](q1g_state* x) {
+                x->launch(name, 2.0 * x->total() * x->bsz(), [&] {
+                    return launch_gate_run(x->amps.p, x->prec, x->total(), tile, d, n, arith, x->stream);
+                });
+            });
+        }
+    };
+    std::vector<int> all(run.size());
+    std::iota(all.begin(), all.end(), 0);
     double cost = 0.0;
-    const std::vector<RunPass> passes = group_runs(list, s->nbits, total, s->prec, s->fp64_exact, &cost);
-    if (s->prec == kC128 && !s->fp64_exact && p->tensor_cores && s->nbits >= 12 &&
-        cost > 2.0 * z_pass_us(total)) {
+    const std::vector<RunPass> passes = group(all, &cost);
+    if (pairs && p->tensor_cores && s->nbits >= 12 && cost > 2.0 * z_pass_us(total)) {
         std::vector<std::vector<int>> bits;
         for (const PlainGate& g : run) bits.push_back(g.gate.bits);
         const std::vector<FusedBlock> blocks = fuse(bits, s->nbits, 5);
-        bool faster = (double)blocks.size() * z_pass_us(total) < cost;
-        for (const FusedBlock& b : blocks) faster = faster && b.qubits.size() <= 5;
+        // the blocks in order: one for the tensor cores, or the gates of
+        // neighbours that are not, as tile passes
+        struct Part {
+            int block = -1;
+            std::vector<int> gates;
+            std::vector<RunPass> passes;
+        };
+        std::vector<Part> parts;
+        double us = 0.0;
+        bool faster = true;
+        for (size_t i = 0; i < blocks.size(); ++i) {
+            const FusedBlock& b = blocks[i];
+            faster = faster && b.qubits.size() <= 5;
+            if (std::any_of(b.gates.begin(), b.gates.end(), [&](int g) { return rounds_all(run[g].op); })) {
+                parts.emplace_back();
+                parts.back().block = (int)i;
+                us += z_pass_us(total);
+                continue;
+            }
+            if (parts.empty() || parts.back().block >= 0) parts.emplace_back();
+            parts.back().gates.insert(parts.back().gates.end(), b.gates.begin(), b.gates.end());
+        }
+        for (Part& part : parts) {
+            if (part.block >= 0 || !faster) continue;
+            double tiles = 0.0;
+            part.passes = group(part.gates, &tiles);
+            us += tiles;
+        }
+        faster = faster && us < cost;
         if (faster) {
             std::vector<SeqGate> gates;
             for (const PlainGate& g : run) gates.push_back(g.gate);
-            std::vector<std::vector<cd>> mats;
-            for (const FusedBlock& b : blocks) {
-                mats.push_back(block_matrix(b, gates));
-                faster = faster && tc_block_bounded(mats.back().data(), 1 << b.qubits.size());
+            std::vector<std::vector<cd>> mats(blocks.size());
+            for (const Part& part : parts) {
+                if (part.block < 0) continue;
+                const FusedBlock& b = blocks[part.block];
+                mats[part.block] = block_matrix(b, gates);
+                faster = faster && tc_block_bounded(mats[part.block].data(), 1 << b.qubits.size());
             }
             if (faster) {
-                for (size_t i = 0; i < blocks.size(); ++i) {
-                    const std::vector<int>& q = blocks[i].qubits;
-                    const GateOp op = classify(mats[i].data(), (int)q.size(), q.data(), s->nbits);
+                for (const Part& part : parts) {
+                    if (part.block < 0) {
+                        emit_passes(part.gates, part.passes);
+                        continue;
+                    }
+                    const std::vector<int>& q = blocks[part.block].qubits;
+                    const std::vector<cd>& mat = mats[part.block];
+                    const GateOp op = classify(mat.data(), (int)q.size(), q.data(), s->nbits);
                     if (op.kind == GateOp::Dense) {
                         tensor_cores();
-                        lower_z_block(s, mats[i], q, stage, emit);
+                        lower_z_block(s, mat, q, stage, emit);
                     } else if (op.kind != GateOp::Noop) {
                         one(op);
                     }
@@ -1454,24 +1526,7 @@ static void lower_plain_gates(q1g_plan* p, q1g_state* s, const std::vector<Plain
             }
         }
     }
-    const char* name = s->prec == kC64 ? "gate_run_c64" : s->fp64_exact ? "gate_run_c128_fp64" : "gate_run_c128";
-    std::vector<RunOp> table;
-    for (const RunPass& pass : passes) {
-        uint64_t touched = 0;
-        for (int i : pass.ops) touched += run[i].op.touched(total);
-        if (pass.ops.size() < 2 || (touched <= total && total * s->bsz() > (uint64_t(64) << 20))) {
-            for (int i : pass.ops) one(run[i].op);
-            continue;
-        }
-        table.clear();
-        for (int i : pass.ops) table.push_back(make_run_op(run[i].op, pass.tile));
-        const RunOp* d = static_cast<const RunOp*>(stage(table.data(), table.size() * sizeof(RunOp)));
-        emit([name, tile = pass.tile, d, n = (int)table.size()](q1g_state* x) {
-            x->launch(name, 2.0 * x->total() * x->bsz(), [&] {
-                return launch_gate_run(x->amps.p, x->prec, x->total(), tile, d, n, x->fp64_exact, x->stream);
-            });
-        });
-    }
+    emit_passes(all, passes);
 }
 
 // Device bytes of a block's staged data at most: a run table entry per gate
@@ -1694,6 +1749,26 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
         lower_plain_gates(p, s, plain, stage, emit, tensor_cores);
         plain.clear();
     };
+    // A complex128 block of gates of 0, +-1 and +-i alone: a dense product would
+    // round the amplitudes that the gates only move, so they go with the plain
+    // gates, as long as the tile passes cost no more than a dense pass (about 30
+    // CX at 26 qubits).
+    auto take_unit_gates = [&](size_t i) {
+        std::vector<PlainGate> units;
+        for (int g : p->blocks[i].gates) {
+            GateOp o = classify(gates[g].mat.data(), (int)gates[g].bits.size(), gates[g].bits.data(), s->nbits);
+            if (o.kind == GateOp::Noop) continue;
+            if (!is_unit(o)) return false;
+            units.push_back({std::move(o), gates[g]});
+        }
+        std::vector<const GateOp*> list;
+        for (const PlainGate& g : units) list.push_back(&g.op);
+        double cost = 0.0;
+        group_runs(list, s->nbits, s->total(), s->prec, false, &cost);
+        if (cost > z_pass_us(s->total())) return false;
+        for (PlainGate& g : units) plain.push_back(std::move(g));
+        return true;
+    };
     for (size_t i = first; i < nb; ++i) {
         if (p->blocks[i].phase_run && !phase_kernels_take(s)) {
             for (int g : p->blocks[i].gates) {
@@ -1715,6 +1790,7 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
                 plain.push_back({ops[i], {bbits[i], bmats[i]}});
                 continue;
             }
+            if (s->prec == kC128 && !s->fp64_exact && take_unit_gates(i)) continue;
         }
         if (p->blocks[i].phase_run) {
             // an uncontrolled gate just before (a Fourier transform's first

@@ -25,6 +25,15 @@ bool run_takes(const GateOp& op)
     return small(op.m2, 4) && small(op.m2 + 4, 4);
 }
 
+bool is_unit(const GateOp& op)
+{
+    int swap, u0, u1;
+    if (op.kind == GateOp::Phase) return unit_code(op.ph[0], op.ph[1]) >= 0;
+    return op.kind == GateOp::Pair && mono_pair(op.m2, swap, u0, u1);
+}
+
+bool rounds_all(const GateOp& op) { return op.kind == GateOp::Pair && op.map.nz == 1 && !is_unit(op); }
+
 namespace {
 
 uint64_t positions_mask(const GateOp& op)
@@ -32,13 +41,6 @@ uint64_t positions_mask(const GateOp& op)
     uint64_t m = 0;
     for (int q = 0; q < op.map.nz; ++q) m |= uint64_t(1) << op.map.zpos[q];
     return m;
-}
-
-bool is_mono(const GateOp& op)
-{
-    int swap, u0, u1;
-    if (op.kind == GateOp::Phase) return unit_code(op.ph[0], op.ph[1]) >= 0;
-    return mono_pair(op.m2, swap, u0, u1);
 }
 
 // What an op costs (measured on one GB300): microseconds of a CTA that has
@@ -52,7 +54,7 @@ struct OpCost {
 OpCost op_cost(const GateOp& op, int prec, bool fp64_exact)
 {
     const double w = op.kind == GateOp::Pair ? 1.0 : 0.5;
-    if (is_mono(op)) return {0.3, 0.3e-3 * w, 0.2e-3 * w};
+    if (is_unit(op)) return {0.3, 0.3e-3 * w, 0.2e-3 * w};
     if (prec == kC64) return {0.35, 0.45e-3 * w, 0.3e-3 * w};
     if (fp64_exact) return {0.4, 4.5e-3 * w, 4.0e-3 * w};
     return {0.35, 1.2e-3 * w, 1.0e-3 * w};

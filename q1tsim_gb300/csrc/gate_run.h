@@ -61,6 +61,14 @@ uint64_t run_need(const GateOp& op);
 // Whether an op can be part of a run: a pair or a phase whose matrix does not
 // grow amplitudes (rows of |re| + |im| sums <= 2.01), on at most 12 positions.
 bool run_takes(const GateOp& op);
+// Whether a gate moves and re-signs amplitudes without arithmetic (entries of
+// 0, +-1 and +-i).
+bool is_unit(const GateOp& op);
+// Whether a gate's arithmetic rounds every amplitude of the state (an
+// uncontrolled pair update).  Only beside such a gate may the others' amplitudes
+// be held rounded: without one, some amplitudes are touched by no arithmetic
+// and keep their bits.
+bool rounds_all(const GateOp& op);
 // Groups `ops` (in order; every one run_takes and not a Noop) into passes on
 // a state of nbits qubits.  Ops on disjoint positions may change places.
 // prec / fp64_exact choose the cost model's arithmetic rates.
@@ -70,9 +78,13 @@ std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits
 // The op in the tile's local coordinates.
 RunOp make_run_op(const GateOp& op, const RunTile& tile);
 
+// A complex128 pass's arithmetic: in the state's type (FP64, or gates that
+// is_unit alone), in double-float pairs beside a gate that rounds_all, or in
+// pairs with the amplitudes followed that no gate rounds.
+enum class RunArith { kPlain, kPairs, kPairsPartly };
 // gate_run.cu: applies d_ops[0..nops) (nops <= kRunMaxOps) to every tile of
-// `total` amplitudes.
+// `total` amplitudes (complex64: any arith).
 cudaError_t launch_gate_run(void* amps, int prec, uint64_t total, const RunTile& tile, const RunOp* d_ops, int nops,
-                            bool fp64_exact, cudaStream_t st);
+                            RunArith arith, cudaStream_t st);
 
 }  // namespace q1g
