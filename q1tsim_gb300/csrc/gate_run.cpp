@@ -67,8 +67,8 @@ struct Item {
 };
 
 // Takes, in order, every remaining item that can move to the front and
-// whose needed positions lie in S.
-double absorb(const std::vector<Item>& items, const std::vector<int>& left, uint64_t S, uint64_t all,
+// whose needed positions lie in S (in_order: up to the first whose do not).
+double absorb(const std::vector<Item>& items, const std::vector<int>& left, uint64_t S, uint64_t all, bool in_order,
               std::vector<int>* taken)
 {
     uint64_t blocked = 0;
@@ -80,7 +80,7 @@ double absorb(const std::vector<Item>& items, const std::vector<int>& left, uint
             if (taken) taken->push_back(i);
         } else {
             blocked |= it.full;
-            if ((blocked & all) == all) break;
+            if (in_order || (blocked & all) == all) break;
         }
     }
     return got;
@@ -141,7 +141,7 @@ std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits
             uint64_t best_set = 0;
             double best_got = -1.0;
             auto consider = [&](uint64_t S) {
-                const double got = absorb(items, left, S, all, nullptr);
+                const double got = absorb(items, left, S, all, fp64_exact, nullptr);
                 if (got > best_got) {
                     best_got = got;
                     best_set = S;
@@ -156,7 +156,7 @@ std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits
                         S |= it.need;
                     } else {
                         blocked |= it.full;
-                        if ((blocked & all) == all) break;
+                        if (fp64_exact || (blocked & all) == all) break;
                     }
                 }
                 consider(S);
@@ -166,7 +166,7 @@ std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits
             for (int a = low; a + w <= nbits; ++a) consider(low_mask | (((uint64_t(1) << w) - 1) << a));
             RunPass p;
             std::vector<int> taken;
-            absorb(items, left, best_set, all, &taken);
+            absorb(items, left, best_set, all, fp64_exact, &taken);
             if (taken.empty()) {     // an op that needs more positions than the low ones leave room for
                 best_set = items[left[0]].need;
                 taken.push_back(left[0]);

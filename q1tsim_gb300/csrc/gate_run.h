@@ -70,7 +70,9 @@ bool is_unit(const GateOp& op);
 // and keep their bits.
 bool rounds_all(const GateOp& op);
 // Groups `ops` (in order; every one run_takes and not a Noop) into passes on
-// a state of nbits qubits.  Ops on disjoint positions may change places.
+// a state of nbits qubits.  Ops on disjoint positions may change places, which
+// changes roundings; with fp64_exact, whose purpose is the rounding of the gates
+// one by one, they keep their order.
 // prec / fp64_exact choose the cost model's arithmetic rates.
 // *cost_us: the model's time for them.
 std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits, uint64_t total, int prec,
