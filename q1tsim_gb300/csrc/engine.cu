@@ -1606,6 +1606,7 @@ static size_t run_subspace_prefix(q1g_plan* p, q1g_state* s, const double* mats,
     q1g_state* c = s->compact.get();
     c->stream = s->stream;
     c->fp64_exact = s->fp64_exact;
+    c->tc_wait_ns = s->tc_wait_ns;
     c->prof = s->prof;
     c->nshots = s->nshots;
     const uint64_t b = s->basis[0];
