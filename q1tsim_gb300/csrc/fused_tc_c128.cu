@@ -317,7 +317,10 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
     const uint64_t count = (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
 
     build_operands(mat, smem, tid);
-    if (tid == 0) {
+    // (every .aligned instruction below follows a __syncwarp, or a vote or block
+    // barrier of CUDA's, after the last branch of single lanes; warp 0 has none
+    // before it allocates)
+    if (tid == 32) {
         *abort_flag = 0;
         mbar_init(mbar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -425,6 +428,7 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
                 row_fp64(sbase + kZOffIn + q * kZWarp * 16u, rslot, p, mat + 256 * part, y);
                 for (int j = 0; j < 8; ++j) a[bases[i % kZBases] + offset_of(j)] = y[j];
             }
+            __syncwarp();
             asm volatile("bar.sync %0, 128;" ::"r"(1u + q) : "memory");
 #pragma unroll
             for (int j = 0; j < 8; ++j) x[j] = lds_amp(at(in, j));    // (not kept across the call)
@@ -460,8 +464,8 @@ k_fused_tc_c128(double2* __restrict__ a, uint64_t ntiles, const __grid_constant_
         bool ok = true;
         float acc[5][16];
         if (warp == 15 && lane == 0) put_base(it + 2);
+        __syncwarp();      // (that lane, or lane 0 of warp 0, which issues, may be behind)
         if (kLast) {
-            __syncwarp();      // (lane 0 of warp 0 may be behind, issuing)
             ok = wait_phase(mbar, (uint32_t)(it - 1) & 1u, abort_flag, wait_ns);
             __syncwarp();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
