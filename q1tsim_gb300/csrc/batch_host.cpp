@@ -18,10 +18,11 @@ q1g_batch::~q1g_batch()
     if (graph) cudaGraphDestroy(graph);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
-    if (stream) {
-        cudaStreamSynchronize(stream);
-        cudaStreamDestroy(stream);
-    }
+    if (!stream) return;
+    const bool idle = cudaStreamSynchronize(stream) == cudaSuccess;
+    for (DevBuf* b : {&arena, &results, &dcircuits, &dops, &dmats, &dtables, &lfact, &scratch, &queue, &traffic})
+        b->release(idle);
+    cudaStreamDestroy(stream);
 }
 
 namespace q1g {

@@ -243,7 +243,7 @@ int q1g_state_compare(q1g_state* a, q1g_state* b, double* out5)
         const uint64_t n = a->ncols * a->N;
         const uint64_t want = (n + 255) / 256;
         const unsigned blocks = (unsigned)std::min<uint64_t>(want ? want : 1, 152 * 16);
-        DevBuf part;
+        DevBuf part(&a->stream);
         part.ensure(6 * blocks * sizeof(double));
         std::vector<double> h(6 * blocks);
         auto pass = [&](double wa, double wb, double* sums, double* mx) {
@@ -683,6 +683,7 @@ int q1g_state_device_amplitudes(q1g_state* s, void** ptr, size_t* bytes)
         s->settle_norms();
         s->sync();
         *ptr = s->amps.p;
+        s->amps.lent = true;
         if (bytes) *bytes = s->total() * s->bsz();
     });
 }

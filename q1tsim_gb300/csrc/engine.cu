@@ -30,53 +30,98 @@ void check_cuda(cudaError_t e, const char* what)
 // cudaFree of a 27-qubit complex128 state (2 GiB) take 1.7 ms, its product
 // state 1.0.  Bounded (kPoolBytes a device, the oldest blocks make room);
 // returned when an allocation fails and by q1g_release_cached_memory.  A block
-// enters only after the device has finished everything (as cudaFree waits, too),
-// so any stream or thread may have it next.
+// enters with an event behind its last use and is taken on the stream that used
+// it, which then waits for the event on the device, or once the event has
+// happened: neither a release nor a take waits on the host or touches other
+// streams (to synchronise the device would end a capture on any of them).
 namespace {
 
 constexpr size_t kPoolBytes = size_t(4) << 30;
 constexpr size_t kPoolBlocks = 256;
 constexpr int kPoolDevices = 64;
 
+bool capturing(cudaStream_t st)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();
+    return true;
+}
+
 struct DevicePool {
     struct Block {
         size_t size;
         void* p;
+        cudaStream_t stream;     // of the event
+        cudaEvent_t last;        // null: idle
     };
     std::mutex mu;
     std::deque<Block> blocks;      // oldest first
     size_t bytes = 0;
 
-    // The smallest block of at least `size` bytes and not much more, or null.
-    void* take(size_t size, size_t* got)
+    static void free(const Block& b)
     {
-        std::lock_guard<std::mutex> lock(mu);
-        const size_t most = std::max(size + size / 8, size_t(1) << 16);
-        auto best = blocks.end();
-        for (auto it = blocks.begin(); it != blocks.end(); ++it)
-            if (it->size >= size && it->size <= most && (best == blocks.end() || it->size < best->size)) best = it;
-        if (best == blocks.end()) return nullptr;
-        void* q = best->p;
-        *got = best->size;
-        bytes -= best->size;
-        blocks.erase(best);
-        return q;
+        if (b.last) {
+            cudaEventSynchronize(b.last);
+            cudaEventDestroy(b.last);
+        }
+        cudaFree(b.p);
     }
-    // Keeps a block; the oldest ones make room.
-    void put(void* q, size_t size)
+    // The smallest block of at least `size` bytes and not much more that stream
+    // `st` (null: any) may use, or null.
+    void* take(size_t size, const cudaStream_t* st, size_t* got)
     {
-        std::vector<void*> out;
+        if (st && capturing(*st)) return nullptr;
+        Block b;
         {
             std::lock_guard<std::mutex> lock(mu);
-            while (!blocks.empty() && (bytes + size > kPoolBytes || blocks.size() >= kPoolBlocks)) {
-                out.push_back(blocks.front().p);
+            const size_t most = std::max(size + size / 8, size_t(1) << 16);
+            auto best = blocks.end();
+            for (auto it = blocks.begin(); it != blocks.end(); ++it) {
+                if (it->size < size || it->size > most || (best != blocks.end() && it->size >= best->size)) continue;
+                if (it->last && !(st && it->stream == *st)) {
+                    if (cudaEventQuery(it->last) != cudaSuccess) {
+                        (void)cudaGetLastError();
+                        continue;
+                    }
+                    cudaEventDestroy(it->last);
+                    it->last = nullptr;
+                }
+                best = it;
+            }
+            if (best == blocks.end()) return nullptr;
+            b = *best;
+            bytes -= b.size;
+            blocks.erase(best);
+        }
+        if (b.last) {
+            // (the handle may be another stream's by now)
+            const cudaError_t e = cudaStreamWaitEvent(*st, b.last, 0);
+            if (e != cudaSuccess) {
+                (void)cudaGetLastError();
+                free(b);
+                return nullptr;
+            }
+            cudaEventDestroy(b.last);
+        }
+        *got = b.size;
+        return b.p;
+    }
+    // Keeps a block; the oldest ones make room.
+    void put(const Block& b)
+    {
+        std::vector<Block> out;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            while (!blocks.empty() && (bytes + b.size > kPoolBytes || blocks.size() >= kPoolBlocks)) {
+                out.push_back(blocks.front());
                 bytes -= blocks.front().size;
                 blocks.pop_front();
             }
-            blocks.push_back({size, q});
-            bytes += size;
+            blocks.push_back(b);
+            bytes += b.size;
         }
-        for (void* o : out) cudaFree(o);
+        for (const Block& o : out) free(o);
     }
     void trim()
     {
@@ -86,7 +131,7 @@ struct DevicePool {
             all.swap(blocks);
             bytes = 0;
         }
-        for (const Block& o : all) cudaFree(o.p);
+        for (const Block& o : all) free(o);
     }
 };
 
@@ -134,7 +179,7 @@ void DevBuf::ensure(size_t b)
     int device;
     DevicePool* pool = current_pool(&device);
     size_t got = size;
-    void* q = pool ? pool->take(size, &got) : nullptr;
+    void* q = pool ? pool->take(size, user, &got) : nullptr;
     if (!q) {
         cudaError_t e = cudaMalloc(&q, size);
         if (e == cudaErrorMemoryAllocation && pool) {
@@ -154,21 +199,29 @@ void DevBuf::ensure(size_t b)
     dev = device;
 }
 
-void DevBuf::release()
+void DevBuf::release(bool idle)
 {
     if (p) {
+        // Memory that the caller has seen, or of which no stream is known, is
+        // freed: cudaFree waits for whatever uses it.
         int device;
-        DevicePool* pool = bytes <= kPoolBytes ? current_pool(&device) : nullptr;
-        const bool idle = pool && device == dev && cudaDeviceSynchronize() == cudaSuccess;
-        if (idle) {
-            pool->put(p, bytes);
-        } else {
-            (void)cudaGetLastError();
-            cudaFree(p);
+        DevicePool* pool = bytes <= kPoolBytes && !lent ? current_pool(&device) : nullptr;
+        cudaEvent_t last = nullptr;
+        bool keep = pool && device == dev && (idle || (user && !capturing(*user)));
+        if (keep && !idle) {
+            keep = cudaEventCreateWithFlags(&last, cudaEventDisableTiming) == cudaSuccess;
+            if (keep && cudaEventRecord(last, *user) != cudaSuccess) {
+                cudaEventDestroy(last);
+                keep = false;
+            }
+            if (!keep) (void)cudaGetLastError();
         }
+        if (keep) pool->put({bytes, p, last ? *user : nullptr, last});
+        else cudaFree(p);
     }
     p = nullptr;
     bytes = 0;
+    lent = false;
     dev = -1;
 }
 
@@ -258,9 +311,10 @@ q1g_state::~q1g_state()
 {
     compact.reset();   // it runs on this state's stream: free it while the stream exists
     unary_plan.reset();
-    if (stream) cudaStreamSynchronize(stream);
+    const bool idle = stream && cudaStreamSynchronize(stream) == cudaSuccess &&
+                      (!copy_stream || cudaStreamSynchronize(copy_stream) == cudaSuccess);
+    for (DevBuf* b : {&amps, &spare, &dscratch, &uscratch, &colbuf, &errbuf}) b->release(idle);
     if (copy_stream) {
-        cudaStreamSynchronize(copy_stream);
         cudaEventDestroy(copy_event);
         cudaStreamDestroy(copy_stream);
     }

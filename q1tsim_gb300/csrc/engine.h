@@ -32,25 +32,31 @@ struct Error : std::exception {
 
 void check_cuda(cudaError_t e, const char* what);
 
-// Grow-only device allocation.
+// Grow-only device allocation.  `user`: the stream in whose order every use of
+// the memory lies (a state's buffers), null where several streams use it or the
+// stream may be gone when the buffer goes (a plan's).
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
-    DevBuf() = default;
+    bool lent = false;      // the caller has the pointer
+    explicit DevBuf(const cudaStream_t* stream = nullptr) : user(stream) {}
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     void ensure(size_t b);
-    void release();
-    void swap(DevBuf& o)
+    // idle: nothing that uses the memory is under way
+    void release(bool idle = false);
+    void swap(DevBuf& o)        // (with the same user)
     {
         std::swap(p, o.p);
         std::swap(bytes, o.bytes);
+        std::swap(lent, o.lent);
         std::swap(dev, o.dev);
     }
     ~DevBuf() { release(); }
     template <typename T> T* as() const { return static_cast<T*>(p); }
 
 private:
+    const cudaStream_t* user;
     int dev = -1;
 };
 // Device memory that released buffers left for new ones, and its return.
@@ -111,13 +117,13 @@ struct q1g_state {
     // compare, single-qubit measurement, conditional gates).
     bool norm_pending = false;
 
-    q1g::DevBuf amps, spare;
-    q1g::DevBuf dscratch;   // doubles
-    q1g::DevBuf uscratch;   // uint64
-    q1g::DevBuf colbuf;     // CollapseCol table
-    q1g::DevBuf errbuf;     // error flag of bounded device waits
-    q1g::HostBuf hstage;    // pinned staging for results
     cudaStream_t stream = nullptr;
+    q1g::DevBuf amps{&stream}, spare{&stream};
+    q1g::DevBuf dscratch{&stream};   // doubles
+    q1g::DevBuf uscratch{&stream};   // uint64
+    q1g::DevBuf colbuf{&stream};     // CollapseCol table
+    q1g::DevBuf errbuf{&stream};     // error flag of bounded device waits
+    q1g::HostBuf hstage;    // pinned staging for results
     bool own_stream = false;
     cudaStream_t copy_stream = nullptr;    // of the words' upload in measure_all, made on first use
     cudaEvent_t copy_event = nullptr;

@@ -86,9 +86,9 @@ void histogram_words(const uint64_t* words, size_t n, uint64_t* keys, uint64_t* 
     while (cap < 2 * (uint64_t)n) cap <<= 1;
     // words | table keys | table counts | compacted keys | compacted counts | 2 counters
     const size_t bytes = (n + 4 * cap + 2) * sizeof(uint64_t);
-    DevBuf buf;
+    DevBuf buf(&st);
     buf.ensure(bytes);
-    DevBuf errb;
+    DevBuf errb(&st);
     errb.ensure(sizeof(int));
     uint64_t* d_words = buf.as<uint64_t>();
     auto* d_keys = reinterpret_cast<unsigned long long*>(d_words + n);
