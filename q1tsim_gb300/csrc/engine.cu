@@ -32,8 +32,8 @@ void check_cuda(cudaError_t e, const char* what)
 // returned when an allocation fails and by q1g_release_cached_memory.  A block
 // enters with an event behind its last use and is taken on the stream that used
 // it, which then waits for the event on the device, or once the event has
-// happened: neither a release nor a take waits on the host or touches other
-// streams (to synchronise the device would end a capture on any of them).
+// happened.  Memory that several streams may use waits for all of them with
+// finish_device.
 namespace {
 
 constexpr size_t kPoolBytes = size_t(4) << 30;
@@ -46,6 +46,17 @@ bool capturing(cudaStream_t st)
     if (cudaStreamIsCapturing(st, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
     (void)cudaGetLastError();
     return true;
+}
+
+// Waits for everything on the device: cudaFree does, of a small block in 2 us
+// where nothing is under way, and is no invalid call while another thread's
+// stream is captured, as cudaDeviceSynchronize is (it ends the capture).
+bool finish_device()
+{
+    void* q = nullptr;
+    if (cudaMalloc(&q, 1) == cudaSuccess && cudaFree(q) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
 }
 
 struct DevicePool {
@@ -202,19 +213,21 @@ void DevBuf::ensure(size_t b)
 void DevBuf::release(bool idle)
 {
     if (p) {
-        // Memory that the caller has seen, or of which no stream is known, is
-        // freed: cudaFree waits for whatever uses it.
         int device;
-        DevicePool* pool = bytes <= kPoolBytes && !lent ? current_pool(&device) : nullptr;
+        DevicePool* pool = bytes <= kPoolBytes ? current_pool(&device) : nullptr;
         cudaEvent_t last = nullptr;
-        bool keep = pool && device == dev && (idle || (user && !capturing(*user)));
+        bool keep = pool && device == dev && (idle || !user || !capturing(*user));
         if (keep && !idle) {
-            keep = cudaEventCreateWithFlags(&last, cudaEventDisableTiming) == cudaSuccess;
-            if (keep && cudaEventRecord(last, *user) != cudaSuccess) {
-                cudaEventDestroy(last);
-                keep = false;
+            if (user && !lent) {
+                keep = cudaEventCreateWithFlags(&last, cudaEventDisableTiming) == cudaSuccess;
+                if (keep && cudaEventRecord(last, *user) != cudaSuccess) {
+                    cudaEventDestroy(last);
+                    keep = false;
+                }
+                if (!keep) (void)cudaGetLastError();
+            } else {
+                keep = finish_device();
             }
-            if (!keep) (void)cudaGetLastError();
         }
         if (keep) pool->put({bytes, p, last ? *user : nullptr, last});
         else cudaFree(p);
@@ -313,7 +326,7 @@ q1g_state::~q1g_state()
     unary_plan.reset();
     const bool idle = stream && cudaStreamSynchronize(stream) == cudaSuccess &&
                       (!copy_stream || cudaStreamSynchronize(copy_stream) == cudaSuccess);
-    for (DevBuf* b : {&amps, &spare, &dscratch, &uscratch, &colbuf, &errbuf}) b->release(idle);
+    for (DevBuf* b : {&amps, &spare, &dscratch, &uscratch, &colbuf, &errbuf}) b->release(idle && !b->lent);
     if (copy_stream) {
         cudaEventDestroy(copy_event);
         cudaStreamDestroy(copy_stream);

@@ -38,7 +38,7 @@ void check_cuda(cudaError_t e, const char* what);
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
-    bool lent = false;      // the caller has the pointer
+    bool lent = false;      // the caller has the pointer, for streams of its own
     explicit DevBuf(const cudaStream_t* stream = nullptr) : user(stream) {}
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;

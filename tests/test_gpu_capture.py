@@ -54,6 +54,22 @@ def test_state_freed_during_a_capture(n):
     assert not states
 
 
+def test_lent_memory_and_plans_freed_during_a_capture():
+    """Memory that more streams than the state's may use, and plans'."""
+    from q1tsim_gb300 import Plan
+    from q1tsim_gb300.sharded import EngineShard
+    shard = EngineShard(16, 1, "c128")
+    shard.amplitudes().zero_()
+    bits = [[q] for q in range(16)]
+    plan = Plan(16, bits, 0)
+    shard.state.apply_plan(plan, np.tile(np.asarray(G.H().matrix()).ravel(), 16).view(np.float64))
+    shard.state.synchronize()
+    kept = [shard.state, plan]
+    del shard, plan
+    _capture(kept.clear)
+    assert not kept
+
+
 def test_state_grown_during_a_capture():
     s = VectorState(16, 64, "c128")
     for q in range(4):
@@ -68,3 +84,26 @@ def test_state_grown_during_a_capture():
     _capture(grow)
     assert s.ncols == 16
     np.testing.assert_allclose(np.linalg.norm(s.states(), axis=0), 1.0, rtol=0, atol=1e-12)
+
+
+def test_lent_memory_waits_for_the_callers_stream():
+    """A state freed while another stream still reads its amplitudes: a new
+    state does not get the memory before the reader is done."""
+    import torch
+    from q1tsim_gb300.sharded import EngineShard
+    n = 22
+    for _ in range(4):
+        shard = EngineShard(n, 1, "c128")
+        a = shard.amplitudes()
+        a.copy_(torch.full_like(a, 2.0))
+        torch.cuda.synchronize()
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(20_000_000)         # some 10 ms
+            b = a.clone()
+        del a, shard
+        s = VectorState(n, 1, "c128")
+        s.apply_gate(G.H(), [0])
+        s.synchronize()
+        stream.synchronize()
+        assert bool((b == 2.0).all())
