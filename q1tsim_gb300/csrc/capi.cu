@@ -148,7 +148,7 @@ int q1g_state_from_amplitudes(const double* amps, size_t nr_bits, size_t nr_shot
                 });
             }
             s->sync();
-            if (s->spare.bytes > (size_t(1) << 30)) s->spare.release();
+            s->spare.release();
             s->sparse = false;
             s->basis.clear();
             double nrm = 0.0;

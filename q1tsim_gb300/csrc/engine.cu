@@ -522,10 +522,6 @@ struct CondRange {
     bool apply;
 };
 
-// A split's old columns are kept for the next one up to this size: allocating
-// 1 GB and freeing it again takes longer (1 to 2 ms) than the split itself.
-constexpr size_t kKeptSpareBytes = size_t(4) << 30;
-
 static std::vector<CondRange> conditional_ranges(const std::vector<uint64_t>& counts,
                                                  const uint8_t* control)
 {
@@ -572,7 +568,7 @@ void q1g_state::apply_conditional(const uint8_t* control, size_t ncontrol, const
         spare.ensure(nr * N * bsz());
         copy_columns("column_copy", 2.0 * nr, spare.p, 0, cols);
         amps.swap(spare);
-        if (spare.bytes > kKeptSpareBytes) spare.release();
+        release_spare();
         ncols = nr;
     }
     if (!same_layout) {
@@ -584,6 +580,15 @@ void q1g_state::apply_conditional(const uint8_t* control, size_t ncontrol, const
     for (size_t j = 0; j < ranges.size(); ++j) counts[j] = ranges[j].len;
     for (size_t j = 0; j < ranges.size(); ++j)
         if (ranges[j].apply) apply_op(op, col_ptr(j), N);
+}
+
+// The columns before a split go to the kept memory, where the next split finds
+// them.  A pointer to them that the caller has ended with their shape
+// (q1g_state_device_amplitudes), so the state's stream is the last user.
+void q1g_state::release_spare()
+{
+    spare.lent = false;
+    spare.release();
 }
 
 // New columns `cols` of amps into dst (launch_collapse_copy); moved: columns'
@@ -702,7 +707,7 @@ void q1g_state::measure(size_t qbit, size_t cbit, uint64_t* res, size_t res_len,
         spare.ensure(new_nr * N * bsz());
         copy_columns("collapse", 1.5 * new_nr, spare.p, pos, cols);
         amps.swap(spare);
-        if (spare.bytes > kKeptSpareBytes) spare.release();
+        release_spare();
     }
     ncols = new_nr;
     counts = nc;

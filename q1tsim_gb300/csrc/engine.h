@@ -205,6 +205,7 @@ struct q1g_state {
     void apply_conditional(const uint8_t* control, size_t ncontrol, const double* mat, size_t k,
                            const size_t* bits, size_t nbits_given);
     void copy_columns(const char* name, double moved, void* dst, int pos, const std::vector<q1g::CollapseCol>& cols);
+    void release_spare();
     std::vector<double> zero_weights(size_t qbit);
     void measure(size_t qbit, size_t cbit, uint64_t* res, size_t res_len, const double* uniforms,
                  size_t nu, q1g_rng* rng, bool collapse);
