@@ -788,10 +788,19 @@ void q1g_state::measure_all(const size_t* cbits, size_t ncbits, uint64_t* res, s
         const uint64_t nspc = uniforms ? 0 : nshots + ncols;
         // The group sums (1/16 of a complex64 state, 1/16 of a complex128 one)
         // pay where the shots would read more than that from whole chunks:
-        // from one shot per 32 chunks on; up to 1 GiB of scratch.
+        // from one shot per 32 chunks on; up to 1 GiB of scratch, and where the
+        // device has that.
         const uint64_t group_doubles = prec == kC64 ? ncols * ncc * 16 : ncols * ncc * 32;
-        const bool groups = chunk == 256 && nshots * 32 >= ncols * ncc && group_doubles <= (uint64_t(1) << 27);
-        const uint64_t nd = ncols * ncc + ncols + scan_tmp + nshots + 2 * nspc + (groups ? group_doubles : 0) + 16;
+        bool groups = chunk == 256 && nshots * 32 >= ncols * ncc && group_doubles <= (uint64_t(1) << 27);
+        const uint64_t nd = ncols * ncc + ncols + scan_tmp + nshots + 2 * nspc + 16;
+        if (groups) {
+            try {
+                dscratch.ensure((nd + group_doubles) * sizeof(double));
+            } catch (const Error& e) {
+                if (e.code != Q1G_ERR_OUT_OF_MEMORY) throw;
+                groups = false;
+            }
+        }
         dscratch.ensure(nd * sizeof(double));
         double* d_sums = dscratch.as<double>();
         double* d_group = d_sums + ((ncols * ncc + 15) & ~uint64_t(15));     // 128-byte lines

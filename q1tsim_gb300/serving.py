@@ -39,10 +39,21 @@ class Request:
         self.result = None
         self.error = None
 
+    def least_bytes(self):
+        """Device memory that the request cannot do without: the state plus
+        sampling scratch (chunk sums, uniforms, outcomes)."""
+        return (self._amp() << self.circuit.nr_qbits) + 48 * self.shots + (8 << max(self.circuit.nr_qbits - 8, 0))
+
     def state_bytes(self):
-        amp = 16 if self.circuit.precision == "c128" else 8
-        # the state plus sampling scratch (chunk sums, uniforms, outcomes)
-        return (amp << self.circuit.nr_qbits) + 48 * self.shots + (8 << max(self.circuit.nr_qbits - 8, 0))
+        """least_bytes and the group sums that measure_all keeps for many
+        shots (1/16 of the state, up to 1 GiB, where the device has it)."""
+        n, groups = self.circuit.nr_qbits, 0
+        if n >= 8 and 32 * self.shots >= 1 << (n - 8):
+            groups = (self._amp() << n) // 16
+        return self.least_bytes() + (groups if groups <= 1 << 30 else 0)
+
+    def _amp(self):
+        return 16 if self.circuit.precision == "c128" else 8
 
     @property
     def latency(self):
@@ -93,8 +104,8 @@ class Server:
 
     # ------------------------------------------------------------ client
     def submit(self, req):
-        if req.state_bytes() > self.budget:
-            raise ValueError(f"request {req.rid} needs {req.state_bytes()} bytes, above the HBM budget")
+        if req.least_bytes() > self.budget:
+            raise ValueError(f"request {req.rid} needs {req.least_bytes()} bytes, above the HBM budget")
         with self.cv:
             self.pending.append(req)
             self.cv.notify_all()
@@ -107,11 +118,16 @@ class Server:
             t.join()
 
     # ------------------------------------------------------------ worker
+    def _charge(self, req):
+        """What a request takes of the budget (all of it at most: the group
+        sums of the largest ones are optional)."""
+        return min(req.state_bytes(), self.budget)
+
     def _admit(self):
         """Oldest pending request that fits, or None (FIFO head only)."""
-        if self.pending and self.used + self.pending[0].state_bytes() <= self.budget:
+        if self.pending and self.used + self._charge(self.pending[0]) <= self.budget:
             req = self.pending.popleft()
-            self.used += req.state_bytes()
+            self.used += self._charge(req)
             self.peak_used = max(self.peak_used, self.used)
             self.inflight += 1
             self.peak_inflight = max(self.peak_inflight, self.inflight)
@@ -149,7 +165,7 @@ class Server:
                 req.error = repr(e)
             req.done = time.perf_counter()
             with self.cv:
-                self.used -= req.state_bytes()
+                self.used -= self._charge(req)
                 self.inflight -= 1
                 self.completed.append(req)
                 self.cv.notify_all()
