@@ -1476,9 +1476,9 @@ struct PlainGate {
 
 // Microseconds of a complex128 tensor-core pass (6.2 to 6.9 per tile of an SM: 0.70 ms
 // at 26 qubits), or of a block's matrix on the host where that is longer.
-static double z_pass_us(uint64_t total)
+static double z_pass_us(uint64_t total, int sms)
 {
-    return std::max(5.0 + 6.4 * std::ceil((double)(total >> 12) / 152.0), 100.0);
+    return std::max(5.0 + 6.4 * std::ceil((double)(total >> 12) / sms), 100.0);
 }
 
 // A run of plain gates: as tile passes (gate_run.h), or, on complex128
@@ -1508,7 +1508,7 @@ static void lower_plain_gates(q1g_plan* p, q1g_state* s, const std::vector<Plain
     auto group = [&](const std::vector<int>& at, double* cost) {
         std::vector<const GateOp*> list;
         for (int i : at) list.push_back(&run[i].op);
-        return group_runs(list, s->nbits, total, s->prec, s->fp64_exact, cost);
+        return group_runs(list, s->nbits, total, s->prec, s->fp64_exact, cost, s->sm_count());
     };
     const bool pairs = s->prec == kC128 && !s->fp64_exact;
     std::vector<RunOp> table;
@@ -1544,7 +1544,7 @@ static void lower_plain_gates(q1g_plan* p, q1g_state* s, const std::vector<Plain
     std::iota(all.begin(), all.end(), 0);
     double cost = 0.0;
     const std::vector<RunPass> passes = group(all, &cost);
-    if (pairs && p->tensor_cores && s->nbits >= 12 && cost > 2.0 * z_pass_us(total)) {
+    if (pairs && p->tensor_cores && s->nbits >= 12 && cost > 2.0 * z_pass_us(total, s->sm_count())) {
         std::vector<std::vector<int>> bits;
         for (const PlainGate& g : run) bits.push_back(g.gate.bits);
         const std::vector<FusedBlock> blocks = fuse(bits, s->nbits, 5);
@@ -1564,7 +1564,7 @@ static void lower_plain_gates(q1g_plan* p, q1g_state* s, const std::vector<Plain
             if (std::any_of(b.gates.begin(), b.gates.end(), [&](int g) { return rounds_all(run[g].op); })) {
                 parts.emplace_back();
                 parts.back().block = (int)i;
-                us += z_pass_us(total);
+                us += z_pass_us(total, s->sm_count());
                 continue;
             }
             if (parts.empty() || parts.back().block >= 0) parts.emplace_back();
@@ -1846,8 +1846,8 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
         std::vector<const GateOp*> list;
         for (const PlainGate& g : units) list.push_back(&g.op);
         double cost = 0.0;
-        group_runs(list, s->nbits, s->total(), s->prec, false, &cost);
-        if (cost > z_pass_us(s->total())) return false;
+        group_runs(list, s->nbits, s->total(), s->prec, false, &cost, s->sm_count());
+        if (cost > z_pass_us(s->total(), s->sm_count())) return false;
         for (PlainGate& g : units) plain.push_back(std::move(g));
         return true;
     };

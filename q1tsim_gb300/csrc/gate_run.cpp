@@ -105,7 +105,7 @@ RunTile make_tile(uint64_t S, int bits)
 }  // namespace
 
 std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits, uint64_t total, int prec,
-                                bool fp64_exact, double* cost_us)
+                                bool fp64_exact, double* cost_us, int sms)
 {
     const int m = (int)ops.size();
     std::vector<Item> items(m);
@@ -132,7 +132,7 @@ std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits
         if (bytes <= 32e6) low = prec == kC128 ? 1 : 2;
         low = std::min(low, T);
         const uint64_t low_mask = (uint64_t(1) << low) - 1;
-        const double tiles = (double)(total >> T), per_sm = std::ceil(tiles / 152.0);
+        const double tiles = (double)(total >> T), per_sm = std::ceil(tiles / sms);
         std::vector<RunPass> passes;
         std::vector<int> left(m);
         for (int i = 0; i < m; ++i) left[i] = i;

@@ -74,9 +74,9 @@ bool rounds_all(const GateOp& op);
 // changes roundings; with fp64_exact, whose purpose is the rounding of the gates
 // one by one, they keep their order.
 // prec / fp64_exact choose the cost model's arithmetic rates.
-// *cost_us: the model's time for them.
+// *cost_us: the model's time for them, on a device of `sms` SMs.
 std::vector<RunPass> group_runs(const std::vector<const GateOp*>& ops, int nbits, uint64_t total, int prec,
-                                bool fp64_exact, double* cost_us = nullptr);
+                                bool fp64_exact, double* cost_us = nullptr, int sms = 152);
 // The op in the tile's local coordinates.
 RunOp make_run_op(const GateOp& op, const RunTile& tile);
 
