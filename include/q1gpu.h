@@ -289,6 +289,14 @@ int q1g_batch_info(const q1g_batch* b, size_t* ncircuits, size_t* total_runs, si
  * reads and writes (gate blocks, measurement, collapse, sampling) and the
  * classical words it updates, as counted by the kernel. */
 int q1g_batch_traffic(const q1g_batch* b, uint64_t* bytes);
+/* CTAs that run one of the largest circuits together (its words do not depend
+ * on it): 2, 4 or 8 for every circuit of 12 qubits and more ahead of the first
+ * smaller one in the queue (longest first), 1 for none, 0 (the default) as the
+ * estimate says.  Before the first run. */
+int q1g_batch_set_team_size(q1g_batch* b, int size);
+/* How the last run was laid out: its first `circuits` circuits on `count` teams
+ * of `size` CTAs (0, 1, 0: every circuit on one). */
+int q1g_batch_teams(const q1g_batch* b, int* circuits, int* size, int* count);
 
 /* ---- profiling: per-kernel CUDA-event timing on the state's stream */
 int q1g_profile_enable(q1g_state* s, int enable);

@@ -38,6 +38,10 @@ def _protos(L):
     L.q1g_batch_info.restype = ctypes.c_int
     L.q1g_batch_traffic.argtypes = [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint64)]
     L.q1g_batch_traffic.restype = ctypes.c_int
+    L.q1g_batch_set_team_size.argtypes = [ctypes.c_void_p, ctypes.c_int]
+    L.q1g_batch_set_team_size.restype = ctypes.c_int
+    L.q1g_batch_teams.argtypes = [ctypes.c_void_p] + 3 * [ctypes.POINTER(ctypes.c_int)]
+    L.q1g_batch_teams.restype = ctypes.c_int
     L._batch_protos = True
 
 
@@ -140,6 +144,17 @@ class Batch:
             res.append(out[off:off + s])
             off += s
         return res
+
+    def set_team_size(self, size=0):
+        """CTAs that run one of the largest circuits together (q1g_batch_set_team_size):
+        1, 2, 4 or 8, 0 = as the estimate says.  Before the first run."""
+        check(_lib.load().q1g_batch_set_team_size(self._h, int(size)), "batch_set_team_size")
+
+    def teams(self):
+        """How the last run was laid out: (circuits on teams, CTAs of a team, teams)."""
+        v = [ctypes.c_int() for _ in range(3)]
+        check(_lib.load().q1g_batch_teams(self._h, *(ctypes.byref(x) for x in v)))
+        return tuple(x.value for x in v)
 
     def info(self):
         nc, runs, arena, nops = (ctypes.c_size_t() for _ in range(4))

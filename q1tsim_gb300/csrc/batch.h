@@ -5,6 +5,14 @@
 
 #include "engine.h"
 
+namespace q1g {
+// How a batch's largest circuits run: the first `circuits` of the queue on
+// `count` teams of `size` CTAs.
+struct TeamPlan {
+    int circuits = 0, size = 1, count = 0;
+};
+}  // namespace q1g
+
 struct q1g_batch {
     int width = 4;                      // fusion width (<= 4)
     std::vector<q1g::BatchCircuit> circuits;   // in add order; res_off set at build
@@ -16,6 +24,8 @@ struct q1g_batch {
     uint64_t arena_amps = 0;
     uint64_t scratch_per_cta = 0;
     int sms = 0;
+    int team_size = 0;                  // CTAs of a team as asked for (0: chosen by the estimate)
+    q1g::TeamPlan teams;                // set at build
     q1g::DevBuf arena, results, dcircuits, dops, dmats, dtables, lfact, scratch, queue, traffic;
     q1g::HostBuf hresults, htraffic;
     cudaStream_t stream = nullptr;
@@ -32,11 +42,6 @@ void batch_add_circuit(q1g_batch* b, size_t nr_bits, size_t nr_shots, uint64_t s
                        const size_t* nbits_per_op, const size_t* bits_flat, const double* mats_flat,
                        const size_t* args);
 void batch_run(q1g_batch* b, uint64_t* results, size_t len);
-// How a batch's largest circuits run: the first `circuits` of the queue on
-// `count` teams of `size` CTAs.
-struct TeamPlan {
-    int circuits = 0, size = 1, count = 0;
-};
 // Teams of `size` CTAs, of which `count` run at once; us: each circuit's time on
 // one, in queue order.
 struct TeamChoice {

@@ -274,7 +274,17 @@ static void batch_build(q1g_batch* b)
         alone.push_back(time[i]);
         able.push_back(b->circuits[i].nbits >= kBatchTeamBits);
     }
-    const TeamPlan teams = plan_teams(alone, able, b->sms, choices);
+    b->teams = plan_teams(alone, able, b->sms, choices);
+    if (b->team_size) {
+        b->teams = TeamPlan{};
+        for (const TeamChoice& c : choices)
+            if (c.size == b->team_size && c.count > 0) {
+                const auto first_small = std::find(able.begin(), able.end(), char(0));
+                b->teams = {(int)(first_small - able.begin()), c.size, c.count};
+            }
+    }
+    if (b->teams.circuits == 0) b->teams = TeamPlan{};
+    const TeamPlan& teams = b->teams;
     std::vector<BatchCircuit> queue;
     uint64_t off = 0, per_cta = 16;
     for (size_t i : order) {

@@ -590,6 +590,27 @@ int q1g_batch_info(const q1g_batch* b, size_t* ncircuits, size_t* total_runs, si
     });
 }
 
+int q1g_batch_set_team_size(q1g_batch* b, int size)
+{
+    return guarded([&] {
+        need(b, "batch");
+        if (size < 0 || size > 8 || (size & (size - 1)))
+            throw Error(Q1G_ERR_INVALID_ARGUMENT, "a team has 1, 2, 4 or 8 CTAs, or 0 to choose");
+        if (b->built) throw Error(Q1G_ERR_INVALID_ARGUMENT, "batch already ran: set the team size before the first run");
+        b->team_size = size;
+    });
+}
+
+int q1g_batch_teams(const q1g_batch* b, int* circuits, int* size, int* count)
+{
+    return guarded([&] {
+        need(b, "batch");
+        if (circuits) *circuits = b->teams.circuits;
+        if (size) *size = b->teams.size;
+        if (count) *count = b->teams.count;
+    });
+}
+
 int q1g_batch_traffic(const q1g_batch* b, uint64_t* bytes)
 {
     return guarded([&] {
