@@ -1428,12 +1428,14 @@ static size_t lower_phase_group(q1g_plan* p, q1g_state* s, size_t i, const GateO
 // Whether a dense block (its classified op, matrix and qubits) on this state
 // runs on the tensor cores: complex64 in pairs of f16 halves (fused_tc.cu),
 // complex128 in six digits (fused_tc_c128.cu) unless FP64 arithmetic was asked
-// for.
+// for.  Complex128 blocks with controls stay on the kernels that leave the other
+// amplitudes alone: the digits would round those to the largest of their row.
 static bool tc_takes(const q1g_plan* p, const q1g_state* s, const GateOp& op, const std::vector<cd>& mat,
                      const std::vector<int>& bits)
 {
     return p->tensor_cores && s->nbits >= 12 && !(s->prec == kC128 && s->fp64_exact) && op.kind == GateOp::Dense &&
-           op.t >= 3 && bits.size() <= 5 && tc_block_bounded(mat.data(), 1 << bits.size());
+           op.t >= 3 && bits.size() <= 5 && (s->prec == kC64 || op.map.nz == op.t) &&
+           tc_block_bounded(mat.data(), 1 << bits.size());
 }
 
 // A block as a tensor-core pass of a complex128 state.
@@ -1851,6 +1853,26 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
         for (PlainGate& g : units) plain.push_back(std::move(g));
         return true;
     };
+    // A complex128 block that is not one for the tensor cores, gate by gate (its
+    // product would take the FP64 pipe from four qubits on).
+    auto take_apart = [&](size_t i) {
+        for (int g : p->blocks[i].gates) {
+            const SeqGate& q = gates[g];
+            GateOp o = classify(q.mat.data(), (int)q.bits.size(), q.bits.data(), s->nbits);
+            if (o.kind == GateOp::Noop) continue;
+            if (run_takes(o)) {
+                plain.push_back({std::move(o), q});
+                continue;
+            }
+            flush_plain();
+            if (tc_takes(p, s, o, q.mat, q.bits)) {
+                tensor_cores();
+                lower_z_block(s, q.mat, q.bits, stage, emit);
+            } else {
+                emit([o](q1g_state* x) { x->apply_op(o, x->amps.as<char>(), x->total()); });
+            }
+        }
+    };
     for (size_t i = first; i < nb; ++i) {
         if (p->blocks[i].phase_run && !phase_kernels_take(s)) {
             for (int g : p->blocks[i].gates) {
@@ -1873,6 +1895,11 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
                 continue;
             }
             if (s->prec == kC128 && !s->fp64_exact && take_unit_gates(i)) continue;
+            if (s->prec == kC128 && !s->fp64_exact && p->tensor_cores && s->nbits >= 12 && ops[i].t >= 3 &&
+                p->blocks[i].gates.size() > 1 && ops[i].map.nz != ops[i].t) {
+                take_apart(i);
+                continue;
+            }
         }
         if (p->blocks[i].phase_run) {
             // an uncontrolled gate just before (a Fourier transform's first
