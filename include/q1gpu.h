@@ -86,8 +86,9 @@ void q1g_last_error_args(uint64_t* a0, uint64_t* a1);
 int q1g_version(void);
 /* Visible device: SM count and memory.  Any pointer may be NULL. */
 int q1g_device_info(int* sm_count, size_t* free_bytes, size_t* total_bytes);
-/* Up to 4 GiB of device memory that freed states leave is kept for the next
- * ones (and counted as free above); this returns it to the device. */
+/* Up to 4 GiB of device memory that freed states and replaced columns leave is
+ * kept for the next ones (and counted as free above); this returns it to the
+ * device. */
 int q1g_release_cached_memory(void);
 
 /* ---- construction: VectorState::new / from_qubit_coefs (src/vectorstate.rs:41-83) */

@@ -1476,8 +1476,10 @@ struct PlainGate {
     SeqGate gate;
 };
 
-// Microseconds of a complex128 tensor-core pass (6.2 to 6.9 per tile of an SM: 0.70 ms
-// at 26 qubits), or of a block's matrix on the host where that is longer.
+// Microseconds of a complex128 tensor-core pass, or of a block's matrix on the
+// host where that is longer.  26 qubits, 108 tiles per SM: 657 us straight to
+// memory and 752 staged (6.1 and 7.0 per tile); which one a block takes is known
+// only once it is laid out.
 static double z_pass_us(uint64_t total, int sms)
 {
     return std::max(5.0 + 6.4 * std::ceil((double)(total >> 12) / sms), 100.0);
@@ -2035,7 +2037,7 @@ static void lower_and_run(q1g_plan* p, q1g_state* s, const double* mats, size_t 
 // only: the result is FP64's, where the gates would each round at 2^-48 (a
 // 24-qubit circuit of 2 layers: 9e-15 off before, 5e-15 now), in the time of the
 // tile pass that it saves (16 qubits, 20 layers: 400 us either way; 26 qubits,
-// 6 layers, in the compact state: 12.1 ms with the gates, 11.5 so).  Returns the
+// 6 layers, in the compact state: 0.6 ms less than with the gates).  Returns the
 // number of blocks done.
 static size_t run_product_lead(const q1g_plan* p, q1g_state* s, const double* mats)
 {

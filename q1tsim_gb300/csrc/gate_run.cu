@@ -16,9 +16,10 @@
 // memory is read and written once per 40-60 gates), on small ones the
 // latency of a gate's chain, about 0.5 us.  Measured on one GB300 against one
 // launch and one HBM pass per gate: complex128 brick circuits of 10 qubits,
-// depth 8 (116 gates) 0.63 -> 0.12 ms (with the plan's launches kept), 16 qubits,
-// depth 20 (470 gates) 2.86 -> 0.40 ms, 26 qubits, depth 6 (231 gates) 59.9 ->
-// 35.5 ms (complex128 states of that size take the tensor cores now, 11.5 ms).
+// depth 8 (116 gates), with shots, 0.63 -> 0.12 ms, 16 qubits, depth 20 (470
+// gates) 2.86 -> 0.40 ms, both with the plan's launches kept; 26 qubits, depth 6
+// (231 gates) 59.9 -> 35.5 ms (most gates of complex128 states of that size take
+// the tensor cores now: 9.4 ms).
 #include <algorithm>
 #include <mutex>
 #include <set>
@@ -130,12 +131,13 @@ __device__ __forceinline__ void apply_plain(E* t, const RunOp& o, int bits)
 
 // ------------------------------------------------ double-float arithmetic
 //
-// One pair per thread in scalar FP32 instructions: the packed FP32x2 forms
-// run at the same FMA rate but need their operands in adjacent registers,
-// and the moves that takes cost more issue slots than the packing saves
-// (26 qubits: 30.4 ms packed, 33.6 ms scalar, of 60 ms gate by gate; 16 qubits:
-// 0.38 and 0.32 ms); and a small tile has only as many pairs as threads,
-// where one pair's chain is the time.
+// One pair per thread in scalar FP32 instructions.  The packed FP32x2 forms
+// run at the same FMA rate but need their operands in adjacent registers: with
+// the amplitudes as they lie the moves cost more issue slots than the packing
+// saves (26 qubits, depth 6: 43.6 ms, 35.5 scalar).  With parts in planes of their
+// own and two pairs per thread that was 30.4 ms, but 16 qubits took 0.38 ms for
+// 0.32: a small tile has only as many pairs as threads, one pair's chain is the
+// time, and small states are what this kernel serves in complex128.
 
 // A staged amplitude (re.h, re.l, im.h, im.l), component by component.
 __device__ __forceinline__ DF re_of(float4 v) { return DF{v.x, v.y}; }

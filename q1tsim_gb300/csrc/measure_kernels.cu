@@ -250,9 +250,9 @@ __global__ void __launch_bounds__(kScanThreads) k_pair_scan_tiles(ScanPair s)
 // Outcome probabilities are summed hierarchically, with the same arithmetic
 // in the reduction and in the search so the two agree: p_i = |a_i|^2 in the
 // state's precision, groups of 8 consecutive p_i summed sequentially in that
-// precision, chunks of 32 groups (256 amplitudes) summed in FP64, and the
-// FP64 exclusive prefix over chunks.  A shot finds its chunk by a search on that
-// prefix, its group by a warp scan of the chunk's 32 group sums, and its
+// precision, chunks of 32 groups (256 amplitudes) summed in the state's
+// precision too (chunk_total, sampling.cuh), and the FP64 exclusive prefix over
+// chunks.  A shot finds its chunk by a search on that prefix, its group by a warp scan of the chunk's 32 group sums, and its
 // amplitude by a sequential scan of the group.
 
 // One warp per chunk of `chunk` (<= 256) amplitudes.  groups (or null): the 32
